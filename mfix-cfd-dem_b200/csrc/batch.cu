@@ -637,7 +637,8 @@ int dem_sys_download_pairs(dem_handle* h, int32_t s, int32_t* ni, int32_t* nb, d
   }
   if (ni) cudaMemcpyAsync(ni, tmp, sizeof(int) * max_pip, cudaMemcpyDeviceToHost, h->stream);
   if (nb && P) cudaMemcpyAsync(nb, tmp + max_pip, sizeof(int) * P, cudaMemcpyDeviceToHost, h->stream);
-  if (pf && P) cudaMemcpyAsync(pf, h->pft[h->pcur] + 3 * (size_t)e[0], sizeof(double) * 3 * P, cudaMemcpyDeviceToHost, h->stream);
+  if (pf && P)
+    if (int rc = download_history(h, e[0], P, pf)) return rc;
   return check_cuda(h, cudaStreamSynchronize(h->stream), "download system pairs");
 }
 

@@ -644,7 +644,8 @@ int dem_download_pairs(dem_handle* h, int32_t* ni, int32_t* nb, double* pf, int6
   if ((nb || pf) && cap < P) return set_err(h, DEM_ERR_CAPACITY, "pair capacity too small");
   if (ni) cudaMemcpyAsync(ni, h->row_end[h->rb], sizeof(int) * h->n, cudaMemcpyDeviceToHost, h->stream);
   if (nb && P) cudaMemcpyAsync(nb, h->nbrs[h->rb], sizeof(int) * P, cudaMemcpyDeviceToHost, h->stream);
-  if (pf && P) cudaMemcpyAsync(pf, h->pft[h->pcur], sizeof(double) * 3 * P, cudaMemcpyDeviceToHost, h->stream);
+  if (pf && P)
+    if (int rc = download_history(h, 0, P, pf)) return rc;
   if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "download pairs")) return rc;
   if (ni) for (int i = 0; i < h->n; ++i) ni[i] += 1;
   if (nb) for (long long c = 0; c < P; ++c) nb[c] += 1;
@@ -678,7 +679,7 @@ int dem_upload_pairs(dem_handle* h, const int32_t* ni, const int32_t* nb, const 
   cudaMemcpyAsync(h->row_end[h->rb], re.data(), sizeof(int) * h->n, cudaMemcpyHostToDevice, h->stream);
   if (np) {
     cudaMemcpyAsync(h->nbrs[h->rb], nbr.data(), sizeof(int) * np, cudaMemcpyHostToDevice, h->stream);
-    cudaMemcpyAsync(h->pft[h->pcur], pf, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, h->stream);
+    if (int rc = upload_history(h, np, pf)) return rc;
   }
   h->n_pairs = np;
   h->np_stale = false;

@@ -140,9 +140,16 @@ __device__ __forceinline__ const DevParams& sysp(const DevParams& p, const Batch
 // What the two particles of a contact pair need to add the pair's terms to
 // FC/TOW in the reference's order: FC_TMP, CROSS(NORMAL, FT) with the two
 // lever arms (the torques are DIST_CL*TOW_force and DIST_CI*TOW_force), and
-// KN_DES and OVERLAP_N for the rolling-friction torque.  80 bytes.
+// KN_DES and OVERLAP_N for the rolling-friction torque.
 struct PairRec {
   double fc[3], tf[3], dcl2, dci2, kn, ov;
+};
+// The record in memory, 80 bytes a pair in two arrays: (fc, tf, dcl2, dci2)
+// as two aligned 32-byte words, read and written with one instruction each,
+// and (kn, ov), which only a system with rolling friction writes and reads.
+struct RecStore {
+  double4* main;   // [2 * pair], [2 * pair + 1]
+  double2* roll;   // [pair]
 };
 
 struct FacetBinEntry {  // one entry of facets_at_dg(cell)
@@ -287,13 +294,17 @@ struct dem_handle {
   int* row_cnt = nullptr;     // n
   int* row_end[2] = {nullptr, nullptr};   // n (current / previous build)
   int* nbrs[2] = {nullptr, nullptr};      // cap
-  double* pft[2] = {nullptr, nullptr};    // 3*cap; pft[pcur] is current, the other takes the carry-over of a rebuild
+  // 3*cap, a plane of cap values per component (neighbouring pairs' values
+  // lie side by side); pft[pcur] is current, the other takes the carry-over
+  // of a rebuild
+  double* pft[2] = {nullptr, nullptr};
   int* in_cnt = nullptr;      // n
   int* in_start = nullptr;    // n+1
-  int* in_fill = nullptr;     // n
+  int* in_fill = nullptr;     // n: fill counts while the transpose is made, then the first slot of each
+                              // incoming list whose owner has a higher index (the list's end when none)
   int2* in_pair = nullptr;    // cap
   int* in_pos = nullptr;      // cap: slot of each pair in its neighbour's incoming list (inverse of in_pair)
-  uint8_t* in_flag = nullptr; // cap: PF_CONTACT of the pair at each incoming slot (split-precision records)
+  uint8_t* in_flag = nullptr; // cap: PF_CONTACT of the pair at each incoming slot
   int* pair_owner = nullptr;  // cap
   // cap: PF_* bits of each pair, one array per history buffer: pflagb[pcur]
   // goes with pft[pcur] (the other is stencil-rank scratch during a build
@@ -305,7 +316,10 @@ struct dem_handle {
   float* pgap = nullptr;      // cap: gap |d| - (r_i + r_j) of each pair at the last build, rounded down
   double* skin = nullptr;     // [0]: bound on any particle's displacement since the last build
   unsigned* vslot = nullptr;  // [32]: per-step displacement bounds, as float bits
-  demb::PairRec* prec = nullptr; // cap: contact terms of the last force pass
+  void* prec = nullptr;       // 80*cap bytes: contact terms of the last force pass
+  demb::RecStore recs() const {
+    return {static_cast<double4*>(prec), reinterpret_cast<double2*>(static_cast<char*>(prec) + 64 * pair_cap)};
+  }
   int rb = 0;                 // which row_end/nbrs buffer is current
 
   // walls
@@ -399,6 +413,10 @@ int ensure_pair_capacity(dem_handle* h, long long need);
 int build_transpose(dem_handle* h, int nb);    // neighbor.cu
 void launch_neigh_count(dem_handle* h, const int* skip = nullptr);        // neighbor.cu: count pass of the pair build
 void set_hist_flags(dem_handle* h);            // neighbor.cu: PF_HIST from the current history
+// neighbor.cu: the history of pairs [first, first + count) between its planes
+// and PFT_NEIGHBOR's (3,P) order on the host
+int download_history(dem_handle* h, long long first, long long count, double* pf);
+int upload_history(dem_handle* h, long long count, const double* pf);
 void launch_skin(dem_handle* h);               // force.cu: adds the step's displacement to the bound
 void skin_unknown(dem_handle* h);              // force.cu: positions changed from outside: no pair skipped
 void launch_wall_gaps(dem_handle* h);          // force.cu: wall clearances at a build (with the pair gaps)
@@ -505,6 +523,96 @@ struct ProfScope {
   ProfScope(dem_handle* hh, int cls);
   ~ProfScope();
 };
+
+// ---------------------------------------------------------------------------
+// 32-byte loads and stores (one instruction per lane where double4 takes
+// two; the address must be 32-byte aligned).  A lane that gathers a particle's
+// state or a contact record touches one sector per word, and the kernels
+// that do so are bound by the number of such accesses the L1 takes in.  The
+// loads are for arrays that the kernel does not write.
+__device__ __forceinline__ double4 ld32(const double4* p) {
+  double4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st32(double4* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+// Contact bits (PF_CONTACT, bit 0 of each flag byte) of flags[base,
+// base + cnt), cnt <= 32, as a mask: the bytes are read as aligned 32-bit
+// words (the flag arrays carry 16 bytes of padding past their capacity).
+__device__ __forceinline__ unsigned contact_mask(const uint8_t* __restrict__ flags, int base, int cnt) {
+  static_assert(PF_CONTACT == 1, "contact bit is bit 0");
+  unsigned mask = 0u;
+  const int w0 = base & ~3;
+  for (int w = w0; w < base + cnt; w += 4) {
+    const uint32_t v = *reinterpret_cast<const uint32_t*>(flags + w) & 0x01010101u;
+    const unsigned b4 = (v | (v >> 7) | (v >> 14) | (v >> 21)) & 0xFu;  // byte k -> bit k
+    const int sh = w - base;
+    mask |= sh >= 0 ? (b4 << sh) : (b4 >> -sh);
+  }
+  return cnt >= 32 ? mask : (mask & ((1u << cnt) - 1u));
+}
+
+// The pairs of a warp's window [c0, c0 + WIN_PAIRS) that a pair kernel has to
+// look at, as a queue in shared memory: pair offset in the window, PF_HIST
+// and PF_CONTACT of the last pass above it.  A pair whose gap at the build
+// exceeds `reach` (twice the displacement bound since, rounded up) with a
+// zero history is apart without a look at its particles: its flags are
+// cleared and it is left out.  A lane screens four consecutive pairs from one
+// load of flags and one of gaps; the queue then gives every lane a pair, so
+// the contact arithmetic and its gathers run on full warps (about 0.4 of a
+// dense bed's pairs are in contact).  Returns the queue's length, the same
+// in every lane.
+constexpr int WIN_PAIRS = 128;
+constexpr int WQ_CONTACT = 1 << 7, WQ_HIST = 1 << 8;
+__device__ __forceinline__ int screen_window(long long c0w, long long np, uint8_t* __restrict__ pflag,
+                                             uint8_t* __restrict__ in_flag, const int* __restrict__ in_pos,
+                                             const float* __restrict__ pgap, float reach, uint16_t* queue) {
+  static_assert(PF_CONTACT << 7 == WQ_CONTACT && PF_HIST << 7 == WQ_HIST, "flags move up by seven bits");
+  const int lane = threadIdx.x & 31;
+  const long long c0 = c0w + 4 * lane;
+  uint32_t fw = 0;  // the four flags, one per byte
+  float g[4] = {0.f, 0.f, 0.f, 0.f};
+  int live = 4;
+  if (c0 + 3 < np) {
+    fw = *reinterpret_cast<const uint32_t*>(pflag + c0);
+    const float4 gq = *reinterpret_cast<const float4*>(pgap + c0);
+    g[0] = gq.x; g[1] = gq.y; g[2] = gq.z; g[3] = gq.w;
+  } else {
+    live = c0 < np ? (int)(np - c0) : 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (j < live) { fw |= (uint32_t)pflag[c0 + j] << (8 * j); g[j] = pgap[c0 + j]; }
+  }
+  unsigned need = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (j >= live) break;
+    const uint8_t f = (uint8_t)(fw >> (8 * j));
+    if ((f & PF_HIST) || !(g[j] > reach)) {
+      need |= 1u << j;
+    } else if (f) {
+      pflag[c0 + j] = 0;
+      if (f & PF_CONTACT) in_flag[in_pos[c0 + j]] = 0;
+    }
+  }
+  const int mine = __popc(need);
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  int at = incl - mine;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if ((need >> j) & 1u)
+      queue[at++] = (uint16_t)((4 * lane + j) | (((fw >> (8 * j)) & (PF_CONTACT | PF_HIST)) << 7));
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, incl, 31);
+}
 
 // ---------------------------------------------------------------------------
 // Device helpers.  All FP64 arithmetic in the parity kernels is compiled

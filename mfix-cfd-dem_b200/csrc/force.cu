@@ -549,134 +549,107 @@ k_walls(DevParams p0, BatchView bv, WallCtx w, const int* __restrict__ wlist, co
 }
 
 // Kernel 2 (per pair): one CC iteration of CALC_FORCE_DEM, evaluated once
-// per pair.  A pair whose gap at the last build is more than twice the
-// bound on any particle's displacement since (and whose history is zero) is
-// apart without a look at the particles: the reference's apart test would
-// find it apart and leave its zero history zero, so it is skipped.  The
-// apart test of the others needs only the two positions; velocities, spins
-// and masses are gathered only for pairs in contact.  The tangential history
-// PFT is updated in place (only this kernel reads it).  pflag keeps, per
-// pair, PF_CONTACT (in contact at this pass) and PF_HIST (history nonzero),
-// so a pair that stays apart with a zero history costs no history traffic.
-// The contact terms go to a record that both particles read back in
-// kernel 3, and both particles of a contact are marked in `touched`.
+// per pair.  A warp takes a window of WIN_PAIRS pairs, queues those that may
+// be in contact (screen_window) and gives each lane one of the queue.  The
+// apart test needs only the two positions; velocities, spins and masses are
+// gathered only for pairs in contact.  The tangential history PFT is updated
+// in place (only this kernel reads it).  pflag keeps, per pair, PF_CONTACT
+// (in contact at this pass) and PF_HIST (history nonzero), so a pair that
+// stays apart with a zero history costs no history traffic; in_flag keeps the
+// neighbour's view of PF_CONTACT in transpose order.  The contact terms go to
+// a record that both particles read back in kernel 3, and both particles of a
+// contact are marked in `touched`.
+// Bound by latency and by the accesses the L1 takes in, not by DRAM (a fifth of
+// its throughput).  The 1,000,000-sphere bed with 1.67 M of its 4.4 M pairs in contact:
+// 248 us with four pairs per thread (12 of 32 lanes in contact at a time) and
+// records written 8 bytes at a time, 156 us so.
 template <int COLL, bool B>
 __global__ void __launch_bounds__(256, 2)
 k_pairs(DevParams p0, BatchView bv, const int* __restrict__ d_np, long long cap, const int* __restrict__ owner,
-        const int* __restrict__ nbrs, const double4* __restrict__ pos4, const double4* __restrict__ vel4,
-        const double4* __restrict__ omg4, const int8_t* __restrict__ state, const uint8_t* __restrict__ phase,
-        double* __restrict__ pft, uint8_t* __restrict__ pflag, uint8_t* __restrict__ touched,
-        const float* __restrict__ pgap, const double* __restrict__ skin, PairRec* __restrict__ prec,
-        DevErr* __restrict__ err) {
+        const int* __restrict__ nbrs, const int* __restrict__ in_pos, const double4* __restrict__ pos4,
+        const double4* __restrict__ vel4, const double4* __restrict__ omg4, const int8_t* __restrict__ state,
+        const uint8_t* __restrict__ phase, double* __restrict__ pft, uint8_t* __restrict__ pflag,
+        uint8_t* __restrict__ in_flag, uint8_t* __restrict__ touched, const float* __restrict__ pgap,
+        const double* __restrict__ skin, RecStore rec, DevErr* __restrict__ err) {
+  __shared__ uint16_t s_queue[256 / 32][WIN_PAIRS];
   // persistent grid-stride loop over the device-side pair count (the grid
   // size does not depend on the list, so the launch can live in a graph)
   const long long np = min((long long)*d_np, cap);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const double reach = 2.0 * skin[0];
+  const float reach = __double2float_ru(2.0 * skin[0]);
   unsigned long long ncont = 0;
   unsigned eflags = 0;
-  // four consecutive pairs per iteration: their flags and gaps arrive in
-  // one load each, so a run of apart pairs costs few dependent loads
-  const long long ng = (np + 3) / 4;
-  for (long long g4 = (long long)blockIdx.x * blockDim.x + threadIdx.x; g4 < ng; g4 += stride) {
-    const long long c0 = 4 * g4;
-    uint32_t fw = 0;  // the four flags, one per byte
-    float4 gq = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c0 + 3 < np) {
-      fw = *reinterpret_cast<const uint32_t*>(pflag + c0);
-      gq = *reinterpret_cast<const float4*>(pgap + c0);
-    } else {
-      if (c0 < np) { fw |= pflag[c0]; gq.x = pgap[c0]; }
-      if (c0 + 1 < np) { fw |= (uint32_t)pflag[c0 + 1] << 8; gq.y = pgap[c0 + 1]; }
-      if (c0 + 2 < np) { fw |= (uint32_t)pflag[c0 + 2] << 16; gq.z = pgap[c0 + 2]; }
-    }
-    // bit j: pair c0+j is provably apart
-    const unsigned apart = ((!(fw & PF_HIST) && (double)gq.x > reach) ? 1u : 0u) |
-                           ((!((fw >> 8) & PF_HIST) && (double)gq.y > reach) ? 2u : 0u) |
-                           ((!((fw >> 16) & PF_HIST) && (double)gq.z > reach) ? 4u : 0u) |
-                           ((!((fw >> 24) & PF_HIST) && (double)gq.w > reach) ? 8u : 0u);
-    // the particles of the group's pairs in one load each, when any pair
-    // needs them (a group past the list's end has fewer than four)
-    int4 o4 = make_int4(0, 0, 0, 0), n4 = make_int4(0, 0, 0, 0);
-    const unsigned live = c0 + 3 < np ? 15u : (1u << (unsigned)(np - c0)) - 1u;
-    if (~apart & live) {
-      if (c0 + 3 < np) {
-        o4 = *reinterpret_cast<const int4*>(owner + c0);
-        n4 = *reinterpret_cast<const int4*>(nbrs + c0);
-      } else {
-        o4.x = owner[c0]; n4.x = nbrs[c0];
-        if (c0 + 1 < np) { o4.y = owner[c0 + 1]; n4.y = nbrs[c0 + 1]; }
-        if (c0 + 2 < np) { o4.z = owner[c0 + 2]; n4.z = nbrs[c0 + 2]; }
-      }
-    }
-#pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
-    const long long cc = c0 + j;
-    if (cc >= np) break;
-    const uint8_t f0 = (uint8_t)(fw >> (8 * j));
-    // provably apart: its gap at the build exceeds what the two particles
-    // can have closed since, and its history is zero (stays zero)
-    if ((apart >> j) & 1u) {
-      if (f0) pflag[cc] = 0;
-      continue;
-    }
-    const int ll = j == 0 ? o4.x : (j == 1 ? o4.y : (j == 2 ? o4.z : o4.w));
-    const int i = j == 0 ? n4.x : (j == 1 ? n4.y : (j == 2 ? n4.z : n4.w));
-    uint8_t f = f0 & PF_HIST;  // NONEXISTENT partner or zero distance: history kept
-    double* ph = pft + 3 * cc;
-    // the states and the positions in one round of loads (any slot's
-    // position can be read; it is used only for existing particles)
-    const double4 a = pos4[ll], b = pos4[i];
-    const int8_t sl = state[ll], si = state[i];
-    if (si != DEM_STATE_NONEXISTENT && sl != DEM_STATE_NONEXISTENT) {
-      const DevParams& p = sysp<B>(p0, bv, ll);
-      PState L, I;
-      L.x[0] = a.x; L.x[1] = a.y; L.x[2] = a.z; L.r = a.w;
-      I.x[0] = b.x; I.x[1] = b.y; I.x[2] = b.z; I.r = b.w;
-      const double r_lm = L.r + I.r;
-      double dist[3];
+  uint16_t* queue = s_queue[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const long long stride = (long long)WIN_PAIRS * ((gridDim.x * blockDim.x) >> 5);
+  for (long long w0 = (long long)WIN_PAIRS * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w0 < np; w0 += stride) {
+    const int nq = screen_window(w0, np, pflag, in_flag, in_pos, pgap, reach, queue);
+    for (int k = lane; k < nq; k += 32) {
+      const int e = queue[k];
+      const long long cc = w0 + (e & (WIN_PAIRS - 1));
+      const uint8_t f0 = (uint8_t)(e >> 7);
+      const int ll = owner[cc], i = nbrs[cc];
+      uint8_t f = f0 & PF_HIST;  // NONEXISTENT partner or zero distance: history kept
+      // the states and the positions in one round of loads (any slot's
+      // position can be read; it is used only for existing particles)
+      const double4 a = ld32(pos4 + ll), b = ld32(pos4 + i);
+      const int8_t sl = state[ll], si = state[i];
+      if (si != DEM_STATE_NONEXISTENT && sl != DEM_STATE_NONEXISTENT) {
+        const DevParams& p = sysp<B>(p0, bv, ll);
+        PState L, I;
+        L.x[0] = a.x; L.x[1] = a.y; L.x[2] = a.z; L.r = a.w;
+        I.x[0] = b.x; I.x[1] = b.y; I.x[2] = b.z; I.r = b.w;
+        const double r_lm = L.r + I.r;
+        double dist[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        double pj = I.x[c];
-        double s = periodic_shift(p, c, pj - L.x[c]);
-        if (s != 0.0) pj = pj + s;
-        dist[c] = pj - L.x[c];
+        for (int c = 0; c < 3; ++c) {
+          double pj = I.x[c];
+          double s = periodic_shift(p, c, pj - L.x[c]);
+          if (s != 0.0) pj = pj + s;
+          dist[c] = pj - L.x[c];
+        }
+        const double d2 = dot3(dist, dist);
+        if (d2 > (r_lm - SMALL_NUMBER) * (r_lm - SMALL_NUMBER)) {
+          if (f0 & PF_HIST) { pft[cc] = 0.0; pft[cap + cc] = 0.0; pft[2 * cap + cc] = 0.0; }
+          f = 0;
+        } else if (d2 == 0.0) {
+          eflags |= EF_ZERO_DIST;
+          err->zero_a = ll; err->zero_b = i;
+        } else {
+          const double4 va = ld32(vel4 + ll), vb = ld32(vel4 + i), wa = ld32(omg4 + ll), wb = ld32(omg4 + i);
+          double pin[3] = {0.0, 0.0, 0.0};
+          if (f0 & PF_HIST) { pin[0] = pft[cc]; pin[1] = pft[cap + cc]; pin[2] = pft[2 * cap + cc]; }
+          L.v[0] = va.x; L.v[1] = va.y; L.v[2] = va.z; L.m = va.w;
+          I.v[0] = vb.x; I.v[1] = vb.y; I.v[2] = vb.z; I.m = vb.w;
+          L.w[0] = wa.x; L.w[1] = wa.y; L.w[2] = wa.z;
+          I.w[0] = wb.x; I.w[1] = wb.y; I.w[2] = wb.z;
+          // one solids phase: no phase to look up
+          L.ph = p.nph > 1 ? phase[ll] : 0;
+          I.ph = p.nph > 1 ? phase[i] : 0;
+          double pout[3];
+          PairRec r;
+          contact_force<COLL>(p, L, I, dist, d2, pin, pout, r);
+          pft[cc] = pout[0]; pft[cap + cc] = pout[1]; pft[2 * cap + cc] = pout[2];
+          st32(rec.main + 2 * cc, r.fc[0], r.fc[1], r.fc[2], r.tf[0]);
+          st32(rec.main + 2 * cc + 1, r.tf[1], r.tf[2], r.dcl2, r.dci2);
+          if (p.mew_r > 0.0) rec.roll[cc] = make_double2(r.kn, r.ov);
+          touched[ll] = 1;
+          touched[i] = 1;
+          f = PF_CONTACT | ((pout[0] != 0.0 || pout[1] != 0.0 || pout[2] != 0.0) ? PF_HIST : 0);
+          ++ncont;
+        }
       }
-      const double d2 = dot3(dist, dist);
-      if (d2 > (r_lm - SMALL_NUMBER) * (r_lm - SMALL_NUMBER)) {
-        if (f0 & PF_HIST) { ph[0] = 0.0; ph[1] = 0.0; ph[2] = 0.0; }
-        f = 0;
-      } else if (d2 == 0.0) {
-        eflags |= EF_ZERO_DIST;
-        err->zero_a = ll; err->zero_b = i;
-      } else {
-        const double4 va = vel4[ll], vb = vel4[i], wa = omg4[ll], wb = omg4[i];
-        L.v[0] = va.x; L.v[1] = va.y; L.v[2] = va.z; L.m = va.w;
-        I.v[0] = vb.x; I.v[1] = vb.y; I.v[2] = vb.z; I.m = vb.w;
-        L.w[0] = wa.x; L.w[1] = wa.y; L.w[2] = wa.z;
-        I.w[0] = wb.x; I.w[1] = wb.y; I.w[2] = wb.z;
-        L.ph = phase[ll]; I.ph = phase[i];
-        double pin[3] = {0.0, 0.0, 0.0};
-        if (f0 & PF_HIST) { pin[0] = ph[0]; pin[1] = ph[1]; pin[2] = ph[2]; }
-        double pout[3];
-        PairRec r;
-        contact_force<COLL>(p, L, I, dist, d2, pin, pout, r);
-        ph[0] = pout[0]; ph[1] = pout[1]; ph[2] = pout[2];
-        prec[cc] = r;
-        touched[ll] = 1;
-        touched[i] = 1;
-        f = PF_CONTACT | ((pout[0] != 0.0 || pout[1] != 0.0 || pout[2] != 0.0) ? PF_HIST : 0);
-        ++ncont;
+      if (f != f0) {
+        pflag[cc] = f;
+        if ((f ^ f0) & PF_CONTACT) in_flag[in_pos[cc]] = f & PF_CONTACT;
       }
     }
-    if (f != f0) pflag[cc] = f;
-    }
+    __syncwarp();  // the queue is read before the next window fills it
   }
   for (int o = 16; o > 0; o >>= 1) {
     ncont += __shfl_down_sync(0xffffffffu, ncont, o);
     eflags |= __shfl_down_sync(0xffffffffu, eflags, o);
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     if (ncont) atomicAdd(&err->n_contacts, ncont);
     if (eflags) atomicOr(&err->flags, eflags);
   }
@@ -702,83 +675,62 @@ __device__ __forceinline__ void add_pair_terms(const DevParams& p, const PairRec
   if (roll && om > 0.0) add_rolling(p, r, w, om, o, t);
 }
 
-// The records of the set bits of `mask` in ascending order; each record's
-// load is issued before the previous record is added.
-template <bool NBR, class Idx>
-__device__ __forceinline__ void add_flagged(const DevParams& p, unsigned mask, Idx idx,
-                                            const PairRec* __restrict__ prec, bool roll, double r,
-                                            const double w[3], double om, double f[3], double t[3]) {
-  if (!mask) return;
-  PairRec cur = prec[idx(__ffs(mask) - 1)];
-  mask &= mask - 1u;
-  while (true) {
-    const bool more = mask != 0u;
-    PairRec nxt;
-    if (more) {
-      nxt = prec[idx(__ffs(mask) - 1)];
-      mask &= mask - 1u;
-    }
-    add_pair_terms<NBR>(p, cur, roll, r, w, om, f, t);
-    if (!more) break;
-    cur = nxt;
-  }
+__device__ __forceinline__ PairRec load_record(const RecStore& rec, int cc, bool roll) {
+  PairRec r;
+  const double4 a = ld32(rec.main + 2 * (size_t)cc), b = ld32(rec.main + 2 * (size_t)cc + 1);
+  r.fc[0] = a.x; r.fc[1] = a.y; r.fc[2] = a.z;
+  r.tf[0] = a.w; r.tf[1] = b.x; r.tf[2] = b.y;
+  r.dcl2 = b.z; r.dci2 = b.w;
+  r.kn = 0.0; r.ov = 0.0;
+  if (roll) { const double2 q = rec.roll[cc]; r.kn = q.x; r.ov = q.y; }
+  return r;
 }
 
-// Incoming entries from q on (sorted by owner) whose owner is at most lim,
-// 32 at a time: the window's contact flags are read first (independent
-// loads), then the flagged records.  Returns the first entry not taken.
-__device__ __forceinline__ int add_incoming(const DevParams& p, int q, int ie, int lim,
-                                            const int2* __restrict__ in_pair, const uint8_t* __restrict__ pflag,
-                                            const PairRec* __restrict__ prec, bool roll, double r,
-                                            const double w[3], double om, double f[3], double t[3]) {
-  while (q < ie) {
-    const int cnt = min(32, ie - q);
-    unsigned mask = 0u;
-    int stop = cnt;
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-      if (k < cnt) {
-        const int2 e = in_pair[q + k];
-        if (e.x > lim && k < stop) stop = k;
-        if (pflag[e.y] & PF_CONTACT) mask |= 1u << k;
+// The records of the contacts among the entries [q, e) of the particle's
+// incoming list (NBR, pair indices in in_pair) or its own row, in order, 32
+// entries at a time: the contact flags, which lie in the entries' order, are
+// read as words, then the flagged records, each issued before the previous
+// one is added.
+template <bool NBR>
+__device__ __forceinline__ void add_range(const DevParams& p, int q, int e, const uint8_t* __restrict__ flags,
+                                          const int2* __restrict__ in_pair, const RecStore& rec, bool roll, double r,
+                                          const double w[3], double om, double f[3], double t[3]) {
+  for (int base = q; base < e; base += 32) {
+    unsigned mask = contact_mask(flags, base, min(32, e - base));
+    if (!mask) continue;
+    auto pair = [&](int k) { return NBR ? in_pair[base + k].y : base + k; };
+    PairRec cur = load_record(rec, pair(__ffs(mask) - 1), roll);
+    mask &= mask - 1u;
+    while (true) {
+      const bool more = mask != 0u;
+      PairRec nxt;
+      if (more) {
+        nxt = load_record(rec, pair(__ffs(mask) - 1), roll);
+        mask &= mask - 1u;
       }
+      add_pair_terms<NBR>(p, cur, roll, r, w, om, f, t);
+      if (!more) break;
+      cur = nxt;
     }
-    if (stop < 32) mask &= (1u << stop) - 1u;
-    const int base = q;
-    add_flagged<true>(p, mask, [&](int k) { return in_pair[base + k].y; }, prec, roll, r, w, om, f, t);
-    q += stop;
-    if (stop < cnt) break;
-  }
-  return q;
-}
-
-// The particle's own row [rs, re), 32 entries at a time.
-__device__ __forceinline__ void add_own(const DevParams& p, int rs, int re, const uint8_t* __restrict__ pflag,
-                                        const PairRec* __restrict__ prec, bool roll, double r, const double w[3],
-                                        double om, double f[3], double t[3]) {
-  for (int base = rs; base < re; base += 32) {
-    const int cnt = min(32, re - base);
-    unsigned mask = 0u;
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k)
-      if (k < cnt && (pflag[base + k] & PF_CONTACT)) mask |= 1u << k;
-    add_flagged<false>(p, mask, [&](int k) { return base + k; }, prec, roll, r, w, om, f, t);
   }
 }
 
 // Kernel 3 (per particle): sums FC/TOW in the serial reference's order --
 // wall terms, pairs owned by lower-index particles (ascending owner), the
-// particle's own row, pairs owned by higher-index particles -- and either
-// stores them (MODE 0) or integrates them in place of CFNEWVALUES
-// (MODE 1 = Euler, MODE 2 = Adams-Bashforth).
+// particle's own row, pairs owned by higher-index particles (in_mid is the
+// first of them; a NORMAL particle has none) -- and either stores them
+// (MODE 0) or integrates them in place of CFNEWVALUES (MODE 1 = Euler, MODE
+// 2 = Adams-Bashforth).
+// Same bed: 179 us with records read 8 bytes at a time and each incoming
+// pair's flag looked up at random, 125 us so.
 template <int MODE, bool B>
 __global__ void __launch_bounds__(256, 3)
 k_gather(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, const double4* __restrict__ vel_c,
          const double4* __restrict__ omg_c, double4* __restrict__ pos_n, double4* __restrict__ vel_n,
          double4* __restrict__ omg_n, const int8_t* __restrict__ state, const double* __restrict__ wf,
-         const int* __restrict__ row_end, const int* __restrict__ in_start, const int2* __restrict__ in_pair,
-         const uint8_t* __restrict__ pflag, uint8_t* __restrict__ touched, uint8_t* __restrict__ wall_hit,
-         const PairRec* __restrict__ prec,
+         const int* __restrict__ row_end, const int* __restrict__ in_start, const int* __restrict__ in_mid,
+         const int2* __restrict__ in_pair, const uint8_t* __restrict__ pflag, const uint8_t* __restrict__ in_flag,
+         uint8_t* __restrict__ touched, uint8_t* __restrict__ wall_hit, RecStore rec,
          double* __restrict__ fc, double* __restrict__ tow, double* __restrict__ acc_old,
          double* __restrict__ rot_acc_old, unsigned* __restrict__ vslot,
          CellOut cells) {
@@ -805,11 +757,10 @@ k_gather(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, const do
     const double r = pos_c[me].w;
     double om = 0.0;
     if (roll) om = sqrt(dot3(w, w));
-    const int rs = me ? row_end[me - 1] : 0, re = row_end[me];
-    const int is = in_start[me], ie = in_start[me + 1];
-    const int q = add_incoming(p, is, ie, me, in_pair, pflag, prec, roll, r, w, om, f, t);
-    add_own(p, rs, re, pflag, prec, roll, r, w, om, f, t);
-    add_incoming(p, q, ie, INT_MAX, in_pair, pflag, prec, roll, r, w, om, f, t);
+    const int is = in_start[me], ie = in_start[me + 1], mid = in_mid[me];
+    add_range<true>(p, is, mid, in_flag, in_pair, rec, roll, r, w, om, f, t);
+    add_range<false>(p, me ? row_end[me - 1] : 0, row_end[me], pflag, nullptr, rec, roll, r, w, om, f, t);
+    if (mid < ie) add_range<true>(p, mid, ie, in_flag, in_pair, rec, roll, r, w, om, f, t);
   }
   const double4 X = pos_c[me], V = vel_c[me];
   const double x[3] = {X.x, X.y, X.z}, v[3] = {V.x, V.y, V.z};
@@ -867,8 +818,9 @@ static void launch_pairs_t(dem_handle* h) {
   const int c = h->cur;
   const int T = h->tune.pair_threads;
   k_pairs<COLL, B><<<(unsigned)(h->n_sm * h->tune.pair_bpsm), T, 0, h->stream>>>(
-      h->dp, h->bview(), h->d_np, h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->pos4[c], h->vel4[c], h->omg4[c],
-      h->state, h->phase, h->pft[h->pcur], h->pflag(), h->touched, h->pgap, h->skin, h->prec, h->derr);
+      h->dp, h->bview(), h->d_np, h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c],
+      h->omg4[c], h->state, h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin,
+      h->recs(), h->derr);
   DEM_LAUNCH(h);
 }
 
@@ -877,8 +829,9 @@ static void launch_gather_t(dem_handle* h) {
   const int T = h->tune.gather_threads, G = (h->nl() + T - 1) / T;
   const int c = h->cur;
   k_gather<MODE, B><<<G, T, 0, h->stream>>>(h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
-                                            h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start, h->in_pair, h->pflag(),
-                                            h->touched, h->wall_hit, h->prec, h->fc, h->tow, h->acc_old,
+                                            h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start,
+                                            h->in_fill, h->in_pair, h->pflag(), h->in_flag, h->touched, h->wall_hit,
+                                            h->recs(), h->fc, h->tow, h->acc_old,
                                             h->rot_acc_old, h->vslot, gather_cells<MODE, B>(h));
   DEM_LAUNCH(h);
 }
@@ -1008,21 +961,22 @@ int run_split_force_error(dem_handle* h, double* rel_err) {
   if (!h->have_state || !h->have_pairs) return set_err(h, DEM_ERR_STATE, "state or pair list missing");
   const size_t n = h->n, cm = h->dp.cmax, P = (size_t)host_pairs(h);
   const size_t b_fid = sizeof(int) * cm * n, b_pft = sizeof(double) * 3 * cm * n;
-  const size_t b_hist = sizeof(double) * 3 * P;
+  const size_t b_hist = sizeof(double) * P;  // of one component's plane
   // both passes start from the same wall and pair histories (each pass
   // updates them in place)
-  char* snap = (char*)stage_buffer(h, b_fid + b_pft + n + b_hist + 2 * P + 64);
+  char* snap = (char*)stage_buffer(h, b_fid + b_pft + n + 3 * b_hist + 2 * P + 64);
   if (!snap) return set_err(h, DEM_ERR_CUDA, "cudaMalloc stage");
   char* s_live = snap + b_fid + b_pft;
   char* s_hist = s_live + n;
-  char* s_flag = s_hist + b_hist;
+  char* s_flag = s_hist + 3 * b_hist;
   char* s_inflag = s_flag + P;
   auto save = [&]() {
     cudaMemcpyAsync(snap, h->wall_fid, b_fid, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(snap + b_fid, h->wall_pft, b_pft, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(s_live, h->wall_live, n, cudaMemcpyDeviceToDevice, h->stream);
     if (P) {
-      cudaMemcpyAsync(s_hist, h->pft[h->pcur], b_hist, cudaMemcpyDeviceToDevice, h->stream);
+      for (int c = 0; c < 3; ++c)
+        cudaMemcpyAsync(s_hist + c * b_hist, h->pft[h->pcur] + c * h->pair_cap, b_hist, cudaMemcpyDeviceToDevice, h->stream);
       cudaMemcpyAsync(s_flag, h->pflag(), P, cudaMemcpyDeviceToDevice, h->stream);
       cudaMemcpyAsync(s_inflag, h->in_flag, P, cudaMemcpyDeviceToDevice, h->stream);
     }
@@ -1032,7 +986,8 @@ int run_split_force_error(dem_handle* h, double* rel_err) {
     cudaMemcpyAsync(h->wall_pft, snap + b_fid, b_pft, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(h->wall_live, s_live, n, cudaMemcpyDeviceToDevice, h->stream);
     if (P) {
-      cudaMemcpyAsync(h->pft[h->pcur], s_hist, b_hist, cudaMemcpyDeviceToDevice, h->stream);
+      for (int c = 0; c < 3; ++c)
+        cudaMemcpyAsync(h->pft[h->pcur] + c * h->pair_cap, s_hist + c * b_hist, b_hist, cudaMemcpyDeviceToDevice, h->stream);
       cudaMemcpyAsync(h->pflag(), s_flag, P, cudaMemcpyDeviceToDevice, h->stream);
       cudaMemcpyAsync(h->in_flag, s_inflag, P, cudaMemcpyDeviceToDevice, h->stream);
     }

@@ -812,32 +812,63 @@ __global__ void k_remap(DevParams p0, BatchView bv, const int* __restrict__ d_np
       const int so = ll ? old_end[ll - 1] : 0, eo = old_end[ll];
       for (int co = so; co < eo; ++co) {
         if (old_nbrs[co] == nb) {
-          a = old_pft[3 * (size_t)co]; b = old_pft[3 * (size_t)co + 1]; c = old_pft[3 * (size_t)co + 2];
+          a = old_pft[co]; b = old_pft[cap + co]; c = old_pft[2 * cap + co];
           break;
         }
       }
     }
-    pft[3 * cc] = a; pft[3 * cc + 1] = b; pft[3 * cc + 2] = c;
+    pft[cc] = a; pft[cap + cc] = b; pft[2 * cap + cc] = c;
     pflag[cc] = (a != 0.0 || b != 0.0 || c != 0.0) ? PF_HIST : 0;
     pgap[cc] = pair_gap<B>(p0, bv, ll, nb, pos4, state);
   }
 }
 
 // PF_HIST bits of a pair list whose history was set from the host.
-__global__ void k_hist_flags(const int* __restrict__ d_np, const double* __restrict__ pft,
+__global__ void k_hist_flags(const int* __restrict__ d_np, const double* __restrict__ pft, long long cap,
                              uint8_t* __restrict__ pflag) {
   const long long np = *d_np, stride = (long long)gridDim.x * blockDim.x;
   for (long long cc = (long long)blockIdx.x * blockDim.x + threadIdx.x; cc < np; cc += stride) {
-    const double* q = pft + 3 * cc;
-    pflag[cc] = (q[0] != 0.0 || q[1] != 0.0 || q[2] != 0.0) ? PF_HIST : 0;
+    pflag[cc] = (pft[cc] != 0.0 || pft[cap + cc] != 0.0 || pft[2 * cap + cc] != 0.0) ? PF_HIST : 0;
   }
 }
 
+// The history's planes to PFT_NEIGHBOR's (3,P) order and back.
+template <bool OUT>
+__global__ void k_history_order(long long count, long long cap, double* __restrict__ planes,
+                                double* __restrict__ triples) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= count) return;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (OUT) triples[3 * k + c] = planes[c * cap + k];
+    else planes[c * cap + k] = triples[3 * k + c];
+  }
+}
 
+int download_history(dem_handle* h, long long first, long long count, double* pf) {
+  double* st = (double*)stage_buffer(h, sizeof(double) * 3 * (size_t)count + 64);
+  if (!st) return set_err(h, DEM_ERR_CUDA, "cudaMalloc stage");
+  k_history_order<true><<<(unsigned)((count + 255) / 256), 256, 0, h->stream>>>(count, h->pair_cap,
+                                                                                h->pft[h->pcur] + first, st);
+  DEM_LAUNCH(h);
+  return check_cuda(h, cudaMemcpyAsync(pf, st, sizeof(double) * 3 * (size_t)count, cudaMemcpyDeviceToHost, h->stream),
+                    "download history");
+}
+
+int upload_history(dem_handle* h, long long count, const double* pf) {
+  double* st = (double*)stage_buffer(h, sizeof(double) * 3 * (size_t)count + 64);
+  if (!st) return set_err(h, DEM_ERR_CUDA, "cudaMalloc stage");
+  if (int rc = check_cuda(h, cudaMemcpyAsync(st, pf, sizeof(double) * 3 * (size_t)count, cudaMemcpyHostToDevice,
+                                             h->stream), "upload history")) return rc;
+  k_history_order<false><<<(unsigned)((count + 255) / 256), 256, 0, h->stream>>>(count, h->pair_cap, h->pft[h->pcur],
+                                                                                 st);
+  DEM_LAUNCH(h);
+  return check_cuda(h, cudaGetLastError(), "upload history");
+}
 
 void set_hist_flags(dem_handle* h) {
   const int T = 256;
-  k_hist_flags<<<pair_grid(h, T), T, 0, h->stream>>>(h->d_np, h->pft[h->pcur], h->pflag());
+  k_hist_flags<<<pair_grid(h, T), T, 0, h->stream>>>(h->d_np, h->pft[h->pcur], h->pair_cap, h->pflag());
   DEM_LAUNCH(h);
 }
 
@@ -869,12 +900,13 @@ __global__ void k_in_fill(const int* __restrict__ d_np, const int* __restrict__ 
 // incoming pairs of each particle in ascending pair index (= owner order);
 // each pair's slot in the list (in_pos) and a cleared contact flag of the
 // slot (in_flag: no pair of a new list is in contact before its first force
-// pass)
+// pass); and the first slot whose owner has a higher index (in_mid)
 __global__ void k_in_sort(int n, const int* __restrict__ in_start, int2* __restrict__ in_pair,
-                          int* __restrict__ in_pos, uint8_t* __restrict__ in_flag) {
+                          int* __restrict__ in_pos, uint8_t* __restrict__ in_flag, int* __restrict__ in_mid) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const int s = in_start[j], e = in_start[j + 1], m = e - s;
+  int below = 0;  // entries owned by lower-index particles: they come first
   constexpr int R = 16;  // lists up to R long are sorted in registers
   if (m <= R) {
     // each entry goes to the place given by the number of smaller pair
@@ -888,11 +920,13 @@ __global__ void k_in_sort(int n, const int* __restrict__ in_start, int2* __restr
         int r = 0;
 #pragma unroll
         for (int d = 0; d < R; ++d) r += v[d].y < v[c].y;
+        below += v[c].x <= j;
         in_pair[s + r] = v[c];
         in_pos[v[c].y] = s + r;
         in_flag[s + r] = 0;
       }
     }
+    in_mid[j] = s + below;
     return;
   }
   for (int a = s + 1; a < e; ++a) {
@@ -902,9 +936,11 @@ __global__ void k_in_sort(int n, const int* __restrict__ in_start, int2* __restr
     in_pair[b + 1] = v;
   }
   for (int a = s; a < e; ++a) {
+    below += in_pair[a].x <= j;
     in_pos[in_pair[a].y] = a;
     in_flag[a] = 0;
   }
+  in_mid[j] = s + below;
 }
 
 // Transpose of the current list (buffer nb, pair count in d_np): incoming
@@ -920,7 +956,7 @@ int build_transpose(dem_handle* h, int nb) {
   if (int rc = check_cuda(h, cudaMemsetAsync(h->in_fill, 0, sizeof(int) * n, h->stream), "memset")) return rc;
   k_in_fill<<<BP, T, 0, h->stream>>>(h->d_np, h->nbrs[nb], h->pair_owner, h->in_start, h->in_fill, h->in_pair);
   DEM_LAUNCH(h);
-  k_in_sort<<<B, T, 0, h->stream>>>(n, h->in_start, h->in_pair, h->in_pos, h->in_flag);
+  k_in_sort<<<B, T, 0, h->stream>>>(n, h->in_start, h->in_pair, h->in_pos, h->in_flag, h->in_fill);
   DEM_LAUNCH(h);
   return check_cuda(h, cudaGetLastError(), "transpose");
 }
@@ -954,7 +990,7 @@ int ensure_pair_capacity(dem_handle* h, long long need) {
   long long cap = h->pair_cap > 0 ? h->pair_cap : need;
   while (cap < need) cap *= 2;
   const long long old = h->pair_cap;  // the whole old allocation (the count may be stale)
-  int* nb[2]; double* pf[2]; int2* inp; int* own; uint8_t* pfl[2]; PairRec* prc; float* gap;
+  int* nb[2]; double* pf[2]; int2* inp; int* own; uint8_t* pfl[2]; void* prc; float* gap;
   int* ipos; uint8_t* ifl;
   for (int b = 0; b < 2; ++b) {
     if (int rc = check_cuda(h, cudaMalloc(&nb[b], sizeof(int) * cap), "cudaMalloc nbrs")) return rc;
@@ -971,7 +1007,9 @@ int ensure_pair_capacity(dem_handle* h, long long need) {
   if (old > 0) {
     // keep the current list and history (the rebuild reads them)
     cudaMemcpyAsync(nb[h->rb], h->nbrs[h->rb], sizeof(int) * old, cudaMemcpyDeviceToDevice, h->stream);
-    cudaMemcpyAsync(pf[h->pcur], h->pft[h->pcur], sizeof(double) * 3 * old, cudaMemcpyDeviceToDevice, h->stream);
+    for (int c = 0; c < 3; ++c)
+      cudaMemcpyAsync(pf[h->pcur] + c * cap, h->pft[h->pcur] + c * old, sizeof(double) * old, cudaMemcpyDeviceToDevice,
+                      h->stream);
     cudaMemcpyAsync(inp, h->in_pair, sizeof(int2) * old, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(own, h->pair_owner, sizeof(int) * old, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(pfl[h->pcur], h->pflag(), old, cudaMemcpyDeviceToDevice, h->stream);

@@ -63,7 +63,9 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   char* snap = (char*)stage_buffer(h, sizeof(double) * 3 * P + 2 * P + 64);
   if (!snap) return set_err(h, DEM_ERR_CUDA, "cudaMalloc stage");
   if (P) {
-    cudaMemcpyAsync(snap, h->pft[h->pcur], sizeof(double) * 3 * P, cudaMemcpyDeviceToDevice, h->stream);
+    for (size_t c = 0; c < 3; ++c)
+      cudaMemcpyAsync(snap + sizeof(double) * c * P, h->pft[h->pcur] + c * h->pair_cap, sizeof(double) * P,
+                      cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(snap + sizeof(double) * 3 * P, h->pflag(), P, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(snap + sizeof(double) * 3 * P + P, h->in_flag, P, cudaMemcpyDeviceToDevice, h->stream);
   }
@@ -97,7 +99,9 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   }
   h->tune = best;
   if (P) {
-    cudaMemcpyAsync(h->pft[h->pcur], snap, sizeof(double) * 3 * P, cudaMemcpyDeviceToDevice, h->stream);
+    for (size_t c = 0; c < 3; ++c)
+      cudaMemcpyAsync(h->pft[h->pcur] + c * h->pair_cap, snap + sizeof(double) * c * P, sizeof(double) * P,
+                      cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(h->pflag(), snap + sizeof(double) * 3 * P, P, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(h->in_flag, snap + sizeof(double) * 3 * P + P, P, cudaMemcpyDeviceToDevice, h->stream);
   }

@@ -1,0 +1,55 @@
+"""Sizes at which the kernels of a step change their way of working, against
+the oracle.
+
+- the pair kernels take windows of 128 pairs, a lane screening four of them:
+  pair counts at and around multiples of both.
+
+FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
+the split path is held to the tolerances of its own tests (positions 1e-6,
+velocities 1e-3 of the largest).
+"""
+import numpy as np
+import pytest
+
+from cases import state_arrays
+from gpu_util import compare_pairs, compare_state, pair_both, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(m, precision, nsn=10):
+    """m + 1 spheres of 1 mm in a row along x, 0.98 d apart: m pairs, each in
+    contact at the start, with small seeded velocities across the row."""
+    from mfix_dem import params as P
+    d, n = 1e-3, m + 1
+    rng = np.random.default_rng(300 + m)
+    pos = np.empty((3, n))
+    pos[0] = (np.arange(n) + 2.0) * 0.98 * d
+    pos[1] = pos[2] = 4.0 * d
+    vel = rng.uniform(-0.02, 0.02, (3, n))
+    arr = state_arrays(pos, vel, np.zeros((3, n)), np.full(n, 0.5 * d), np.full(n, 2500.0))
+    hi = ((n + 4.0) * d, 8.0 * d, 8.0 * d)
+    case = P.DemCase(d_p0=(d,), ro_s0=(2500.0,), coll_model="LSD", kn=1000.0, kn_w=1000.0, des_en_input=0.9,
+                     des_en_wall_input=[0.9], mew=0.2, mew_w=0.2, mew_r=0.01, mew_rw=0.01, domain_hi=hi,
+                     neighbor_search_n=nsn, force_precision=precision)
+    prm, _ = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
+    return prm, arr, P.default_walls((0.0, 0.0, 0.0), hi)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 127, 128, 129, 255, 385])
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+def test_pair_windows(m, prec):
+    from mfix_dem import abi
+    g, o = pair_both(*_chain(m, abi.DEM_PREC_SPLIT if prec == "split" else abi.DEM_PREC_FP64))
+    assert g.pair_count() == m
+    for steps in (1, 2, 30):
+        g.step(steps)
+        o.step(steps)
+        if prec == "fp64":
+            compare_state(g, o, exact=True)
+            compare_pairs(g, o)
+            assert g.stats()["n_contacts"] == o.stats()["n_contacts"]
+    if prec == "split":
+        sg, so = g.download_state(), o.download_state()
+        assert rel_err(sg["pos"], so["pos"]) <= 1e-6
+        assert rel_err(sg["vel"], so["vel"]) <= 1e-3
