@@ -334,7 +334,6 @@ struct dem_handle {
   double* wall_pft = nullptr; // [i][cmax][3]
   uint8_t* wall_live = nullptr; // [i] 1 when some wall slot may be in use
   uint8_t* wall_cand = nullptr; // [i] 1 when the particle's DES cell holds facets
-  int* wall_list = nullptr;     // this step's particles with wall work (arbitrary order)
   float* wgap = nullptr;        // [i] clearance from the facets of its DES cell at the last build
   // outflow boundaries (single handles): host copy, device copy, the
   // FIRST_PASS of UPDATE_EXIT_DES_VEL
@@ -359,7 +358,6 @@ struct dem_handle {
   void* d_seed = nullptr;
   int seed_cap = 0;
   long long inflow_added = 0;
-  int* d_nwall = nullptr;       // their count
   double* wf = nullptr;       // [i][6] wall force and torque of the last force pass (valid with wall_hit)
 
   // scan scratch
@@ -479,9 +477,7 @@ void handle_arrays(dem_handle* h, size_t n, size_t nc, size_t nfc, F&& A) {
   A((void**)&h->touched, n);
   A((void**)&h->wall_hit, n);
   A((void**)&h->wall_cand, n);
-  A((void**)&h->wall_list, sizeof(int) * n);
   A((void**)&h->wgap, sizeof(float) * n);
-  A((void**)&h->d_nwall, sizeof(int));
   A((void**)&h->skin, sizeof(double));
   A((void**)&h->vslot, sizeof(unsigned) * 32);
   A((void**)&h->derr, sizeof(DevErr));

@@ -224,118 +224,164 @@ __device__ __forceinline__ int get_collision(const DevParams& p, const WallCtx& 
   return free_index;
 }
 
-// The wall contacts of one particle in a cell with facets.  `live` says
-// whether any of its history slots may be in use; when none is, no slot is
-// searched for the facets it does not touch (REMOVE_COLLISION would find
-// nothing).  The particle's velocity, spin, mass and phase are read at its
-// first contact only.
+// The wall contacts of one particle in a cell with facets, by a group of
+// WALL_LANES lanes (mask gm, lane gl of the group).  A cell of a triangulated
+// wall holds tens of facets and a particle touches one or two of them, so the
+// lanes test the cell's facets side by side (extent, plane and closest point:
+// a chain of loads and FP64 arithmetic each) and the few that matter are then
+// taken in the facets' order, as the reference's loop does: the history slots
+// (GET/REMOVE_COLLISION choose and free slots in that order) and the sums of
+// the force and torque terms.  `live` says whether any history slot may be in
+// use; when none is, no slot is searched for the facets it does not touch
+// (REMOVE_COLLISION would find nothing).  The particle's velocity, spin, mass
+// and phase are read by the lanes in contact only.  f and t are the same in
+// every lane; returns the number of contacts.
+// Five hoppers of 160,000 spheres in all (a triangulated cone, 128 facets):
+// 143 us per step with a thread per particle, of it 99 us this, and 68 us so.
+constexpr int WALL_LANES = 8;
 template <int COLL>
-__device__ void wall_contacts(const DevParams& p, const WallCtx& w, int me, PState& s, bool live,
-                              const double4* __restrict__ vel4, const double4* __restrict__ omg4,
-                              const uint8_t* __restrict__ phase, double f[3], double t[3],
-                              unsigned long long& nwc, unsigned& eflags) {
+__device__ int wall_contacts(const DevParams& p, const WallCtx& w, int me, const double x[3], double r, bool live,
+                             unsigned gm, int gl, const double4* __restrict__ vel4,
+                             const double4* __restrict__ omg4, const uint8_t* __restrict__ phase, double f[3],
+                             double t[3], unsigned& eflags) {
   const int cell = p.cell_off + w.dg_pijk[me] - 1;
   const int fs = w.fbin_start[cell], fe = w.fbin_start[cell + 1];
-  bool have_kin = false;
-  const double r = s.r;
+  const int g0 = __ffs(gm) - 1;  // the group's first lane in the warp
   const double radsq = r * r;
-  double pmax[3], pmin[3];
+  int nwc = 0;
+  for (int q0 = fs; q0 < fe; q0 += WALL_LANES) {
+    const int q = q0 + gl;
+    enum { NONE, MISS, HIT };
+    int what = NONE, nf = -1;
+    double dist[3] = {0.0, 0.0, 0.0}, distsq = 0.0;
+    if (q < fe) {
+      const FacetBinEntry e = w.fbin[q];
+      nf = e.id;
+      what = MISS;
+      const double xd = x[e.dir];
+      if (!(e.mn > xd + r) && !(e.mx < xd - r)) {
+        const double* V = w.vertex + 9 * (size_t)nf;
+        const double* N = w.norm_face + 3 * (size_t)nf;
+        double d1[3] = {V[0] - x[0], V[1] - x[1], V[2] - x[2]};
+        double nn[3] = {N[0], N[1], N[2]};
+        const double line_t = dot3(d1, nn);
+        if (!(line_t <= -1.0001 * r)) {
+          double cpt[3]; bool poe; int edge;
+          closest_pt(p, w, nf, x, cpt, poe, edge);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) { pmax[c] = s.x[c] + r; pmin[c] = s.x[c] - r; }
-  for (int q = fs; q < fe; ++q) {
-    const FacetBinEntry e = w.fbin[q];
-    const int nf = e.id;
-    if (e.mn > pmax[e.dir]) { if (live) remove_collision(p, w, me, nf); continue; }
-    if (e.mx < pmin[e.dir]) { if (live) remove_collision(p, w, me, nf); continue; }
-    const double* V = w.vertex + 9 * (size_t)nf;
-    const double* N = w.norm_face + 3 * (size_t)nf;
-    double d1[3] = {V[0] - s.x[0], V[1] - s.x[1], V[2] - s.x[2]};
-    double nn[3] = {N[0], N[1], N[2]};
-    const double line_t = dot3(d1, nn);
-    if (line_t <= -1.0001 * r) { if (live) remove_collision(p, w, me, nf); continue; }
-    double cpt[3]; bool poe; int edge;
-    closest_pt(p, w, nf, s.x, cpt, poe, edge);
-    double dist[3] = {cpt[0] - s.x[0], cpt[1] - s.x[1], cpt[2] - s.x[2]};
-    const double distsq = dot3(dist, dist);
-    if (distsq >= radsq - SMALL_NUMBER) { if (live) remove_collision(p, w, me, nf); continue; }
-    if (poe && w.ignore_edge[4 * (size_t)nf + edge]) continue;
-    if (!have_kin) {
-      const double4 b = vel4[me], c = omg4[me];
-      s.v[0] = b.x; s.v[1] = b.y; s.v[2] = b.z; s.m = b.w;
-      s.w[0] = c.x; s.w[1] = c.y; s.w[2] = c.z;
-      s.ph = phase[me];
-      have_kin = true;
-    }
-    const double distmod = sqrt(distsq);
-    double nrm[3] = {dist[0], dist[1], dist[2]};
-    if (distsq > 0) { const double sq = sqrt(distsq); for (int c = 0; c < 3; ++c) nrm[c] = dist[c] / sq; }
-    const double overlap_n = r - distmod;
-    double wxn[3]; cross3(s.w, nrm, wxn);
-    double vrel[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { vrel[c] = s.v[c] + distmod * wxn[c]; vrel[c] = vrel[c] - (0.0 + 0.0); }
-    const double vrn = dot3(vrel, nrm);
-    double vt[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) vt[c] = vrel[c] - vrn * nrm[c];
-    double kn_w, kt_w, etan_w, etat_w;
-    const int ph = s.ph;
-    if (COLL == DEM_COLL_HERTZ) {
-      double so = 0.0;
-      if (overlap_n > 0) so = sqrt(overlap_n);
-      kn_w = p.hkwn[ph] * so * sqrt(r);
-      kt_w = p.hkwt[ph] * so * sqrt(r);
-      etan_w = p.etanw[ph] * sqrt(so) * sqrt(p.hkwn[ph] * sqrt(r) * s.m);
-      etat_w = p.etatw[ph] * sqrt(so) * sqrt(p.hkwt[ph] * sqrt(r) * s.m);
-    } else {
-      kn_w = p.kn_w; kt_w = p.kt_w;
-      etan_w = p.etanw[ph] * sqrt(s.m);
-      etat_w = p.etatw[ph] * sqrt(s.m);
-    }
-    double fn[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) fn[c] = -(kn_w * overlap_n * nrm[c] + etan_w * vrn * nrm[c]);
-    double hist[3];
-    const int slot = get_collision(p, w, me, nf, cell, hist);
-    if (slot < 0) { eflags |= EF_WALL_SLOTS; continue; }
-    double ot[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) ot[c] = p.dt * vt[c] + hist[c];
-    const double mag = sqrt(dot3(ot, ot));
-    double ft[3];
-    if (mag > 0.0) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) ft[c] = -kt_w * ot[c] - etat_w * vt[c];
-      const double ftmd = sqrt(dot3(ft, ft));
-      const double fnmd = p.mew_w * sqrt(dot3(fn, fn));
-      if (ftmd > fnmd) {
-        double tg[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) tg[c] = ot[c] / mag;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ft[c] = -fnmd * tg[c];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ot[c] = (fnmd / kt_w) * tg[c];
+          for (int c = 0; c < 3; ++c) dist[c] = cpt[c] - x[c];
+          distsq = dot3(dist, dist);
+          if (!(distsq >= radsq - SMALL_NUMBER))
+            what = (poe && w.ignore_edge[4 * (size_t)nf + edge]) ? NONE : HIT;
+        }
       }
-    } else {
-      ft[0] = ft[1] = ft[2] = 0.0;
     }
-    double* wp = w.wall_pft + ((size_t)me * p.cmax + slot) * 3;  // UPDATE_COLLISION
-    wp[0] = ot[0]; wp[1] = ot[1]; wp[2] = ot[2];
-    ++nwc;
+    const unsigned hits = (__ballot_sync(gm, what == HIT) & gm) >> g0;
+    unsigned gone = 0;  // facets not touched that a history slot still holds
+    if (live) {
+      bool held = false;
+      if (what == MISS) {
+        const int* fid = w.wall_fid + (size_t)me * p.cmax;
+        for (int s = 0; s < p.cmax; ++s) held = held || fid[s] == nf;
+      }
+      gone = (__ballot_sync(gm, held) & gm) >> g0;
+    }
+    int slot = -1;
+    double hist[3] = {0.0, 0.0, 0.0};
+    for (unsigned todo = hits | gone; todo; todo &= todo - 1u) {
+      if (gl == __ffs(todo) - 1) {
+        if (what == HIT) slot = get_collision(p, w, me, nf, cell, hist);
+        else remove_collision(p, w, me, nf);
+      }
+      __syncwarp(gm);  // the next facet sees the slots as this one left them
+    }
+    if (!hits) continue;
+    double fn[3] = {0.0, 0.0, 0.0}, ft[3] = {0.0, 0.0, 0.0}, tq[3] = {0.0, 0.0, 0.0}, rl[3] = {0.0, 0.0, 0.0};
+    int terms = 0;  // 1: force and torque, 2: rolling friction too
+    if (what == HIT && slot < 0) eflags |= EF_WALL_SLOTS;
+    if (slot >= 0) {
+      const double4 vb = vel4[me], wb = omg4[me];
+      const double sv[3] = {vb.x, vb.y, vb.z}, sw[3] = {wb.x, wb.y, wb.z}, m = vb.w;
+      const int ph = phase[me];
+      const double distmod = sqrt(distsq);
+      double nrm[3] = {dist[0], dist[1], dist[2]};
+      if (distsq > 0) { const double sq = sqrt(distsq); for (int c = 0; c < 3; ++c) nrm[c] = dist[c] / sq; }
+      const double overlap_n = r - distmod;
+      double wxn[3]; cross3(sw, nrm, wxn);
+      double vrel[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) f[c] = f[c] + fn[c] + ft[c];
-    double nxf[3]; cross3(nrm, ft, nxf);
+      for (int c = 0; c < 3; ++c) { vrel[c] = sv[c] + distmod * wxn[c]; vrel[c] = vrel[c] - (0.0 + 0.0); }
+      const double vrn = dot3(vrel, nrm);
+      double vt[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) t[c] = t[c] + distmod * nxf[c];
-    if (p.mew_rw > 0.0) {
-      const double om = sqrt(dot3(s.w, s.w));
-      if (om > 0.0) {
+      for (int c = 0; c < 3; ++c) vt[c] = vrel[c] - vrn * nrm[c];
+      double kn_w, kt_w, etan_w, etat_w;
+      if (COLL == DEM_COLL_HERTZ) {
+        double so = 0.0;
+        if (overlap_n > 0) so = sqrt(overlap_n);
+        kn_w = p.hkwn[ph] * so * sqrt(r);
+        kt_w = p.hkwt[ph] * so * sqrt(r);
+        etan_w = p.etanw[ph] * sqrt(so) * sqrt(p.hkwn[ph] * sqrt(r) * m);
+        etat_w = p.etatw[ph] * sqrt(so) * sqrt(p.hkwt[ph] * sqrt(r) * m);
+      } else {
+        kn_w = p.kn_w; kt_w = p.kt_w;
+        etan_w = p.etanw[ph] * sqrt(m);
+        etat_w = p.etatw[ph] * sqrt(m);
+      }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) t[c] = t[c] + -(p.mew_rw * (2.0 * r) * kn_w * overlap_n * s.w[c] / om);
+      for (int c = 0; c < 3; ++c) fn[c] = -(kn_w * overlap_n * nrm[c] + etan_w * vrn * nrm[c]);
+      double ot[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ot[c] = p.dt * vt[c] + hist[c];
+      const double mag = sqrt(dot3(ot, ot));
+      if (mag > 0.0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ft[c] = -kt_w * ot[c] - etat_w * vt[c];
+        const double ftmd = sqrt(dot3(ft, ft));
+        const double fnmd = p.mew_w * sqrt(dot3(fn, fn));
+        if (ftmd > fnmd) {
+          double tg[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) tg[c] = ot[c] / mag;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) ft[c] = -fnmd * tg[c];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) ot[c] = (fnmd / kt_w) * tg[c];
+        }
+      }
+      double* wp = w.wall_pft + ((size_t)me * p.cmax + slot) * 3;  // UPDATE_COLLISION
+      wp[0] = ot[0]; wp[1] = ot[1]; wp[2] = ot[2];
+      double nxf[3]; cross3(nrm, ft, nxf);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) tq[c] = distmod * nxf[c];
+      terms = 1;
+      if (p.mew_rw > 0.0) {
+        const double om = sqrt(dot3(sw, sw));
+        if (om > 0.0) {
+          terms = 2;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) rl[c] = -(p.mew_rw * (2.0 * r) * kn_w * overlap_n * sw[c] / om);
+        }
+      }
+    }
+    for (unsigned todo = hits; todo; todo &= todo - 1u) {
+      const int b = g0 + __ffs(todo) - 1;
+      const int have = __shfl_sync(gm, terms, b);
+      if (!have) continue;
+      ++nwc;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double a = __shfl_sync(gm, fn[c], b), d = __shfl_sync(gm, ft[c], b), e = __shfl_sync(gm, tq[c], b);
+        f[c] = f[c] + a + d;
+        t[c] = t[c] + e;
+      }
+      if (have == 2) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] = t[c] + __shfl_sync(gm, rl[c], b);
       }
     }
   }
+  return nwc;
 }
 
 // ---------------------------------------------------------------------------
@@ -414,135 +460,108 @@ __global__ void k_wall_gaps(DevParams p0, BatchView bv, WallCtx w, const double4
   wgap[i] = __double2float_rd(sqrt(dmin2) - a.w - 1e-6 * a.w);
 }
 
-// The particles with wall work this step: NORMAL particles whose DES cell
-// holds facets and whose clearance at the last build does not exceed the
-// displacement bound since, and NORMAL particles whose history slots may be
-// in use (k_walls clears them, or updates them).  A thread screens four
-// consecutive particles: their flags arrive in one 32-bit load per array and
-// their clearances in one float4, all issued before any is used, so the
-// kernel waits on memory about once.  Each block of WALL_LIST_T threads
-// appends its particles in index order with one atomic; blocks land in
-// arbitrary order, which does not matter: each particle's wall terms depend
-// on it alone.
-constexpr int WALL_LIST_T = 1024;
-static_assert(WALL_LIST_T == 32 * 32, "one warp scans the warp counts");
+// Kernel 1: wall contacts.  A block screens WALL_T * J particles for those
+// with wall work this step -- NORMAL particles whose DES cell holds facets and
+// whose clearance at the last build does not exceed the displacement bound
+// since, and NORMAL particles whose history slots may be in use -- into a list
+// in shared memory, and its groups of WALL_LANES lanes take the listed
+// particles.  A particle's wall force and torque, the first terms of FC/TOW in
+// the reference's order (CALC_DEM_FORCE_WITH_WALL_STL runs before the pair
+// loop, calc_force_dem.f:113), go to wf; they depend on that particle alone,
+// so the order of the list does not matter.  With J = 4 a thread's four flags
+// arrive in one 32-bit load per array and its clearances in one float4.
+constexpr int WALL_T = 256;
 __device__ __forceinline__ unsigned wall_need(unsigned st, unsigned live, unsigned cand, float gap, double bound) {
   return (st == (unsigned)(uint8_t)DEM_STATE_NORMAL && (live || (cand && !((double)gap > bound)))) ? 1u : 0u;
 }
-__global__ void __launch_bounds__(WALL_LIST_T)
-k_wall_list(int n, const int8_t* __restrict__ state, const uint8_t* __restrict__ wall_cand,
-            const uint8_t* __restrict__ wall_live, const float* __restrict__ wgap, const double* __restrict__ skin,
-            int* __restrict__ list, int* __restrict__ count) {
-  __shared__ int warp_n[WALL_LIST_T / 32];
-  const int i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+template <int COLL, bool B, int J>
+__global__ void __launch_bounds__(WALL_T)
+k_walls(DevParams p0, BatchView bv, WallCtx w, int n, const int8_t* __restrict__ state,
+        const float* __restrict__ wgap, const double* __restrict__ skin, const double4* __restrict__ pos4,
+        const double4* __restrict__ vel4, const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
+        uint8_t* __restrict__ wall_live, const uint8_t* __restrict__ wall_cand, double* __restrict__ wf,
+        uint8_t* __restrict__ wall_hit, DevErr* __restrict__ err) {
+  static_assert(J == 1 || J == 4, "one particle per thread, or four");
+  __shared__ int s_list[WALL_T * J];
+  __shared__ int s_n;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  const int i0 = J * (blockIdx.x * WALL_T + threadIdx.x);
   const double bound = *skin;
-  uint32_t st = 0, lv = 0, cd = 0;
-  float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (i0 + 3 < n) {  // the arrays are separate allocations: 256-byte aligned
-    st = *reinterpret_cast<const uint32_t*>(state + i0);
-    lv = *reinterpret_cast<const uint32_t*>(wall_live + i0);
-    cd = *reinterpret_cast<const uint32_t*>(wall_cand + i0);
-    g = *reinterpret_cast<const float4*>(wgap + i0);
+  unsigned need = 0;  // bit j: particle i0+j has wall work
+  if (J == 4 && i0 + 3 < n) {  // the arrays are separate allocations: 256-byte aligned
+    const uint32_t st = *reinterpret_cast<const uint32_t*>(state + i0);
+    const uint32_t lv = *reinterpret_cast<const uint32_t*>(wall_live + i0);
+    const uint32_t cd = *reinterpret_cast<const uint32_t*>(wall_cand + i0);
+    const float4 g = *reinterpret_cast<const float4*>(wgap + i0);
+    need = wall_need(st & 255u, lv & 255u, cd & 255u, g.x, bound) |
+           (wall_need((st >> 8) & 255u, (lv >> 8) & 255u, (cd >> 8) & 255u, g.y, bound) << 1) |
+           (wall_need((st >> 16) & 255u, (lv >> 16) & 255u, (cd >> 16) & 255u, g.z, bound) << 2) |
+           (wall_need(st >> 24, lv >> 24, cd >> 24, g.w, bound) << 3);
   } else {
-    float gg[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (i0 + j < n) {
-        st |= (uint32_t)(uint8_t)state[i0 + j] << (8 * j);
-        lv |= (uint32_t)wall_live[i0 + j] << (8 * j);
-        cd |= (uint32_t)wall_cand[i0 + j] << (8 * j);
-        gg[j] = wgap[i0 + j];
-      }
-    g = make_float4(gg[0], gg[1], gg[2], gg[3]);
+    for (int j = 0; j < J; ++j)
+      if (i0 + j < n)
+        need |= wall_need((uint8_t)state[i0 + j], wall_live[i0 + j], wall_cand[i0 + j], wgap[i0 + j], bound) << j;
   }
-  // bit j: particle i0+j has wall work (bytes past n are zero: state 0 is
-  // not NORMAL)
-  const unsigned need = wall_need(st & 255u, lv & 255u, cd & 255u, g.x, bound) |
-                        (wall_need((st >> 8) & 255u, (lv >> 8) & 255u, (cd >> 8) & 255u, g.y, bound) << 1) |
-                        (wall_need((st >> 16) & 255u, (lv >> 16) & 255u, (cd >> 16) & 255u, g.z, bound) << 2) |
-                        (wall_need(st >> 24, lv >> 24, cd >> 24, g.w, bound) << 3);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int mine = __popc(need);
   int incl = mine;  // inclusive scan of the counts over the warp
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
   }
-  if (lane == 31) warp_n[warp] = incl;
+  int base = 0;
+  if (lane == 31 && incl) base = atomicAdd(&s_n, incl);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  int at = base + incl - mine;
+  for (int j = 0; j < J; ++j)
+    if ((need >> j) & 1u) s_list[at++] = i0 + j;
   __syncthreads();
-  if (warp == 0) {  // the warps' offsets: a scan of their counts, and one atomic
-    const int c = warp_n[lane];
-    int wi = c;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, wi, o);
-      if (lane >= o) wi += y;
-    }
-    const int tot = __shfl_sync(0xffffffffu, wi, 31);
-    int base = 0;
-    if (lane == 0 && tot) base = atomicAdd(count, tot);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    warp_n[lane] = base + wi - c;
-  }
-  __syncthreads();
-  int at = warp_n[warp] + incl - mine;
-  for (int j = 0; j < 4; ++j)
-    if ((need >> j) & 1u) list[at++] = i0 + j;
-}
-
-// Kernel 1 (per listed particle): wall contacts of NORMAL particles whose DES
-// cell holds facets.  Writes the particle's wall force and torque, which are
-// the first terms of FC/TOW in the reference's order
-// (CALC_DEM_FORCE_WITH_WALL_STL runs before the pair loop,
-// calc_force_dem.f:113).  Persistent grid over the list built by k_wall_list.
-template <int COLL, bool B>
-__global__ void __launch_bounds__(128)
-k_walls(DevParams p0, BatchView bv, WallCtx w, const int* __restrict__ wlist, const int* __restrict__ wcount,
-        const double4* __restrict__ pos4, const double4* __restrict__ vel4,
-        const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
-        uint8_t* __restrict__ wall_live, const uint8_t* __restrict__ wall_cand, double* __restrict__ wf,
-        uint8_t* __restrict__ wall_hit, DevErr* __restrict__ err) {
-  const int nw = *wcount;
+  const int nw = s_n;
   unsigned long long nwc = 0;
   unsigned eflags = 0;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nw; q += gridDim.x * blockDim.x) {
-    const int me = wlist[q];
+  const int gl = lane & (WALL_LANES - 1);
+  const unsigned gm = ((1u << WALL_LANES) - 1u) << (lane & ~(WALL_LANES - 1));
+  for (int k = threadIdx.x / WALL_LANES; k < nw; k += WALL_T / WALL_LANES) {
+    const int me = s_list[k];
     const DevParams& p = sysp<B>(p0, bv, me);
     if (!wall_cand[me]) {
       // no facet near: clear the history once (calc_collision_wall_mod.f:194-198)
       int* fid = w.wall_fid + (size_t)me * p.cmax;
       double* wp = w.wall_pft + (size_t)me * p.cmax * 3;
-      for (int s = 0; s < p.cmax; ++s) fid[s] = -1;
-      for (int s = 0; s < 3 * p.cmax; ++s) wp[s] = 0.0;
-      wall_live[me] = 0;
+      for (int s = gl; s < p.cmax; s += WALL_LANES) fid[s] = -1;
+      for (int s = gl; s < 3 * p.cmax; s += WALL_LANES) wp[s] = 0.0;
+      if (gl == 0) wall_live[me] = 0;
       continue;
     }
-    PState S;
     const double4 a = pos4[me];
-    S.x[0] = a.x; S.x[1] = a.y; S.x[2] = a.z; S.r = a.w;
+    const double x[3] = {a.x, a.y, a.z};
     double f[3] = {0.0, 0.0, 0.0}, t[3] = {0.0, 0.0, 0.0};
     const bool live = wall_live[me] != 0;
-    const unsigned long long nwc0 = nwc;
-    wall_contacts<COLL>(p, w, me, S, live, vel4, omg4, phase, f, t, nwc, eflags);
-    const bool hit = nwc > nwc0;
-    bool used = hit;
-    if (!hit && live) {
-      const int* fid = w.wall_fid + (size_t)me * p.cmax;
-      for (int s = 0; s < p.cmax; ++s) used = used || fid[s] != -1;
-    }
-    if (used != live) wall_live[me] = used ? 1 : 0;
-    if (hit) {
-      // the wall terms are the first terms of FC/TOW; the gather reads
-      // them only for particles marked here
-      double* o = wf + 6 * (size_t)me;
-      o[0] = f[0]; o[1] = f[1]; o[2] = f[2]; o[3] = t[0]; o[4] = t[1]; o[5] = t[2];
-      wall_hit[me] = 1;
+    const int hit = wall_contacts<COLL>(p, w, me, x, a.w, live, gm, gl, vel4, omg4, phase, f, t, eflags);
+    if (gl == 0) {
+      nwc += hit;
+      bool used = hit > 0;
+      if (!hit && live) {
+        const int* fid = w.wall_fid + (size_t)me * p.cmax;
+        for (int s = 0; s < p.cmax; ++s) used = used || fid[s] != -1;
+      }
+      if (used != live) wall_live[me] = used ? 1 : 0;
+      if (hit) {
+        // the gather reads the wall terms only for particles marked here
+        double* o = wf + 6 * (size_t)me;
+        o[0] = f[0]; o[1] = f[1]; o[2] = f[2]; o[3] = t[0]; o[4] = t[1]; o[5] = t[2];
+        wall_hit[me] = 1;
+      }
     }
   }
+  __syncwarp();
   for (int o = 16; o > 0; o >>= 1) {
     nwc += __shfl_down_sync(0xffffffffu, nwc, o);
     eflags |= __shfl_down_sync(0xffffffffu, eflags, o);
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     if (nwc) atomicAdd(&err->n_wall_contacts, nwc);
     if (eflags) atomicOr(&err->flags, eflags);
   }
@@ -798,19 +817,20 @@ static WallCtx wall_ctx(dem_handle* h) {
   return w;
 }
 
+// Particles screened per thread: one while that fills the device once (more
+// blocks then share the listed particles), four past it, where the screening
+// of the others is what the kernel does.
 template <int COLL, bool B>
 static void launch_walls_t(dem_handle* h) {
-  const int c = h->cur;
-  const int T = 128;
-  cudaMemsetAsync(h->d_nwall, 0, sizeof(int), h->stream);
-  const int nq = (h->nl() + 3) / 4;  // four particles per thread
-  k_wall_list<<<(nq + WALL_LIST_T - 1) / WALL_LIST_T, WALL_LIST_T, 0, h->stream>>>(
-      h->nl(), h->state, h->wall_cand, h->wall_live, h->wgap, h->skin, h->wall_list, h->d_nwall);
-  // persistent: the resident blocks of the kernel's register budget
-  k_walls<COLL, B><<<h->n_sm * 4, T, 0, h->stream>>>(h->dp, h->bview(), wall_ctx(h), h->wall_list, h->d_nwall,
-                                                     h->pos4[c], h->vel4[c], h->omg4[c], h->phase, h->wall_live,
-                                                     h->wall_cand, h->wf, h->wall_hit, h->derr);
-  h->launches += 2;
+  const int c = h->cur, n = h->nl();
+  auto go = [&](auto kernel, int per) {
+    kernel<<<(n + WALL_T * per - 1) / (WALL_T * per), WALL_T, 0, h->stream>>>(
+        h->dp, h->bview(), wall_ctx(h), n, h->state, h->wgap, h->skin, h->pos4[c], h->vel4[c], h->omg4[c], h->phase,
+        h->wall_live, h->wall_cand, h->wf, h->wall_hit, h->derr);
+  };
+  if (n <= h->n_sm * 2 * WALL_T) go(k_walls<COLL, B, 1>, 1);
+  else go(k_walls<COLL, B, 4>, 4);
+  DEM_LAUNCH(h);
 }
 
 template <int COLL, bool B>

@@ -2,7 +2,10 @@
 the oracle.
 
 - the pair kernels take windows of 128 pairs, a lane screening four of them:
-  pair counts at and around multiples of both.
+  pair counts at and around multiples of both;
+- the wall work takes one particle per thread up to two blocks per
+  multiprocessor and four past that: bed sizes on both sides, with the counts
+  not a multiple of four.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -11,7 +14,7 @@ velocities 1e-3 of the largest).
 import numpy as np
 import pytest
 
-from cases import state_arrays
+from cases import settling_case, state_arrays
 from gpu_util import compare_pairs, compare_state, pair_both, rel_err
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +56,21 @@ def test_pair_windows(m, prec):
         sg, so = g.download_state(), o.download_state()
         assert rel_err(sg["pos"], so["pos"]) <= 1e-6
         assert rel_err(sg["vel"], so["vel"]) <= 1e-3
+
+
+@pytest.mark.parametrize("n_side", [(43, 41, 42), (43, 41, 43), (45, 41, 43)])
+def test_wall_work_by_size(n_side):
+    """74,045, 75,808 and 79,334 spheres: one per thread up to 75,776 (148
+    multiprocessors); the outer layers start at or in the walls."""
+    box = tuple(0.999e-3 * k for k in n_side)
+    case, prm, arr, walls = settling_case(n_side=n_side, box=box, spacing=0.999, jitter=0.01, vmax=0.2, nsn=5, seed=61)
+    arr = {k: (v[..., :-1].copy() if v.ndim else v) for k, v in arr.items()}   # a count that is no multiple of four
+    g, o = pair_both(prm, arr, walls)
+    g.step(17)
+    o.step(17)
+    compare_state(g, o, exact=True)
+    assert g.stats()["n_wall_contacts"] == o.stats()["n_wall_contacts"] > 1000
+    fg, pg = g.download_wall_history()
+    fo, po = o.download_wall_history()
+    assert np.array_equal(fg, fo)
+    assert np.array_equal(pg[fg >= 0], po[fo >= 0])
