@@ -437,7 +437,6 @@ static int batch_step_once(dem_handle* h, std::vector<uint8_t>& last_due) {
       if (int rc = upload_table(h, s)) return rc;
     }
   }
-  cudaMemsetAsync(&h->derr->n_contacts, 0, 2 * sizeof(unsigned long long), h->stream);
   if (int rc = run_force(h, true)) return rc;
   std::vector<uint8_t> m;
   const bool any_due = due_mask(h, m, nullptr);
@@ -490,7 +489,6 @@ static bool period_aligned(const dem_handle* h, int* nsn) {
 }
 
 static int graph_step(dem_handle* h, bool rebuild, bool anyper) {
-  cudaMemsetAsync(&h->derr->n_contacts, 0, 2 * sizeof(unsigned long long), h->stream);
   if (int rc = run_force(h, true)) return rc;
   if (rebuild || anyper) {
     const size_t S = h->sys.size();
@@ -509,6 +507,7 @@ static int batch_replay_period(dem_handle* h, int N) {
     if (int rc = ensure_pair_capacity(h, 2 * P + 1024)) return rc;
     invalidate_graphs(h);
   }
+  if (h->count_dirty) clear_counts(h);  // a captured step relies on the gather before it
   bool anyper = false;
   for (const SysSlot& S : h->sys)
     if (S.live) anyper = anyper || S.dp.per[0] || S.dp.per[1] || (S.dp.per[2] && !S.dp.no_k);
@@ -527,6 +526,7 @@ static int batch_replay_period(dem_handle* h, int N) {
     if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "sync")) return rc;
     cudaGraph_t graph;
     h->capturing = true;
+    h->joined = true;  // nothing comes before the first node
     if (int rc = check_cuda(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture")) {
       h->capturing = false;
       return rc;
@@ -551,7 +551,7 @@ static int batch_replay_period(dem_handle* h, int N) {
   }
   if (int rc = check_cuda(h, cudaGraphLaunch(h->graphs[key], h->stream), "graph launch")) return rc;
   h->launches += h->graph_kernels[key];
-  for (int j = 0; j < N; ++j) h->cur = 1 - h->cur;
+  for (int j = 0; j < N; ++j) { h->count_set = h->cur; h->cur = 1 - h->cur; }
   h->pcur = 1 - h->pcur;
   h->rb = 1 - h->rb;
   h->np_stale = true;

@@ -209,7 +209,7 @@ int upload_range(dem_handle* h, int off, int cnt, int nph, const double* pos, co
       cudaMemcpyAsync(st + 9 * n + n * a, scal[a], sizeof(double) * n, cudaMemcpyHostToDevice, h->stream);
       k_pack<<<B, T, 0, h->stream>>>(cnt, st + 3 * n * a, st + 9 * n + n * a, dst[a]);
     } else if (a == 0 && note_moves && !state) {
-      k_pack_moved<<<B, T, 0, h->stream>>>(cnt, st, dst[0], h->state + off, h->vslot);
+      k_pack_moved<<<B, T, 0, h->stream>>>(cnt, st, dst[0], h->state + off, h->vslot_note());
     } else {
       k_pack_keepw<<<B, T, 0, h->stream>>>(cnt, st + 3 * n * a, dst[a]);
     }
@@ -759,7 +759,6 @@ int dem_init_neighbors(dem_handle* h) {
 int dem_calc_force(dem_handle* h) {
   SINGLE_GUARD(h);
   if (!h->have_state || !h->have_pairs) return set_err(h, DEM_ERR_STATE, "state or pair list missing");
-  cudaMemsetAsync(&h->derr->n_contacts, 0, 2 * sizeof(unsigned long long), h->stream);
   if (int rc = run_force(h, false)) return rc;
   return fetch_errors(h);
 }
@@ -777,7 +776,6 @@ int dem_cfnewvalues(dem_handle* h) {
 static int step_once(dem_handle* h, int nn) {
   const DevParams& p = h->dp;
   const bool anyper = p.per[0] || p.per[1] || (p.per[2] && !p.no_k);
-  cudaMemsetAsync(&h->derr->n_contacts, 0, 2 * sizeof(unsigned long long), h->stream);
   bool force = false;
   if (h->obc.empty()) {
     if (int rc = run_force(h, true)) return rc;
@@ -815,10 +813,12 @@ static int replay_period(dem_handle* h, int nn0) {
     if (int rc = ensure_pair_capacity(h, 2 * P + 1024)) return rc;
     invalidate_graphs(h);
   }
+  if (h->count_dirty) clear_counts(h);  // a captured step relies on the gather before it
   const int key = (h->cur << 2) | (h->pcur << 1) | h->rb;
   if (!h->graphs[key]) {
     cudaGraph_t graph;
     h->capturing = true;
+    h->joined = true;  // nothing comes before the first node
     if (int rc = check_cuda(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture")) {
       h->capturing = false;
       return rc;
@@ -850,6 +850,7 @@ static int replay_period(dem_handle* h, int nn0) {
   // buffer parities and bookkeeping after the period: N force passes flip
   // the state buffers, the rebuild flips the list and history buffers
   for (int j = 0; j < nsn; ++j) {
+    h->count_set = h->cur;
     h->cur = 1 - h->cur;
     h->s_time = h->s_time + h->prm.dtsolid;
     h->steps_done++;
@@ -896,8 +897,8 @@ int dem_get_stats(dem_handle* h, dem_stats* s) {
   cudaMemcpyAsync(h->herr, h->derr, sizeof(DevErr), cudaMemcpyDeviceToHost, h->stream);
   if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "stats")) return rc;
   s->n_pairs = host_pairs(h);
-  s->n_contacts = (int64_t)h->herr->n_contacts;
-  s->n_wall_contacts = (int64_t)h->herr->n_wall_contacts;
+  s->n_contacts = (int64_t)h->herr->count[h->count_set].pairs;
+  s->n_wall_contacts = (int64_t)h->herr->count[h->count_set].walls;
   s->n_rogue_removed = (int64_t)h->herr->rogue_removed;
   s->n_outflow_removed = (int64_t)h->herr->outflow_removed;
   s->n_inflow_added = (int64_t)h->inflow_added;
@@ -952,8 +953,8 @@ int dem_get_stats_noalloc(dem_handle* h, dem_stats* s) {
   s->n_normal = (int64_t)nn;
   for (int c = 0; c < 3; ++c) { s->mean_vel[c] = mv[c]; s->gran_temp[c] = nn > 0 ? gt[c] / nn : 0.0; }
   s->n_pairs = host_pairs(h);
-  s->n_contacts = (int64_t)h->herr->n_contacts;
-  s->n_wall_contacts = (int64_t)h->herr->n_wall_contacts;
+  s->n_contacts = (int64_t)h->herr->count[h->count_set].pairs;
+  s->n_wall_contacts = (int64_t)h->herr->count[h->count_set].walls;
   s->n_rogue_removed = (int64_t)h->herr->rogue_removed;
   s->n_outflow_removed = (int64_t)h->herr->outflow_removed;
   s->n_inflow_added = (int64_t)h->inflow_added;

@@ -837,7 +837,6 @@ int dem_step_coupled(dem_handle* h, int32_t nn_first, int32_t nsteps) {
   const bool anyper = p.per[0] || p.per[1] || (p.per[2] && !p.no_k);
   for (int k = 0; k < nsteps; ++k) {
     const int nn = nn_first + k;
-    cudaMemsetAsync(&h->derr->n_contacts, 0, 2 * sizeof(unsigned long long), h->stream);
     if (int rc = run_force(h, false)) return rc;              // CALC_FORCE_DEM
     if (int rc = run_calc_drag(h)) return rc;                 // CALC_DRAG_DES
     bool force = false;

@@ -460,7 +460,7 @@ __global__ void k_wall_gaps(DevParams p0, BatchView bv, WallCtx w, const double4
   wgap[i] = __double2float_rd(sqrt(dmin2) - a.w - 1e-6 * a.w);
 }
 
-// Kernel 1: wall contacts.  A block screens WALL_T * J particles for those
+// Kernel 1: wall contacts.  A block screens blockDim.x * J particles for those
 // with wall work this step -- NORMAL particles whose DES cell holds facets and
 // whose clearance at the last build does not exceed the displacement bound
 // since, and NORMAL particles whose history slots may be in use -- into a list
@@ -474,20 +474,33 @@ constexpr int WALL_T = 256;
 __device__ __forceinline__ unsigned wall_need(unsigned st, unsigned live, unsigned cand, float gap, double bound) {
   return (st == (unsigned)(uint8_t)DEM_STATE_NORMAL && (live || (cand && !((double)gap > bound)))) ? 1u : 0u;
 }
+struct WallArgs {
+  WallCtx w;
+  int n;       // particles
+  int blocks;  // blocks that do the wall work
+  const float* __restrict__ wgap;
+  uint8_t* __restrict__ live;
+  const uint8_t* __restrict__ cand;
+  double* __restrict__ wf;
+  uint8_t* __restrict__ hit;
+};
 template <int COLL, bool B, int J>
-__global__ void __launch_bounds__(WALL_T)
-k_walls(DevParams p0, BatchView bv, WallCtx w, int n, const int8_t* __restrict__ state,
-        const float* __restrict__ wgap, const double* __restrict__ skin, const double4* __restrict__ pos4,
-        const double4* __restrict__ vel4, const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
-        uint8_t* __restrict__ wall_live, const uint8_t* __restrict__ wall_cand, double* __restrict__ wf,
-        uint8_t* __restrict__ wall_hit, DevErr* __restrict__ err) {
+__device__ __forceinline__ void wall_block(const DevParams& p0, const BatchView& bv, const WallArgs& wa, int block,
+                                           double bound, const int8_t* __restrict__ state,
+                                           const double4* __restrict__ pos4, const double4* __restrict__ vel4,
+                                           const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
+                                           ContactCount* __restrict__ count, DevErr* __restrict__ err) {
   static_assert(J == 1 || J == 4, "one particle per thread, or four");
+  const WallCtx& w = wa.w;
+  const int n = wa.n;
+  const float* __restrict__ wgap = wa.wgap;
+  uint8_t* __restrict__ wall_live = wa.live;
+  const uint8_t* __restrict__ wall_cand = wa.cand;
   __shared__ int s_list[WALL_T * J];
   __shared__ int s_n;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
-  const int i0 = J * (blockIdx.x * WALL_T + threadIdx.x);
-  const double bound = *skin;
+  const int i0 = J * (block * (int)blockDim.x + (int)threadIdx.x);
   unsigned need = 0;  // bit j: particle i0+j has wall work
   if (J == 4 && i0 + 3 < n) {  // the arrays are separate allocations: 256-byte aligned
     const uint32_t st = *reinterpret_cast<const uint32_t*>(state + i0);
@@ -523,7 +536,7 @@ k_walls(DevParams p0, BatchView bv, WallCtx w, int n, const int8_t* __restrict__
   unsigned eflags = 0;
   const int gl = lane & (WALL_LANES - 1);
   const unsigned gm = ((1u << WALL_LANES) - 1u) << (lane & ~(WALL_LANES - 1));
-  for (int k = threadIdx.x / WALL_LANES; k < nw; k += WALL_T / WALL_LANES) {
+  for (int k = threadIdx.x / WALL_LANES; k < nw; k += blockDim.x / WALL_LANES) {
     const int me = s_list[k];
     const DevParams& p = sysp<B>(p0, bv, me);
     if (!wall_cand[me]) {
@@ -550,9 +563,9 @@ k_walls(DevParams p0, BatchView bv, WallCtx w, int n, const int8_t* __restrict__
       if (used != live) wall_live[me] = used ? 1 : 0;
       if (hit) {
         // the gather reads the wall terms only for particles marked here
-        double* o = wf + 6 * (size_t)me;
+        double* o = wa.wf + 6 * (size_t)me;
         o[0] = f[0]; o[1] = f[1]; o[2] = f[2]; o[3] = t[0]; o[4] = t[1]; o[5] = t[2];
-        wall_hit[me] = 1;
+        wa.hit[me] = 1;
       }
     }
   }
@@ -562,9 +575,19 @@ k_walls(DevParams p0, BatchView bv, WallCtx w, int n, const int8_t* __restrict__
     eflags |= __shfl_down_sync(0xffffffffu, eflags, o);
   }
   if (lane == 0) {
-    if (nwc) atomicAdd(&err->n_wall_contacts, nwc);
+    if (nwc) atomicAdd(&count->walls, nwc);
     if (eflags) atomicOr(&err->flags, eflags);
   }
+}
+
+template <int COLL, bool B, int J>
+__global__ void __launch_bounds__(WALL_T)
+k_walls(DevParams p0, BatchView bv, WallArgs wa, const double* __restrict__ skin,
+        const unsigned* __restrict__ pending, const int8_t* __restrict__ state, const double4* __restrict__ pos4,
+        const double4* __restrict__ vel4, const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
+        ContactCount* __restrict__ count, DevErr* __restrict__ err) {
+  wall_block<COLL, B, J>(p0, bv, wa, blockIdx.x, displacement_bound(skin, pending), state, pos4, vel4, omg4, phase,
+                         count, err);
 }
 
 // Kernel 2 (per pair): one CC iteration of CALC_FORCE_DEM, evaluated once
@@ -582,25 +605,42 @@ k_walls(DevParams p0, BatchView bv, WallCtx w, int n, const int8_t* __restrict__
 // its throughput).  The 1,000,000-sphere bed with 1.67 M of its 4.4 M pairs in contact:
 // 248 us with four pairs per thread (12 of 32 lanes in contact at a time) and
 // records written 8 bytes at a time, 156 us so.
-template <int COLL, bool B>
+// With JW > 0 the first wa.blocks blocks do the wall work instead (JW
+// particles per thread): it reads the same state and writes disjoint arrays,
+// and in one launch the two run side by side with no second stream to fork
+// and join.
+template <int COLL, bool B, int JW>
 __global__ void __launch_bounds__(256, 2)
-k_pairs(DevParams p0, BatchView bv, const int* __restrict__ d_np, long long cap, const int* __restrict__ owner,
+k_pairs(DevParams p0, BatchView bv, WallArgs wa, const int* __restrict__ d_np, long long cap, const int* __restrict__ owner,
         const int* __restrict__ nbrs, const int* __restrict__ in_pos, const double4* __restrict__ pos4,
         const double4* __restrict__ vel4, const double4* __restrict__ omg4, const int8_t* __restrict__ state,
         const uint8_t* __restrict__ phase, double* __restrict__ pft, uint8_t* __restrict__ pflag,
         uint8_t* __restrict__ in_flag, uint8_t* __restrict__ touched, const float* __restrict__ pgap,
-        const double* __restrict__ skin, RecStore rec, DevErr* __restrict__ err) {
+        const double* __restrict__ skin, const unsigned* __restrict__ pending, RecStore rec,
+        ContactCount* __restrict__ count, DevErr* __restrict__ err) {
   __shared__ uint16_t s_queue[256 / 32][WIN_PAIRS];
+  const int z = pdl_wait();
+  pdl_next();
+  const double bound = displacement_bound(skin + z, pending + z);
+  int block = blockIdx.x + z, blocks = gridDim.x;
+  if (JW) {
+    if (block < wa.blocks) {
+      wall_block<COLL, B, JW ? JW : 1>(p0, bv, wa, block, bound, state, pos4, vel4, omg4, phase, count, err);
+      return;
+    }
+    block -= wa.blocks;
+    blocks -= wa.blocks;
+  }
   // persistent grid-stride loop over the device-side pair count (the grid
   // size does not depend on the list, so the launch can live in a graph)
-  const long long np = min((long long)*d_np, cap);
-  const float reach = __double2float_ru(2.0 * skin[0]);
+  const long long np = min((long long)d_np[z], cap);
+  const float reach = __double2float_ru(2.0 * bound);
   unsigned long long ncont = 0;
   unsigned eflags = 0;
   uint16_t* queue = s_queue[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)WIN_PAIRS * ((gridDim.x * blockDim.x) >> 5);
-  for (long long w0 = (long long)WIN_PAIRS * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w0 < np; w0 += stride) {
+  const long long stride = (long long)WIN_PAIRS * ((blocks * (int)blockDim.x) >> 5);
+  for (long long w0 = (long long)WIN_PAIRS * ((block * (int)blockDim.x + (int)threadIdx.x) >> 5) + z; w0 < np; w0 += stride) {
     const int nq = screen_window(w0, np, pflag, in_flag, in_pos, pgap, reach, queue);
     for (int k = lane; k < nq; k += 32) {
       const int e = queue[k];
@@ -669,7 +709,7 @@ k_pairs(DevParams p0, BatchView bv, const int* __restrict__ d_np, long long cap,
     eflags |= __shfl_down_sync(0xffffffffu, eflags, o);
   }
   if (lane == 0) {
-    if (ncont) atomicAdd(&err->n_contacts, ncont);
+    if (ncont) atomicAdd(&count->pairs, ncont);
     if (eflags) atomicOr(&err->flags, eflags);
   }
 }
@@ -752,8 +792,11 @@ k_gather(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, const do
          uint8_t* __restrict__ touched, uint8_t* __restrict__ wall_hit, RecStore rec,
          double* __restrict__ fc, double* __restrict__ tow, double* __restrict__ acc_old,
          double* __restrict__ rot_acc_old, unsigned* __restrict__ vslot,
-         CellOut cells) {
-  const int me = blockIdx.x * blockDim.x + threadIdx.x;
+         CellOut cells, StepEnd end) {
+  const int z = pdl_wait();
+  pdl_next();
+  if (MODE != 0) end_step(end);
+  const int me = blockIdx.x * blockDim.x + threadIdx.x + z;
   if (me >= p0.n) return;
   const DevParams& p = sysp<B>(p0, bv, me);
   const int8_t st = state[me];
@@ -820,40 +863,56 @@ static WallCtx wall_ctx(dem_handle* h) {
 // Particles screened per thread: one while that fills the device once (more
 // blocks then share the listed particles), four past it, where the screening
 // of the others is what the kernel does.
+static bool wall_single(const dem_handle* h) { return h->nl() <= h->n_sm * 2 * WALL_T; }
+static WallArgs wall_args(dem_handle* h, int threads) {
+  const int per = threads * (wall_single(h) ? 1 : 4);
+  WallArgs a;
+  a.w = wall_ctx(h);
+  a.n = h->nl();
+  a.blocks = (h->nl() + per - 1) / per;
+  a.wgap = h->wgap; a.live = h->wall_live; a.cand = h->wall_cand;
+  a.wf = h->wf; a.hit = h->wall_hit;
+  return a;
+}
+
 template <int COLL, bool B>
 static void launch_walls_t(dem_handle* h) {
-  const int c = h->cur, n = h->nl();
-  auto go = [&](auto kernel, int per) {
-    kernel<<<(n + WALL_T * per - 1) / (WALL_T * per), WALL_T, 0, h->stream>>>(
-        h->dp, h->bview(), wall_ctx(h), n, h->state, h->wgap, h->skin, h->pos4[c], h->vel4[c], h->omg4[c], h->phase,
-        h->wall_live, h->wall_cand, h->wf, h->wall_hit, h->derr);
+  const int c = h->cur;
+  const WallArgs wa = wall_args(h, WALL_T);
+  auto go = [&](auto kernel) {
+    kernel<<<wa.blocks, WALL_T, 0, h->stream>>>(h->dp, h->bview(), wa, h->skin, h->vslot_pending(), h->state,
+                                                h->pos4[c], h->vel4[c], h->omg4[c], h->phase, &h->derr->count[c],
+                                                h->derr);
   };
-  if (n <= h->n_sm * 2 * WALL_T) go(k_walls<COLL, B, 1>, 1);
-  else go(k_walls<COLL, B, 4>, 4);
+  if (wall_single(h)) go(k_walls<COLL, B, 1>);
+  else go(k_walls<COLL, B, 4>);
   DEM_LAUNCH(h);
 }
 
 template <int COLL, bool B>
-static void launch_pairs_t(dem_handle* h) {
+static void launch_pairs_t(dem_handle* h, bool walls) {
   const int c = h->cur;
   const int T = h->tune.pair_threads;
-  k_pairs<COLL, B><<<(unsigned)(h->n_sm * h->tune.pair_bpsm), T, 0, h->stream>>>(
-      h->dp, h->bview(), h->d_np, h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c],
-      h->omg4[c], h->state, h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin,
-      h->recs(), h->derr);
-  DEM_LAUNCH(h);
+  const WallArgs wa = wall_args(h, T);
+  auto go = [&](auto kernel) {
+    launch_pdl(h, kernel, (unsigned)(h->n_sm * h->tune.pair_bpsm + (walls ? wa.blocks : 0)), T, h->dp, h->bview(), wa,
+               h->d_np, h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c], h->omg4[c],
+               h->state, h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin,
+               h->vslot_pending(), h->recs(), &h->derr->count[c], h->derr);
+  };
+  if (!walls) go(k_pairs<COLL, B, 0>);
+  else if (wall_single(h)) go(k_pairs<COLL, B, 1>);
+  else go(k_pairs<COLL, B, 4>);
 }
 
 template <int MODE, bool B>
 static void launch_gather_t(dem_handle* h) {
   const int T = h->tune.gather_threads, G = (h->nl() + T - 1) / T;
   const int c = h->cur;
-  k_gather<MODE, B><<<G, T, 0, h->stream>>>(h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
-                                            h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start,
-                                            h->in_fill, h->in_pair, h->pflag(), h->in_flag, h->touched, h->wall_hit,
-                                            h->recs(), h->fc, h->tow, h->acc_old,
-                                            h->rot_acc_old, h->vslot, gather_cells<MODE, B>(h));
-  DEM_LAUNCH(h);
+  launch_pdl(h, k_gather<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
+             h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start, h->in_fill, h->in_pair,
+             h->pflag(), h->in_flag, h->touched, h->wall_hit, h->recs(), h->fc, h->tow, h->acc_old, h->rot_acc_old,
+             h->vslot_note(), gather_cells<MODE, B>(h), step_end(h));
 }
 
 void launch_wall_gaps(dem_handle* h) {
@@ -876,9 +935,9 @@ static void launch_walls(dem_handle* h) {
 }
 
 template <bool B>
-static void launch_pairs_fp64(dem_handle* h) {
-  if (h->dp.coll == DEM_COLL_HERTZ) launch_pairs_t<DEM_COLL_HERTZ, B>(h);
-  else launch_pairs_t<DEM_COLL_LSD, B>(h);
+static void launch_pairs_fp64(dem_handle* h, bool walls) {
+  if (h->dp.coll == DEM_COLL_HERTZ) launch_pairs_t<DEM_COLL_HERTZ, B>(h, walls);
+  else launch_pairs_t<DEM_COLL_LSD, B>(h, walls);
 }
 
 template <bool B>
@@ -891,12 +950,12 @@ static void launch_gather_fp64(dem_handle* h, int mode) {
 // The two timed parts of the force step for the autotuner.
 void launch_pairs_only(dem_handle* h) {
   if (h->dp.prec == DEM_PREC_SPLIT) launch_pairs_split(h);
-  else if (h->batch()) launch_pairs_fp64<true>(h);
-  else launch_pairs_fp64<false>(h);
+  else if (h->batch()) launch_pairs_fp64<true>(h, false);
+  else launch_pairs_fp64<false>(h, false);
 }
 
 void launch_gather_only(dem_handle* h) {
-  if (h->dp.prec == DEM_PREC_SPLIT) launch_gather_split(h, 0);
+  if (h->dp.prec == DEM_PREC_SPLIT) launch_gather_split(h, 0, false);
   else if (h->batch()) launch_gather_fp64<true>(h, 0);
   else launch_gather_fp64<false>(h, 0);
 }
@@ -905,13 +964,16 @@ void launch_gather_only(dem_handle* h) {
 // Euler/AB2 integration into the other state buffer.  The collision model,
 // integrator and force precision are common to all systems of a batch.
 static void launch_force_kernels(dem_handle* h, int mode, bool split) {
-  // The wall kernels and the pair kernel read the same state and write
-  // disjoint arrays (walls: wall_hit, wf and the wall histories; pairs: the
-  // pair histories, flags, records and touched marks), so the wall work runs
-  // on the side stream beside the pair kernel and the gather waits for both
-  // (in a captured step, two branches of the graph).  With the parts of the
-  // step timed (profiling), they run one after the other.
-  const bool side = h->nf > 0 && h->side_stream && !h->prof;
+  // The wall work and the pair kernel read the same state and write disjoint
+  // arrays (walls: wall_hit, wf and the wall histories; pairs: the pair
+  // histories, flags, records and touched marks).  In FP64 they are one
+  // launch; the split pair kernel is built with other arithmetic options and
+  // half the registers, so its wall work runs on the side stream beside it and
+  // the gather waits for both (in a captured step, two branches of the
+  // graph).  With the parts of the step timed (profiling), they run one after
+  // the other.
+  const bool walls = h->nf > 0, merged = walls && !split && !h->prof;
+  const bool side = walls && split && h->side_stream && !h->prof;
   if (side) {
     cudaEventRecord(h->ev_fork, h->stream);
     cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0);
@@ -920,38 +982,45 @@ static void launch_force_kernels(dem_handle* h, int mode, bool split) {
     launch_walls(h);
     h->stream = main;
     cudaEventRecord(h->ev_join, h->side_stream);
-  } else {
+  } else if (!merged) {
     ProfScope ps(h, DEM_PROF_WALLS);
     launch_walls(h);
   }
   {
     ProfScope ps(h, DEM_PROF_PAIRS);
     if (split) launch_pairs_split(h);
-    else if (h->batch()) launch_pairs_fp64<true>(h);
-    else launch_pairs_fp64<false>(h);
+    else if (h->batch()) launch_pairs_fp64<true>(h, merged);
+    else launch_pairs_fp64<false>(h, merged);
   }
-  if (side) cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+  if (side) {
+    cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+    h->joined = true;
+  }
   ProfScope ps(h, DEM_PROF_GATHER);
-  if (split) launch_gather_split(h, mode);
+  if (split) launch_gather_split(h, mode, side);
   else if (h->batch()) launch_gather_fp64<true>(h, mode);
   else launch_gather_fp64<false>(h, mode);
 }
 
-// Displacement bound since the last build += this step's largest particle
-// displacement bound; the slots are cleared for the next step.
-__global__ void k_skin(double* __restrict__ skin, unsigned* __restrict__ vslot, CandState* __restrict__ cand) {
-  const unsigned m = __reduce_max_sync(0xffffffffu, vslot[threadIdx.x]);
-  vslot[threadIdx.x] = 0;
-  if (threadIdx.x == 0) {
-    skin[0] = skin[0] + (double)__uint_as_float(m);
-    if (cand) cand->disp = cand->disp + (double)__uint_as_float(m);  // the candidate list's bound too
-  }
+// The noted displacements join the bound since the last build: the pending
+// set first, then the moves noted since (an upload's, or an integration
+// outside the gather).
+__global__ void k_skin(double* __restrict__ skin, unsigned* __restrict__ pending, unsigned* __restrict__ noted,
+                       CandState* __restrict__ cand) {
+  add_displacement(skin, cand, pending);
+  add_displacement(skin, cand, noted);
+}
+
+void clear_counts(dem_handle* h) {
+  cudaMemsetAsync(h->derr->count, 0, sizeof h->derr->count, h->stream);
+  h->joined = true;
+  h->count_dirty = false;
 }
 
 __global__ void k_set_skin(double* __restrict__ skin, double v) { skin[0] = v; }
 
 void launch_skin(dem_handle* h) {
-  k_skin<<<1, 32, 0, h->stream>>>(h->skin, h->vslot, h->cand);
+  k_skin<<<1, 32, 0, h->stream>>>(h->skin, h->vslot_pending(), h->vslot_note(), h->cand);
   DEM_LAUNCH(h);
 }
 
@@ -966,8 +1035,12 @@ int run_force(dem_handle* h, bool fused) {
   ProfScope ps(h, DEM_PROF_FORCE);
   h->dp.first_pass = h->first_pass ? 1 : 0;
   const int mode = !fused ? 0 : (h->dp.intg == DEM_INTG_AB2 ? 2 : 1);
+  // the counts of this pass start at zero: the last integrating gather
+  // cleared them, or a pass that did not integrate has left its own
+  if (!fused || h->count_dirty) clear_counts(h);
   launch_force_kernels(h, mode, h->dp.prec == DEM_PREC_SPLIT);
-  if (fused) launch_skin(h);
+  h->count_set = h->cur;
+  h->count_dirty = !fused;
   if (int rc = check_cuda(h, cudaGetLastError(), "force kernels")) return rc;
   if (fused) { h->cur = 1 - h->cur; h->first_pass = false; }
   return 0;
@@ -1014,6 +1087,7 @@ int run_split_force_error(dem_handle* h, double* rel_err) {
   };
   std::vector<double> f64(3 * n), f32(3 * n);
   h->dp.first_pass = 0;
+  h->count_dirty = true;  // the counts of the two passes stay
   save();
   launch_force_kernels(h, 0, false);
   cudaMemcpyAsync(f64.data(), h->fc, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream);
@@ -1036,7 +1110,7 @@ static void launch_integrate_t(dem_handle* h) {
   const int T = 256, G = (h->nl() + T - 1) / T;
   const int c = h->cur;
   k_integrate<INTG, B><<<G, T, 0, h->stream>>>(h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->state,
-                                               h->fc, h->tow, h->acc_old, h->rot_acc_old, h->vslot);
+                                               h->fc, h->tow, h->acc_old, h->rot_acc_old, h->vslot_note());
   DEM_LAUNCH(h);
 }
 

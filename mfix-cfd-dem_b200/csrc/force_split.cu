@@ -56,6 +56,19 @@ struct PairTerms {
   bool near;  // the FP32 onset-of-slip test lies within 1e-4 of its threshold
 };
 
+// x_I - x_L of the nearest image and its square.
+__device__ __forceinline__ double separation(const DevParams& p, const double4& a, const double4& b, double dist[3]) {
+  const double xl[3] = {a.x, a.y, a.z}, xi[3] = {b.x, b.y, b.z};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    double pj = xi[c];
+    const double s = periodic_shift(p, c, pj - xl[c]);
+    if (s != 0.0) pj = pj + s;
+    dist[c] = pj - xl[c];
+  }
+  return dist[0] * dist[0] + dist[1] * dist[1] + dist[2] * dist[2];
+}
+
 // The onset-of-slip test of calc_force_dem.f:330-337 in FP64, evaluated as
 // the FP64 kernels do (contact_force), for owner state (xl, vl, wl) and
 // neighbour state (xi, vi, wi) with dist = x_I - x_L and history pin.  The
@@ -241,19 +254,22 @@ k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long lon
               const double4* __restrict__ vel4, const double4* __restrict__ omg4, const int8_t* __restrict__ state,
               const uint8_t* __restrict__ phase, double* __restrict__ pft, uint8_t* __restrict__ pflag,
               uint8_t* __restrict__ in_flag, uint8_t* __restrict__ touched, const float* __restrict__ pgap,
-              const double* __restrict__ skin, Rec32* __restrict__ rec_own, Rec32* __restrict__ rec_in,
-              SlipFix* __restrict__ fix, DevErr* __restrict__ err) {
+              const double* __restrict__ skin, const unsigned* __restrict__ pending, Rec32* __restrict__ rec_own,
+              Rec32* __restrict__ rec_in,
+              SlipFix* __restrict__ fix, ContactCount* __restrict__ count, DevErr* __restrict__ err) {
   __shared__ uint16_t s_queue[256 / 32][WIN_PAIRS];
-  const long long np = min((long long)*d_np, cap);
+  const int z = pdl_wait();
+  pdl_next();
+  const long long np = min((long long)d_np[z], cap);
   // the bound in FP32, rounded up: a pair is skipped only when its gap
   // (rounded down at the build) exceeds it
-  const float reach = __double2float_ru(2.0 * skin[0]);
+  const float reach = __double2float_ru(2.0 * displacement_bound(skin + z, pending + z));
   unsigned long long ncont = 0;
   unsigned eflags = 0;
   uint16_t* queue = s_queue[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)WIN_PAIRS * ((gridDim.x * blockDim.x) >> 5);
-  for (long long w0 = (long long)WIN_PAIRS * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w0 < np; w0 += stride) {
+  for (long long w0 = (long long)WIN_PAIRS * ((int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) + z); w0 < np; w0 += stride) {
     const int nq = screen_window(w0, np, pflag, in_flag, in_pos, pgap, reach, queue);
     for (int k = lane; k < nq; k += 32) {
       const int e = queue[k];
@@ -268,17 +284,9 @@ k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long lon
         const int8_t sl = state[ll], si = state[i];
         if (si != DEM_STATE_NONEXISTENT && sl != DEM_STATE_NONEXISTENT) {
           const DevParams& p = sysp<B>(p0, bv, ll);
-          const double xl[3] = {a.x, a.y, a.z}, xi[3] = {b.x, b.y, b.z};
           double dist[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            double pj = xi[c];
-            const double s = periodic_shift(p, c, pj - xl[c]);
-            if (s != 0.0) pj = pj + s;
-            dist[c] = pj - xl[c];
-          }
+          const double d2 = separation(p, a, b, dist);
           const double r_lm = a.w + b.w;
-          const double d2 = dist[0] * dist[0] + dist[1] * dist[1] + dist[2] * dist[2];
           if (d2 > (r_lm - SMALL_NUMBER) * (r_lm - SMALL_NUMBER)) {
             if (f0 & PF_HIST) { pft[cc] = 0.0; pft[cap + cc] = 0.0; pft[2 * cap + cc] = 0.0; }
             f = 0;
@@ -326,7 +334,7 @@ k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long lon
     eflags |= __shfl_down_sync(0xffffffffu, eflags, o);
   }
   if (lane == 0) {
-    if (ncont) atomicAdd(&err->n_contacts, ncont);
+    if (ncont) atomicAdd(&count->pairs, ncont);
     if (eflags) atomicOr(&err->flags, eflags);
   }
 }
@@ -342,24 +350,18 @@ k_slip_fix(DevParams p0, BatchView bv, SlipFix* __restrict__ fix, const int* __r
            const double4* __restrict__ vel4, const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
            double* __restrict__ pft, long long cap, uint8_t* __restrict__ pflag, Rec32* __restrict__ rec_own,
            Rec32* __restrict__ rec_in) {
-  const unsigned n = min(fix->count, (unsigned)SLIP_FIX_CAP);
+  const int z = pdl_wait();
+  pdl_next();
+  const unsigned n = min(fix[z].count, (unsigned)SLIP_FIX_CAP);
   for (unsigned t = threadIdx.x; t < n; t += blockDim.x) {
     const long long code = fix->pair[t];
     const long long cc = code >> 1;
     const int ll = owner[cc], i = nbrs[cc];
     const DevParams& p = sysp<B>(p0, bv, ll);
     const double4 a = pos4[ll], b = pos4[i];
-    const double xl[3] = {a.x, a.y, a.z}, xi[3] = {b.x, b.y, b.z};
     double dist[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      double pj = xi[c];
-      const double s = periodic_shift(p, c, pj - xl[c]);
-      if (s != 0.0) pj = pj + s;
-      dist[c] = pj - xl[c];
-    }
+    const double d2 = separation(p, a, b, dist);
     const double r_lm = a.w + b.w;
-    const double d2 = dist[0] * dist[0] + dist[1] * dist[1] + dist[2] * dist[2];
     const double4 va = vel4[ll], vb = vel4[i], wa = omg4[ll], wb = omg4[i];
     double pin[3] = {0.0, 0.0, 0.0};
     if (code & 1) { pin[0] = pft[cc]; pin[1] = pft[cap + cc]; pin[2] = pft[2 * cap + cc]; }
@@ -421,8 +423,11 @@ k_gather_split(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, co
                const int* __restrict__ in_start, const uint8_t* __restrict__ pflag, const uint8_t* __restrict__ in_flag,
                const Rec32* __restrict__ rec_own, const Rec32* __restrict__ rec_in, double* __restrict__ fc,
                double* __restrict__ tow, double* __restrict__ acc_old, double* __restrict__ rot_acc_old,
-               unsigned* __restrict__ vslot, CellOut cells) {
-  const int me = blockIdx.x * blockDim.x + threadIdx.x;
+               unsigned* __restrict__ vslot, CellOut cells, StepEnd end) {
+  const int z = pdl_wait();
+  pdl_next();
+  if (MODE != 0) end_step(end);
+  const int me = blockIdx.x * blockDim.x + threadIdx.x + z;
   if (me >= p0.n) return;
   const DevParams& p = sysp<B>(p0, bv, me);
   const int8_t st = state[me];
@@ -478,15 +483,13 @@ template <int COLL, bool B>
 static void launch_pairs_split_t(dem_handle* h) {
   const int c = h->cur;
   const int T = h->tune.pair_threads;
-  k_pairs_split<COLL, B><<<(unsigned)(h->n_sm * h->tune.pair_bpsm), T, 0, h->stream>>>(
-      h->dp, h->bview(), h->d_np, h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c],
-      h->omg4[c], h->state, h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin,
-      rec_own_of(h), rec_in_of(h), h->slipfix, h->derr);
-  DEM_LAUNCH(h);
-  k_slip_fix<COLL, B><<<1, 128, 0, h->stream>>>(h->dp, h->bview(), h->slipfix, h->pair_owner, h->nbrs[h->rb],
-                                                h->in_pos, h->pos4[c], h->vel4[c], h->omg4[c], h->phase,
-                                                h->pft[h->pcur], h->pair_cap, h->pflag(), rec_own_of(h), rec_in_of(h));
-  DEM_LAUNCH(h);
+  launch_pdl(h, k_pairs_split<COLL, B>, (unsigned)(h->n_sm * h->tune.pair_bpsm), T, h->dp, h->bview(), h->d_np,
+             h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c], h->omg4[c], h->state,
+             h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin, h->vslot_pending(),
+             rec_own_of(h), rec_in_of(h), h->slipfix, &h->derr->count[c], h->derr);
+  launch_pdl(h, k_slip_fix<COLL, B>, 1, 128, h->dp, h->bview(), h->slipfix, h->pair_owner, h->nbrs[h->rb], h->in_pos,
+             h->pos4[c], h->vel4[c], h->omg4[c], h->phase, h->pft[h->pcur], h->pair_cap, h->pflag(), rec_own_of(h),
+             rec_in_of(h));
 }
 
 void launch_pairs_split(dem_handle* h) {
@@ -495,22 +498,32 @@ void launch_pairs_split(dem_handle* h) {
   else hz ? launch_pairs_split_t<DEM_COLL_HERTZ, false>(h) : launch_pairs_split_t<DEM_COLL_LSD, false>(h);
 }
 
+// After wall work on the side stream the gather waits for two kernels, which
+// the programmatic launch does not cover.
 template <int MODE, bool B>
-static void launch_gather_split_t(dem_handle* h) {
+static void launch_gather_split_t(dem_handle* h, bool joined) {
   const int T = h->tune.gather_threads, G = (h->nl() + T - 1) / T;
   const int c = h->cur;
-  k_gather_split<MODE, B><<<G, T, 0, h->stream>>>(
-      h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c], h->vel4[1 - c], h->omg4[1 - c],
-      h->state, h->wf, h->wall_hit, h->touched, h->row_end[h->rb], h->in_start, h->pflag(), h->in_flag,
-      rec_own_of(h), rec_in_of(h), h->fc, h->tow, h->acc_old, h->rot_acc_old, h->vslot, gather_cells<MODE, B>(h));
+  auto args = [&](auto&& go) {
+    go(h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c], h->vel4[1 - c], h->omg4[1 - c],
+       h->state, h->wf, h->wall_hit, h->touched, h->row_end[h->rb], h->in_start, h->pflag(), h->in_flag,
+       rec_own_of(h), rec_in_of(h), h->fc, h->tow, h->acc_old, h->rot_acc_old, h->vslot_note(),
+       gather_cells<MODE, B>(h), step_end(h));
+  };
+  if (!joined) {
+    args([&](auto&&... a) { launch_pdl(h, k_gather_split<MODE, B>, G, T, a...); });
+    return;
+  }
+  args([&](auto&&... a) { k_gather_split<MODE, B><<<G, T, 0, h->stream>>>(a...); });
   DEM_LAUNCH(h);
+  h->joined = false;
 }
 
-void launch_gather_split(dem_handle* h, int mode) {
+void launch_gather_split(dem_handle* h, int mode, bool joined) {
   const bool bt = h->batch();
-  if (mode == 0) bt ? launch_gather_split_t<0, true>(h) : launch_gather_split_t<0, false>(h);
-  else if (mode == 1) bt ? launch_gather_split_t<1, true>(h) : launch_gather_split_t<1, false>(h);
-  else bt ? launch_gather_split_t<2, true>(h) : launch_gather_split_t<2, false>(h);
+  if (mode == 0) bt ? launch_gather_split_t<0, true>(h, joined) : launch_gather_split_t<0, false>(h, joined);
+  else if (mode == 1) bt ? launch_gather_split_t<1, true>(h, joined) : launch_gather_split_t<1, false>(h, joined);
+  else bt ? launch_gather_split_t<2, true>(h, joined) : launch_gather_split_t<2, false>(h, joined);
 }
 
 }  // namespace demb

@@ -1056,6 +1056,7 @@ int run_neighbour(dem_handle* h, bool carry_history) {
   const bool bt = h->batch();
   const BatchView bv = h->bview();
   DevErr* e = h->derr;
+  launch_skin(h);  // the last step's displacement, for the candidate list's age
   // first_rogue := none
   if (bt) k_reset_rogue<<<((int)h->sys.size() + 127) / 128, 128, 0, h->stream>>>((int)h->sys.size(), h->d_first_rogue);
   else k_set_int<<<1, 1, 0, h->stream>>>(&e->first_rogue, n);
@@ -1204,6 +1205,7 @@ int run_neighbour(dem_handle* h, bool carry_history) {
   launch_wall_gaps(h);
   if (side) {
     cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+    h->joined = true;
     return trc;
   }
   return build_transpose(h, nb);

@@ -171,11 +171,11 @@ int run_cfnewvalues_outflow(dem_handle* h, bool* force_nsearch) {
   if (h->dp.intg == DEM_INTG_AB2)
     k_integrate_outflow<2><<<G, T, 0, h->stream>>>(h->dp, h->d_obc, nbc, ef, h->dg_pijk, h->pos4[c], h->vel4[c],
                                                    h->omg4[c], h->state, h->fc, h->tow, h->acc_old, h->rot_acc_old,
-                                                   h->vslot);
+                                                   h->vslot_note());
   else
     k_integrate_outflow<1><<<G, T, 0, h->stream>>>(h->dp, h->d_obc, nbc, ef, h->dg_pijk, h->pos4[c], h->vel4[c],
                                                    h->omg4[c], h->state, h->fc, h->tow, h->acc_old, h->rot_acc_old,
-                                                   h->vslot);
+                                                   h->vslot_note());
   DEM_LAUNCH(h);
   launch_skin(h);
   h->first_pass = false;

@@ -106,7 +106,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
     cudaMemcpyAsync(h->in_flag, snap + sizeof(double) * 3 * P + P, P, cudaMemcpyDeviceToDevice, h->stream);
   }
   // the timed pair launches added to the contact counters
-  cudaMemsetAsync(&h->derr->n_contacts, 0, 2 * sizeof(unsigned long long), h->stream);
+  clear_counts(h);
   if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "autotune")) return rc;
   if (out) fill_out(h, out, best_p, best_g, best_n);
   return 0;

@@ -5,7 +5,8 @@ the oracle.
   pair counts at and around multiples of both;
 - the wall work takes one particle per thread up to two blocks per
   multiprocessor and four past that: bed sizes on both sides, with the counts
-  not a multiple of four.
+  not a multiple of four;
+- the contact counts of passes that integrate and passes that do not.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -74,3 +75,32 @@ def test_wall_work_by_size(n_side):
     fo, po = o.download_wall_history()
     assert np.array_equal(fg, fo)
     assert np.array_equal(pg[fg >= 0], po[fo >= 0])
+
+
+def test_contact_counts_of_mixed_passes():
+    """Counts are those of the last force pass, whether it integrated or not."""
+    case, prm, arr, walls = settling_case(n_side=(6, 10, 6), spacing=0.98, jitter=0.02, nsn=5)
+    g, o = pair_both(prm, arr, walls)
+
+    def same():
+        a, b = g.stats(), o.stats()
+        assert (a["n_contacts"], a["n_wall_contacts"]) == (b["n_contacts"], b["n_wall_contacts"])
+        assert a["n_contacts"] > 0
+
+    for s in (g, o):
+        s.calc_force()
+    same()
+    for s in (g, o):
+        s.cfnewvalues()
+        s.nn = 1
+        s.step(3)
+    same()
+    for s in (g, o):
+        s.calc_force()
+        s.calc_force()
+        s.cfnewvalues()
+    same()
+    for s in (g, o):
+        s.step(13, nn_first=6)
+    same()
+    compare_state(g, o, exact=True)
