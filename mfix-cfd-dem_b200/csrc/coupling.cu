@@ -30,14 +30,18 @@ struct Gas {
   double* p_force = nullptr;   // (3, ncell) or null
   double* vol_surr = nullptr;  // ncell
   double* rop_s = nullptr;     // (M, ncell)
-  double* rops_node = nullptr; // (M, ncell)
+  double* dens_node = nullptr; // (M, ncell): node density
   double* vol_node = nullptr;  // ncell: DES_VOL_NODE
   double* drag_am = nullptr;   // ncell: DRAG_AM per node
   double* drag_bm = nullptr;   // (3, ncell): DRAG_BM per node
   double* f_gds = nullptr;     // ncell: F_GDS per cell
-  int* pijk = nullptr;         // (n, 4): i, j, k, ijk (1-based), 0 = none
+  int4* pijk = nullptr;        // n: fluid cell (i, j, k), 1-based, 0 = none, and the place in its cell's list as found
   double* f_gp = nullptr;      // n
-  int* pic_cnt = nullptr; int* pic_start = nullptr; int* pic_list = nullptr;
+  // particles of each fluid cell: pic_cnt is zero between the passes that
+  // count into it, pic_tmp holds the lists in the order found, pic_list in
+  // ascending index, pic_dat what the deposition needs of each entry
+  int* pic_cnt = nullptr; int* pic_start = nullptr; int* pic_tmp = nullptr; int* pic_list = nullptr;
+  double4* pic_dat = nullptr;
   bool have_mean = false;
 };
 
@@ -70,53 +74,56 @@ __device__ __forceinline__ int face_search(const double* f, int nc, double x) {
   return hi;
 }
 
-__global__ void k_pic_locate(DevParams p, GasDev G, double4* __restrict__ pos4, double4* __restrict__ vel4,
-                             double4* __restrict__ omg4, int8_t* __restrict__ state, int* __restrict__ pijk,
-                             int* __restrict__ cnt, double* __restrict__ fc, double* __restrict__ tow,
-                             int* __restrict__ wall_fid, DevErr* __restrict__ err) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= p.n) return;
-  int* pj = pijk + 4 * (size_t)l;
-  if (state[l] == DEM_STATE_NONEXISTENT) { pj[0] = pj[1] = pj[2] = pj[3] = 0; return; }
-  const double4 x = pos4[l];
+// PIC_SEARCH of one particle at x: its fluid cell, a count in it and its
+// place there; false when it lies outside the fluid grid.
+__device__ __forceinline__ bool pic_locate(const GasDev& G, const double4& x, bool counted, int* __restrict__ cnt,
+                                           int4& out) {
   const int i = face_search(G.xe, G.imax, x.x);
   const int j = face_search(G.yn, G.jmax, x.y);
   const int k = G.no_k ? 1 : face_search(G.zt, G.kmax, x.z);
-  if (!(i >= 1 && i <= G.gi2 && j >= 1 && j <= G.gj2 && k >= 1 && k <= G.gk2)) {
-    // outside the fluid grid: DELETE_PARTICLE (particles_in_cell.f:170-180)
-    pos4[l] = make_double4(0.0, 0.0, 0.0, 0.0);
-    vel4[l] = make_double4(0.0, 0.0, 0.0, 3.4028234663852886e38);
-    omg4[l] = make_double4(0.0, 0.0, 0.0, 0.0);
-    for (int a = 0; a < 3; ++a) { fc[(size_t)a * p.n + l] = 0.0; tow[(size_t)a * p.n + l] = 0.0; }
-    for (int s = 0; s < p.cmax; ++s) wall_fid[(size_t)l * p.cmax + s] = -1;
-    state[l] = DEM_STATE_NONEXISTENT;
-    atomicAdd(&err->rogue_removed, 1ull);
-    pj[0] = pj[1] = pj[2] = pj[3] = 0;
-    return;
-  }
-  const int c = gijk(G, i, j, k);
-  pj[0] = i; pj[1] = j; pj[2] = k; pj[3] = c + 1;
-  if (state[l] < DEM_STATE_NORMAL_GHOST) atomicAdd(&cnt[c], 1);
+  if (!(i >= 1 && i <= G.gi2 && j >= 1 && j <= G.gj2 && k >= 1 && k <= G.gk2)) return false;
+  out = make_int4(i, j, k, counted ? atomicAdd(&cnt[gijk(G, i, j, k)], 1) : -1);
+  return true;
 }
 
-__global__ void k_pic_scatter(int n, const int8_t* __restrict__ state, const int* __restrict__ pijk,
-                              const int* __restrict__ start, int* __restrict__ fill, int* __restrict__ list) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= n || state[l] == DEM_STATE_NONEXISTENT || state[l] >= DEM_STATE_NORMAL_GHOST) return;
-  const int c = pijk[4 * (size_t)l + 3] - 1;
-  list[start[c] + atomicAdd(&fill[c], 1)] = l;
+// Outside the fluid grid: DELETE_PARTICLE (particles_in_cell.f:170-180).
+__device__ __forceinline__ void pic_delete(const DevParams& p, int l, double4* __restrict__ pos4,
+                                           double4* __restrict__ vel4, double4* __restrict__ omg4,
+                                           int8_t* __restrict__ state, double* __restrict__ fc,
+                                           double* __restrict__ tow, int* __restrict__ wall_fid,
+                                           DevErr* __restrict__ err) {
+  pos4[l] = make_double4(0.0, 0.0, 0.0, 0.0);
+  vel4[l] = make_double4(0.0, 0.0, 0.0, 3.4028234663852886e38);
+  omg4[l] = make_double4(0.0, 0.0, 0.0, 0.0);
+  for (int a = 0; a < 3; ++a) { fc[(size_t)a * p.n + l] = 0.0; tow[(size_t)a * p.n + l] = 0.0; }
+  for (int s = 0; s < p.cmax; ++s) wall_fid[(size_t)l * p.cmax + s] = -1;
+  state[l] = DEM_STATE_NONEXISTENT;
+  atomicAdd(&err->rogue_removed, 1ull);
 }
 
-__global__ void k_pic_sort(int ncell, const int* __restrict__ start, int* __restrict__ list) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  const int s = start[c], e = start[c + 1];
-  for (int a = s + 1; a < e; ++a) {
-    const int v = list[a];
-    int b = a - 1;
-    while (b >= s && list[b] > v) { list[b + 1] = list[b]; --b; }
-    list[b + 1] = v;
-  }
+__global__ void k_pic_locate(DevParams p, GasDev G, double4* __restrict__ pos4, double4* __restrict__ vel4,
+                             double4* __restrict__ omg4, int8_t* __restrict__ state, int4* __restrict__ pijk,
+                             int* __restrict__ cnt, double* __restrict__ fc, double* __restrict__ tow,
+                             int* __restrict__ wall_fid, DevErr* __restrict__ err) {
+  const int z = pdl_wait();
+  pdl_next();
+  const int l = blockIdx.x * blockDim.x + threadIdx.x + z;
+  if (l >= p.n) return;
+  int4 c = make_int4(0, 0, 0, -1);
+  const int8_t st = state[l];
+  if (st != DEM_STATE_NONEXISTENT && !pic_locate(G, pos4[l], st < DEM_STATE_NORMAL_GHOST, cnt, c))
+    pic_delete(p, l, pos4, vel4, omg4, state, fc, tow, wall_fid, err);
+  pijk[l] = c;
+}
+
+__global__ void k_pic_scatter(GasDev G, int n, const int4* __restrict__ pijk, const int* __restrict__ start,
+                              int* __restrict__ list) {
+  const int z = pdl_wait();
+  pdl_next();
+  const int l = blockIdx.x * blockDim.x + threadIdx.x + z;
+  if (l >= n) return;
+  const int4 c = pijk[l];
+  if (c.w >= 0) list[start[gijk(G, c.x, c.y, c.z)] + c.w] = l;
 }
 
 // Trilinear weights of a point in fluid cell (i,j,k), node (ii,jj,kk) of
@@ -135,6 +142,43 @@ __device__ __forceinline__ void cell_weights(const GasDev& G, int i, int j, int 
     for (int kk = 0; kk < 2; ++kk) for (int jj = 0; jj < 2; ++jj) for (int ii = 0; ii < 2; ++ii)
       w[kk][jj][ii] = xx[ii] * yy[jj] * zz[kk];
   }
+}
+
+// Each list in ascending index: a thread per particle puts it at the place
+// given by the number of smaller indices in its cell's list (a cell holds a
+// few, and neighbouring threads read the same ones), with what the deposition
+// of the cell's nodes needs of it: the trilinear coordinates in the cell and
+// the mass (GARG_2012), or the volume of a NORMAL particle (no
+// interpolation).  The coordinates cost three divisions, here once instead of
+// at each of the eight nodes.
+template <bool GARG>
+__global__ void k_pic_sort(GasDev G, int n, const int4* __restrict__ pijk, const int* __restrict__ start,
+                           const int* __restrict__ tmp, const double4* __restrict__ pos4,
+                           const double4* __restrict__ vel4, const int8_t* __restrict__ state,
+                           int* __restrict__ list, double4* __restrict__ dat) {
+  const int z = pdl_wait();
+  pdl_next();
+  const int l = blockIdx.x * blockDim.x + threadIdx.x + z;
+  if (l >= n) return;
+  const int4 c = pijk[l];
+  if (c.w < 0) return;
+  const int ijk = gijk(G, c.x, c.y, c.z);
+  const int s = start[ijk], e = start[ijk + 1];
+  const double4 x = pos4[l];
+  int at = s;
+  for (int q = s; q < e; ++q) at += tmp[q] < l;
+  list[at] = l;
+  double4 d;
+  if (GARG) {
+    const double dxx = G.xe[c.x] - G.xe[c.x - 1], dyy = G.yn[c.y] - G.yn[c.y - 1];
+    d.x = (x.x - G.xe[c.x - 1]) / dxx;
+    d.y = (x.y - G.yn[c.y - 1]) / dyy;
+    d.z = G.no_k ? 0.0 : (x.z - G.zt[c.z - 1]) / (G.zt[c.z] - G.zt[c.z - 1]);
+    d.w = vel4[l].w;
+  } else {
+    d = make_double4(0.0, 0.0, 0.0, state[l] == DEM_STATE_NORMAL ? ((4.0 / 3.0) * G.pi) * (x.w * (x.w * x.w)) : -1.0);
+  }
+  dat[at] = d;
 }
 
 __device__ __forceinline__ double drag_gidaspow(double epg, double mug, double rog, double ropg, double vrel,
@@ -192,6 +236,17 @@ __device__ __forceinline__ void gas_velocity(const GasDev& G, int i, int j, int 
       }
 }
 
+// CALC_CELL_CENTER_GAS_VEL (drag_gs_des1.f:313-370) on a uniform grid
+// (FX = FX_BAR = 1/2, set_geometry.f:344-345); (i,j,k) is a fluid cell.
+__device__ __forceinline__ void cell_center_vel(const GasDev& G, int i, int j, int k,
+                                                const double* __restrict__ u_g, const double* __restrict__ v_g,
+                                                const double* __restrict__ w_g, double v[3]) {
+  const int ijk = gijk(G, i, j, k);
+  v[0] = 0.5 * u_g[gijk(G, i - 1, j, k)] + 0.5 * u_g[ijk];       // AVG_X_E
+  v[1] = 0.5 * (v_g[gijk(G, i, j - 1, k)] + v_g[ijk]);           // AVG_Y_N
+  v[2] = G.no_k ? 0.0 : 0.5 * (w_g[gijk(G, i, j, k - 1)] + w_g[ijk]);   // AVG_Z_T
+}
+
 // DES_DRAG_GP (drag_gp_des.f:97-257, Model A, Gidaspow): the relaxed F_GP
 // of a particle of radius r with velocity V in gas of void fraction epg;
 // PVOL through *pvol.
@@ -214,7 +269,7 @@ __device__ __forceinline__ double relaxed_fgp(const GasDev& G, double epg, doubl
 // depend on the deposition order).
 template <bool ADD_FC>
 __global__ void k_drag(DevParams p, GasDev G, const double4* __restrict__ pos4, const double4* __restrict__ vel4,
-                       const int8_t* __restrict__ state, const int* __restrict__ pijk,
+                       const int8_t* __restrict__ state, const int4* __restrict__ pijk,
                        const double* __restrict__ ep_g, const double* __restrict__ u_g,
                        const double* __restrict__ v_g, const double* __restrict__ w_g,
                        const double* __restrict__ p_force, double* __restrict__ f_gp, double* __restrict__ fc) {
@@ -222,7 +277,8 @@ __global__ void k_drag(DevParams p, GasDev G, const double4* __restrict__ pos4, 
   if (l >= p.n) return;
   const int8_t st = state[l];
   if (st == DEM_STATE_NONEXISTENT || st >= DEM_STATE_NORMAL_GHOST) return;
-  const int i = pijk[4 * (size_t)l], j = pijk[4 * (size_t)l + 1], k = pijk[4 * (size_t)l + 2];
+  const int4 cell = pijk[l];
+  const int i = cell.x, j = cell.y, k = cell.z;
   if (!gfluid(G, i, j, k)) return;
   const double4 X = pos4[l], V = vel4[l];
   double w[2][2][2], velfp[3];
@@ -237,6 +293,73 @@ __global__ void k_drag(DevParams p, GasDev G, const double4* __restrict__ pos4, 
   for (int c = 0; c < 3; ++c) fc[c * n + l] = fc[c * n + l] + fg * (velfp[c] - vp[c]);
   if (p_force)
     for (int c = 0; c < 3; ++c) fc[c * n + l] = fc[c * n + l] + p_force[3 * (size_t)ijk + c] * pvol;
+}
+
+// The rest of a coupled DES_TIME_STEP after the contact forces, per particle:
+// the drag by DES_INTERP_SCHEME added to FC, CFUPDATEOLD + CFNEWVALUES into
+// the other state buffer (FC and TOW end zero), and -- LOCATE, where neither a
+// periodic wrap nor a rogue deletion comes between -- the cell search of
+// PARTICLES_IN_CELL on the new position.  One pass over the particles instead
+// of three: the drag reads the state that the integration writes, and FC goes
+// through memory once.
+// A coupled step of 500,000 spheres took 401 us before this kernel, the
+// deposition from prepared entries and the two-launch scans, 308 us with them.
+template <int MODE, bool GARG>
+__global__ void k_coupled_step(DevParams p, GasDev G, const double4* __restrict__ pos_c,
+                               const double4* __restrict__ vel_c, const double4* omg_c, double4* __restrict__ pos_n,
+                               double4* __restrict__ vel_n, double4* omg_n, int8_t* __restrict__ state,
+                               int4* __restrict__ pijk, const double* __restrict__ ep_g,
+                               const double* __restrict__ u_g, const double* __restrict__ v_g,
+                               const double* __restrict__ w_g, const double* __restrict__ p_force,
+                               double* __restrict__ f_gp, double* __restrict__ fc, double* __restrict__ tow,
+                               double* __restrict__ acc_old, double* __restrict__ rot_acc_old,
+                               unsigned* __restrict__ vslot, StepEnd end, int locate, int* __restrict__ cnt,
+                               int* __restrict__ wall_fid, DevErr* __restrict__ err) {
+  const int z = pdl_wait();
+  pdl_next();
+  end_step(end);
+  const int me = blockIdx.x * blockDim.x + threadIdx.x + z;
+  if (me >= p.n) return;
+  const size_t n = (size_t)p.n;
+  const int8_t st = state[me];
+  const int4 cell = pijk[me];
+  const double4 X = pos_c[me], V = vel_c[me], W = omg_c[me];
+  const double x[3] = {X.x, X.y, X.z}, v[3] = {V.x, V.y, V.z}, w[3] = {W.x, W.y, W.z};
+  double f[3], t[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    f[c] = fc[c * n + me]; t[c] = tow[c * n + me];
+    fc[c * n + me] = 0.0; tow[c * n + me] = 0.0;
+  }
+  const bool dragged = GARG ? (st != DEM_STATE_NONEXISTENT && st < DEM_STATE_NORMAL_GHOST) : st == DEM_STATE_NORMAL;
+  if (dragged && gfluid(G, cell.x, cell.y, cell.z)) {
+    double velfp[3];
+    if (GARG) {
+      double wt[2][2][2];
+      gas_velocity(G, cell.x, cell.y, cell.z, X, u_g, v_g, w_g, velfp, wt);
+    } else {
+      cell_center_vel(G, cell.x, cell.y, cell.z, u_g, v_g, w_g, velfp);
+    }
+    const int ijk = gijk(G, cell.x, cell.y, cell.z);
+    double pvol;
+    const double fg = relaxed_fgp(G, ep_g[ijk], X.w, velfp, V, f_gp[me], &pvol);
+    f_gp[me] = fg;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] = f[c] + fg * (velfp[c] - v[c]);
+    if (p_force) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) f[c] = f[c] + p_force[3 * (size_t)ijk + c] * pvol;
+    }
+  } else if (!GARG && dragged) {
+    f_gp[me] = 0.0;
+  }
+  const double4 xn = finish_particle<MODE>(p, me, st, x, v, w, X.w, V.w, W.w, f, t, pos_n, vel_n, omg_n, fc, tow,
+                                           acc_old, rot_acc_old, vslot);
+  if (!locate) return;
+  int4 to = make_int4(0, 0, 0, -1);
+  if (st != DEM_STATE_NONEXISTENT && !pic_locate(G, xn, st < DEM_STATE_NORMAL_GHOST, cnt, to))
+    pic_delete(p, me, pos_n, vel_n, omg_n, state, fc, tow, wall_fid, err);
+  pijk[me] = to;
 }
 
 // DRAG_GS_GAS0 deposition as a gather per node: the node's cells in
@@ -294,17 +417,6 @@ __global__ void k_fgds(GasDev G, const double* __restrict__ drag_am, double* __r
 
 // ---- DES_INTERP_SCHEME = NONE: the ...1 routines without a filter ------
 
-// CALC_CELL_CENTER_GAS_VEL (drag_gs_des1.f:313-370) on a uniform grid
-// (FX = FX_BAR = 1/2, set_geometry.f:344-345); (i,j,k) is a fluid cell.
-__device__ __forceinline__ void cell_center_vel(const GasDev& G, int i, int j, int k,
-                                                const double* __restrict__ u_g, const double* __restrict__ v_g,
-                                                const double* __restrict__ w_g, double v[3]) {
-  const int ijk = gijk(G, i, j, k);
-  v[0] = 0.5 * u_g[gijk(G, i - 1, j, k)] + 0.5 * u_g[ijk];       // AVG_X_E
-  v[1] = 0.5 * (v_g[gijk(G, i, j - 1, k)] + v_g[ijk]);           // AVG_Y_N
-  v[2] = G.no_k ? 0.0 : 0.5 * (w_g[gijk(G, i, j, k - 1)] + w_g[ijk]);   // AVG_Z_T
-}
-
 __device__ __forceinline__ double sphere_vol(const GasDev& G, double r) {
   return ((4.0 / 3.0) * G.pi) * (r * (r * r));
 }
@@ -316,13 +428,14 @@ __device__ __forceinline__ double sphere_vol(const GasDev& G, double r) {
 // particles in fluid cells changes.
 template <bool ADD_FC>
 __global__ void k_drag1(DevParams p, GasDev G, const double4* __restrict__ pos4, const double4* __restrict__ vel4,
-                        const int8_t* __restrict__ state, const int* __restrict__ pijk,
+                        const int8_t* __restrict__ state, const int4* __restrict__ pijk,
                         const double* __restrict__ ep_g, const double* __restrict__ u_g,
                         const double* __restrict__ v_g, const double* __restrict__ w_g,
                         const double* __restrict__ p_force, double* __restrict__ f_gp, double* __restrict__ fc) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= p.n || state[l] != DEM_STATE_NORMAL) return;
-  const int i = pijk[4 * (size_t)l], j = pijk[4 * (size_t)l + 1], k = pijk[4 * (size_t)l + 2];
+  const int4 cell = pijk[l];
+  const int i = cell.x, j = cell.y, k = cell.z;
   if (!gfluid(G, i, j, k)) {
     if (ADD_FC) f_gp[l] = 0.0;
     return;
@@ -373,11 +486,13 @@ __global__ void k_gas1_cell(GasDev G, const double4* __restrict__ vel4, const in
 // COMP_MEAN_FIELDS1 with FILTER_SIZE = 0 (comp_mean_fields1.f:46-104) and
 // CALC_EPG_DES, per cell: SOLVOLINC = sum of PVOL of its NORMAL particles in
 // ascending index, ROP_S = RO_S*SOLVOLINC/VOL and EP_G on fluid cells.
-__global__ void k_mean_fields1(GasDev G, const double4* __restrict__ pos4, const uint8_t* __restrict__ phase,
-                               const int8_t* __restrict__ state, const int* __restrict__ pic_start,
+__global__ void k_mean_fields1(GasDev G, const double4* __restrict__ pic_dat, const uint8_t* __restrict__ phase,
+                               const int* __restrict__ pic_start,
                                const int* __restrict__ pic_list, double* __restrict__ rop_s,
                                double* __restrict__ ep_g) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int z = pdl_wait();
+  pdl_next();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x + z;
   if (c >= G.ncell) return;
   const int i = c % G.gi2 + 1, j = (c / G.gi2) % G.gj2 + 1, k = c / (G.gi2 * G.gj2) + 1;
   const bool fl = gfluid(G, i, j, k);
@@ -385,10 +500,10 @@ __global__ void k_mean_fields1(GasDev G, const double4* __restrict__ pos4, const
   for (int m = 0; m < G.M; ++m) sv[m] = 0.0;
   if (fl)
     for (int q = pic_start[c]; q < pic_start[c + 1]; ++q) {
-      const int np = pic_list[q];
-      if (state[np] != DEM_STATE_NORMAL) continue;
-      const int m = phase[np];
-      sv[m] = sv[m] + sphere_vol(G, pos4[np].w);
+      const double pvol = pic_dat[q].w;
+      if (pvol < 0.0) continue;  // not NORMAL
+      const int m = G.M > 1 ? phase[pic_list[q]] : 0;
+      sv[m] = sv[m] + pvol;
     }
   double sum_eps = 0.0;
   for (int m = 0; m < G.M; ++m) {
@@ -399,11 +514,15 @@ __global__ void k_mean_fields1(GasDev G, const double4* __restrict__ pos4, const
   if (fl) ep_g[c] = 1.0 - fmin(1.0, sum_eps);
 }
 
-// COMP_MEAN_FIELDS0 node deposition as a gather over the node's cells.
-__global__ void k_node_deposit(GasDev G, const double4* __restrict__ pos4, const double4* __restrict__ vel4,
-                               const uint8_t* __restrict__ phase, const int* __restrict__ pic_start,
-                               const int* __restrict__ pic_list, double* __restrict__ rops_node) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// COMP_MEAN_FIELDS0 node deposition as a gather over the node's cells, from
+// the entries k_pic_sort laid out in list order (one aligned 32-byte word
+// each, a cell's side by side), divided by the volume around the node.
+__global__ void k_node_deposit(GasDev G, const double4* __restrict__ pic_dat, const uint8_t* __restrict__ phase,
+                               const int* __restrict__ pic_start, const int* __restrict__ pic_list,
+                               const double* __restrict__ vol_surr, double* __restrict__ dens_node) {
+  const int z = pdl_wait();
+  pdl_next();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x + z;
   const int ni = G.imax + 1, nj = G.jmax + 1, nk = G.no_k ? 1 : G.kmax + 1;
   if (t >= ni * nj * nk) return;
   const int I = t % ni + 1, J = (t / ni) % nj + 1, K = t / (ni * nj) + 1;
@@ -417,48 +536,44 @@ __global__ void k_node_deposit(GasDev G, const double4* __restrict__ pos4, const
         const int c = gijk(G, i, j, k);
         const int ii = I - (i - 1), jj = J - (j - 1), kk = G.no_k ? 0 : K - (k - 1);
         for (int q = pic_start[c]; q < pic_start[c + 1]; ++q) {
-          const int np = pic_list[q];
-          const double4 X = pos4[np];
-          double w[2][2][2];
-          cell_weights(G, i, j, k, X.x, X.y, X.z, w);
-          const double temp1 = w[kk][jj][ii] * vel4[np].w;
-          const int m = phase[np];
-          acc[m] = acc[m] + temp1;
+          const double4 d = ld32(pic_dat + q);
+          const double wx = ii ? d.x : 1 - d.x, wy = jj ? d.y : 1 - d.y;
+          double w = wx * wy;
+          if (!G.no_k) w = w * (kk ? d.z : 1 - d.z);
+          const int m = G.M > 1 ? phase[pic_list[q]] : 0;
+          acc[m] = acc[m] + w * d.w;
         }
       }
-  for (int m = 0; m < G.M; ++m) rops_node[(size_t)m * G.ncell + node] = acc[m];
+  const double vs = vol_surr[node];
+  for (int m = 0; m < G.M; ++m) dens_node[(size_t)m * G.ncell + node] = vs == 0.0 ? 0.0 : acc[m] / vs;
 }
 
 // Node -> cell averaging, normalisation and CALC_EPG_DES, per cell.
-__global__ void k_cell_fields(GasDev G, const double* __restrict__ vol_surr, const double* __restrict__ rops_node,
-                              double* __restrict__ rop_s, double* __restrict__ ep_g) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_cell_fields(GasDev G, const double* __restrict__ dens_node, double* __restrict__ rop_s,
+                              double* __restrict__ ep_g) {
+  const int z = pdl_wait();
+  pdl_next();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x + z;
   if (c >= G.ncell) return;
   const int II = c % G.gi2 + 1, JJ = (c / G.gi2) % G.gj2 + 1, KK = c / (G.gi2 * G.gj2) + 1;
   const int ni = G.imax + 1, nj = G.jmax + 1, nk = G.no_k ? 1 : G.kmax + 1;
-  double acc[MAXP];
-  for (int m = 0; m < G.M; ++m) acc[m] = 0.0;
-  for (int K = (G.no_k ? KK : KK - 1); K <= KK; ++K)
-    for (int J = JJ - 1; J <= JJ; ++J)
-      for (int I = II - 1; I <= II; ++I) {
-        if (I < 1 || I > ni || J < 1 || J > nj || K < 1 || K > nk) continue;
-        const int node = gijk(G, I, J, K);
-        const double vs = vol_surr[node];
-        if (vs == 0.0) continue;
-        for (int m = 0; m < G.M; ++m) {
-          const double dens = rops_node[(size_t)m * G.ncell + node] / vs;
-          acc[m] = acc[m] + dens * G.vol;
+  const bool fl = gfluid(G, II, JJ, KK);
+  double sum_eps = 0.0;
+  for (int m = 0; m < G.M; ++m) {
+    double acc = 0.0;
+    for (int K = (G.no_k ? KK : KK - 1); K <= KK; ++K)
+      for (int J = JJ - 1; J <= JJ; ++J)
+        for (int I = II - 1; I <= II; ++I) {
+          if (I < 1 || I > ni || J < 1 || J > nj || K < 1 || K > nk) continue;
+          acc = acc + dens_node[(size_t)m * G.ncell + gijk(G, I, J, K)] * G.vol;
         }
-      }
-  if (gfluid(G, II, JJ, KK)) {
-    double sum_eps = 0.0;
-    for (int m = 0; m < G.M; ++m) {
-      if (acc[m] > 0.0) acc[m] = acc[m] / G.vol;
-      sum_eps = sum_eps + acc[m] / G.ro_s[m];
+    if (fl) {
+      if (acc > 0.0) acc = acc / G.vol;
+      sum_eps = sum_eps + acc / G.ro_s[m];
     }
-    ep_g[c] = 1.0 - fmin(1.0, sum_eps);
+    rop_s[(size_t)m * G.ncell + c] = acc;
   }
-  for (int m = 0; m < G.M; ++m) rop_s[(size_t)m * G.ncell + c] = acc[m];
+  if (fl) ep_g[c] = 1.0 - fmin(1.0, sum_eps);
 }
 
 // CALC_DES_BEDHEIGHT (des_granular_temperature.f:201-267) partial sums:
@@ -508,42 +623,38 @@ static GasDev gas_view(dem_handle* h) {
   return G;
 }
 
-static int run_pic(dem_handle* h) {
+// PARTICLES_IN_CELL; `located`: the integration has done the cell search.
+static int run_pic(dem_handle* h, bool located = false) {
   Gas* s = h->gas;
   const GasDev G = gas_view(h);
   const int T = 256, B = (h->n + T - 1) / T;
-  cudaMemsetAsync(s->pic_cnt, 0, sizeof(int) * (s->ncell + 1), h->stream);
   const int c = h->cur;
-  k_pic_locate<<<B, T, 0, h->stream>>>(h->dp, G, h->pos4[c], h->vel4[c], h->omg4[c], h->state, s->pijk,
-                                       s->pic_cnt, h->fc, h->tow, h->wall_fid, h->derr);
-  DEM_LAUNCH(h);
-  if (int rc = exclusive_scan(h, s->pic_cnt, s->pic_start, s->ncell, s->pic_start + s->ncell)) return rc;
-  cudaMemsetAsync(s->pic_cnt, 0, sizeof(int) * (s->ncell + 1), h->stream);
-  k_pic_scatter<<<B, T, 0, h->stream>>>(h->n, h->state, s->pijk, s->pic_start, s->pic_cnt, s->pic_list);
-  k_pic_sort<<<(s->ncell + T - 1) / T, T, 0, h->stream>>>(s->ncell, s->pic_start, s->pic_list);
-  h->launches += 2;
+  if (!located)
+    launch_pdl(h, k_pic_locate, B, T, h->dp, G, h->pos4[c], h->vel4[c], h->omg4[c], h->state, s->pijk, s->pic_cnt,
+               h->fc, h->tow, h->wall_fid, h->derr);
+  if (int rc = exclusive_scan(h, s->pic_cnt, s->pic_start, s->ncell, s->pic_start + s->ncell, true)) return rc;
+  launch_pdl(h, k_pic_scatter, B, T, G, h->n, s->pijk, s->pic_start, s->pic_tmp);
+  launch_pdl(h, s->g.interp_scheme == DEM_INTERP_NONE ? k_pic_sort<false> : k_pic_sort<true>, B, T, G, h->n, s->pijk,
+             s->pic_start, s->pic_tmp, h->pos4[c], h->vel4[c], h->state, s->pic_list, s->pic_dat);
   return check_cuda(h, cudaGetLastError(), "particles_in_cell");
 }
 
-static int run_mean_fields(dem_handle* h) {
+static int run_mean_fields(dem_handle* h, bool located = false) {
   ProfScope ps(h, DEM_PROF_COUPLING);
-  if (int rc = run_pic(h)) return rc;
+  if (int rc = run_pic(h, located)) return rc;
   Gas* s = h->gas;
   const GasDev G = gas_view(h);
   const int T = 256;
   if (s->g.interp_scheme == DEM_INTERP_NONE) {   // COMP_MEAN_FIELDS1
-    k_mean_fields1<<<(G.ncell + T - 1) / T, T, 0, h->stream>>>(G, h->pos4[h->cur], h->phase, h->state,
-                                                               s->pic_start, s->pic_list, s->rop_s, s->ep_g);
-    DEM_LAUNCH(h);
+    launch_pdl(h, k_mean_fields1, (G.ncell + T - 1) / T, T, G, s->pic_dat, h->phase, s->pic_start, s->pic_list,
+               s->rop_s, s->ep_g);
     s->have_mean = true;
     return check_cuda(h, cudaGetLastError(), "mean fields");
   }
   const int nnodes = (G.imax + 1) * (G.jmax + 1) * (G.no_k ? 1 : G.kmax + 1);
-  const int c = h->cur;
-  k_node_deposit<<<(nnodes + T - 1) / T, T, 0, h->stream>>>(G, h->pos4[c], h->vel4[c], h->phase, s->pic_start,
-                                                            s->pic_list, s->rops_node);
-  k_cell_fields<<<(G.ncell + T - 1) / T, T, 0, h->stream>>>(G, s->vol_surr, s->rops_node, s->rop_s, s->ep_g);
-  h->launches += 2;
+  launch_pdl(h, k_node_deposit, (nnodes + T - 1) / T, T, G, s->pic_dat, h->phase, s->pic_start, s->pic_list,
+             s->vol_surr, s->dens_node);
+  launch_pdl(h, k_cell_fields, (G.ncell + T - 1) / T, T, G, s->dens_node, s->rop_s, s->ep_g);
   s->have_mean = true;
   return check_cuda(h, cudaGetLastError(), "mean fields");
 }
@@ -575,6 +686,25 @@ static int run_drag1(dem_handle* h) {
 // CALC_DRAG_DES: the particle side of the drag by DES_INTERP_SCHEME.
 static int run_calc_drag(dem_handle* h) {
   return h->gas->g.interp_scheme == DEM_INTERP_NONE ? run_drag1(h) : run_drag(h);
+}
+
+// A coupled step after its force pass: drag, integration and, with `locate`,
+// the particles' fluid cells (k_coupled_step).
+static int run_coupled_step(dem_handle* h, bool locate) {
+  ProfScope ps(h, DEM_PROF_INTEGRATE);
+  Gas* s = h->gas;
+  const GasDev G = gas_view(h);
+  const int T = 256, B = (h->n + T - 1) / T;
+  const int c = h->cur;
+  const bool garg = s->g.interp_scheme != DEM_INTERP_NONE, ab2 = h->dp.intg == DEM_INTG_AB2;
+  launch_pdl(h, garg ? (ab2 ? k_coupled_step<2, true> : k_coupled_step<1, true>)
+                     : (ab2 ? k_coupled_step<2, false> : k_coupled_step<1, false>),
+             B, T, h->dp, G, h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c], h->vel4[1 - c], h->omg4[1 - c],
+             h->state, s->pijk, s->ep_g, s->u_g, s->v_g, s->w_g, s->p_force, s->f_gp, h->fc, h->tow, h->acc_old,
+             h->rot_acc_old, h->vslot_note(), step_end(h), locate ? 1 : 0, s->pic_cnt, h->wall_fid, h->derr);
+  h->cur = 1 - c;
+  h->first_pass = false;
+  return check_cuda(h, cudaGetLastError(), "coupled step");
 }
 
 // DRAG_GS_GAS1: F_GP per particle, then the per-cell gather.
@@ -615,8 +745,8 @@ void free_gas(dem_handle* h) {
   Gas* s = h->gas;
   if (!s) return;
   void* ptrs[] = {s->xe, s->yn, s->zt, s->ep_g, s->u_g, s->v_g, s->w_g, s->p_force, s->vol_surr, s->rop_s,
-                  s->rops_node, s->vol_node, s->drag_am, s->drag_bm, s->f_gds, s->pijk, s->f_gp,
-                  s->pic_cnt, s->pic_start, s->pic_list};
+                  s->dens_node, s->vol_node, s->drag_am, s->drag_bm, s->f_gds, s->pijk, s->f_gp,
+                  s->pic_cnt, s->pic_start, s->pic_tmp, s->pic_list, s->pic_dat};
   for (void* q : ptrs) if (q) cudaFree(q);
   delete s;
   h->gas = nullptr;
@@ -708,16 +838,18 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
   if (p_force) A((void**)&s->p_force, sizeof(double) * 3 * nc);
   A((void**)&s->vol_surr, sizeof(double) * nc);
   A((void**)&s->rop_s, sizeof(double) * nc * s->M);
-  A((void**)&s->rops_node, sizeof(double) * nc * s->M);
+  A((void**)&s->dens_node, sizeof(double) * nc * s->M);
   A((void**)&s->vol_node, sizeof(double) * nc);
   A((void**)&s->drag_am, sizeof(double) * nc);
   A((void**)&s->drag_bm, sizeof(double) * 3 * nc);
   A((void**)&s->f_gds, sizeof(double) * nc);
-  A((void**)&s->pijk, sizeof(int) * 4 * (size_t)h->n);
+  A((void**)&s->pijk, sizeof(int4) * (size_t)h->n);
   A((void**)&s->f_gp, sizeof(double) * (size_t)h->n);
   A((void**)&s->pic_cnt, sizeof(int) * (nc + 1));
   A((void**)&s->pic_start, sizeof(int) * (nc + 1));
+  A((void**)&s->pic_tmp, sizeof(int) * (size_t)h->n);
   A((void**)&s->pic_list, sizeof(int) * (size_t)h->n);
+  A((void**)&s->pic_dat, sizeof(double4) * (size_t)h->n);
   if (!ok) { free_gas(h); return set_err(h, DEM_ERR_CUDA, "cudaMalloc gas fields"); }
   cudaMemcpyAsync(s->xe, fx.data(), sizeof(double) * fx.size(), cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(s->yn, fy.data(), sizeof(double) * fy.size(), cudaMemcpyHostToDevice, h->stream);
@@ -729,6 +861,8 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
   if (p_force) cudaMemcpyAsync(s->p_force, p_force, sizeof(double) * 3 * nc, cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(s->vol_surr, vs.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(s->vol_node, vn.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream);
+  cudaMemsetAsync(s->pic_cnt, 0, sizeof(int) * (nc + 1), h->stream);
+  cudaMemsetAsync(s->dens_node, 0, sizeof(double) * nc * s->M, h->stream);
   cudaMemsetAsync(s->drag_am, 0, sizeof(double) * nc, h->stream);
   cudaMemsetAsync(s->drag_bm, 0, sizeof(double) * 3 * nc, h->stream);
   cudaMemsetAsync(s->f_gds, 0, sizeof(double) * nc, h->stream);
@@ -835,25 +969,40 @@ int dem_step_coupled(dem_handle* h, int32_t nn_first, int32_t nsteps) {
   if (nsteps < 0 || nn_first < 1) return set_err(h, DEM_ERR_ARG, "bad step range");
   const DevParams& p = h->dp;
   const bool anyper = p.per[0] || p.per[1] || (p.per[2] && !p.no_k);
+  const bool flow = !h->obc.empty() || !h->ibc.empty();
+  // the kernels of these steps follow one another on the stream
+  struct Chain {
+    dem_handle* h;
+    Chain(dem_handle* hh, bool on) : h(hh) { h->chain = on && !h->prof; h->joined = true; }
+    ~Chain() { h->chain = false; }
+  } chain(h, !flow);
   for (int k = 0; k < nsteps; ++k) {
     const int nn = nn_first + k;
-    if (int rc = run_force(h, false)) return rc;              // CALC_FORCE_DEM
-    if (int rc = run_calc_drag(h)) return rc;                 // CALC_DRAG_DES
-    bool force = false;
-    if (h->obc.empty()) {
-      if (int rc = run_cfnewvalues(h)) return rc;             // CFUPDATEOLD + CFNEWVALUES
-      if (int rc = run_mass_inflow(h)) return rc;             // MASS_INFLOW_DEM
-    } else if (int rc = run_cfnewvalues_outflow(h, &force)) { // + exit velocities, MASS_OUTFLOW_DEM
-      return rc;
+    bool do_nsearch = (nn == 1) || (nn % h->prm.neighbor_search_n == 0);
+    bool located = false;
+    if (!flow) {
+      if (int rc = run_force_open(h)) return rc;              // CALC_FORCE_DEM
+      located = !do_nsearch && !anyper;
+      if (int rc = run_coupled_step(h, located)) return rc;   // CALC_DRAG_DES, CFUPDATEOLD + CFNEWVALUES
+    } else {
+      if (int rc = run_force(h, false)) return rc;
+      if (int rc = run_calc_drag(h)) return rc;
+      if (h->obc.empty()) {
+        if (int rc = run_cfnewvalues(h)) return rc;
+        if (int rc = run_mass_inflow(h)) return rc;           // MASS_INFLOW_DEM
+      } else {                                                // + exit velocities, MASS_OUTFLOW_DEM
+        bool force = false;
+        if (int rc = run_cfnewvalues_outflow(h, &force)) return rc;
+        do_nsearch = do_nsearch || force;
+      }
     }
-    const bool do_nsearch = (nn == 1) || (nn % h->prm.neighbor_search_n == 0) || force;
     if (do_nsearch || anyper) {
       if (int rc = run_desgrid_pic(h, do_nsearch)) return rc;
     }
     if (do_nsearch) {
       if (int rc = run_neighbour(h, true)) return rc;
     }
-    if (int rc = run_mean_fields(h)) return rc;               // PARTICLES_IN_CELL + COMP_MEAN_FIELDS
+    if (int rc = run_mean_fields(h, located)) return rc;      // PARTICLES_IN_CELL + COMP_MEAN_FIELDS
     h->s_time = h->s_time + h->prm.dtsolid;
     h->steps_done++;
   }

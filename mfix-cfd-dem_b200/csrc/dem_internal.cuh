@@ -411,13 +411,17 @@ int set_err(dem_handle* h, int code, const std::string& msg);
 int check_cuda(dem_handle* h, cudaError_t e, const char* what);
 
 // scan.cu: exclusive scan of n ints into out (out may alias in); total
-// written to *d_total (device pointer) when non-null.
-int exclusive_scan(dem_handle* h, const int* in, int* out, int n, int* d_total);
+// written to *d_total (device pointer) when non-null; `clear` zeroes the
+// input behind it (not with out == in); with `go` (device pointer) nothing is
+// done unless *go is set.
+int exclusive_scan(dem_handle* h, int* in, int* out, int n, int* d_total, bool clear = false,
+                   const int* go = nullptr);
 
 // desgrid.cu / neighbor.cu / force.cu / walls.cu host drivers
 int run_desgrid_pic(dem_handle* h, bool sort_cells);
 int run_neighbour(dem_handle* h, bool carry_history);
 int run_force(dem_handle* h, bool fused);
+int run_force_open(dem_handle* h);              // forces into FC/TOW, ended by a kernel of the caller's (end_step, the other state buffer)
 int run_cfnewvalues(dem_handle* h);
 int run_bin_facets(dem_handle* h, const double* vertex_fortran, const double* norm_fortran, int nf);
 int run_split_force_error(dem_handle* h, double* rel_err);
@@ -777,7 +781,7 @@ struct CellOut {
 };
 
 template <int MODE>
-__device__ __forceinline__ void finish_particle(const DevParams& p, int me, int8_t st, const double x[3],
+__device__ __forceinline__ double4 finish_particle(const DevParams& p, int me, int8_t st, const double x[3],
                                                 const double v[3], const double w[3], double r, double m,
                                                 double omoi, const double f[3], const double t[3],
                                                 double4* __restrict__ pos_n, double4* __restrict__ vel_n,
@@ -789,7 +793,7 @@ __device__ __forceinline__ void finish_particle(const DevParams& p, int me, int8
   if (MODE == 0) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) { fc[c * n + me] = f[c]; tow[c * n + me] = t[c]; }
-    return;
+    return make_double4(x[0], x[1], x[2], r);
   }
   const double dt = p.dt;
   double xn[3], vn[3], wn[3];
@@ -846,6 +850,7 @@ __device__ __forceinline__ void finish_particle(const DevParams& p, int me, int8
   if (!keep_w) omg_n[me] = make_double4(wn[0], wn[1], wn[2], omoi);
   // |x_new - x| <= max(|v|, |v_new|) * dt for both integrators
   note_displacement(vslot, st < DEM_STATE_NORMAL_GHOST ? fmax(speed(v), speed(vn)) * dt : 0.0);
+  return xo;  // the new position
 }
 
 }  // namespace demb

@@ -1046,6 +1046,18 @@ int run_force(dem_handle* h, bool fused) {
   return 0;
 }
 
+// The force pass of a step that the caller ends: forces into FC/TOW, then a
+// kernel that integrates them into the other state buffer with end_step
+// (the coupled step, whose drag comes in between).
+int run_force_open(dem_handle* h) {
+  ProfScope ps(h, DEM_PROF_FORCE);
+  h->dp.first_pass = h->first_pass ? 1 : 0;
+  if (h->count_dirty) clear_counts(h);
+  launch_force_kernels(h, 0, h->dp.prec == DEM_PREC_SPLIT);
+  h->count_set = h->cur;
+  return check_cuda(h, cudaGetLastError(), "force kernels");
+}
+
 // Per-step force error of the split path: both paths evaluate FC for the
 // current state (the wall and pair histories are restored between and after
 // them); returns max|F_split - F_fp64| over all components divided by

@@ -1103,6 +1103,7 @@ int run_neighbour(dem_handle* h, bool carry_history) {
     if (int rc = check_cuda(h, cudaMemcpyAsync(&P, h->d_np, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "copy P")) return rc;
     if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "sync")) return rc;
     if (int rc = ensure_pair_capacity(h, (long long)P + 1)) return rc;
+    h->joined = true;
     h->n_pairs = P;
     h->np_stale = false;
   } else {
@@ -1158,6 +1159,7 @@ int run_neighbour(dem_handle* h, bool carry_history) {
                                                  h->stream), "copy candidates")) return rc;
       if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "sync")) return rc;
       if (int rc = ensure_cand_capacity(h, total)) return rc;
+      h->joined = true;
     }
     const long long cap = h->cand_cap;
     cudaMemsetAsync(h->cand_fill, 0, sizeof(int) * n, h->stream);
@@ -1180,6 +1182,7 @@ int run_neighbour(dem_handle* h, bool carry_history) {
     cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0);
     cudaStream_t main = h->stream;
     h->stream = h->side_stream;
+    h->joined = true;
     trc = build_transpose(h, nb);
     h->stream = main;
     cudaEventRecord(h->ev_join, h->side_stream);

@@ -6,6 +6,8 @@ the oracle.
 - the wall work takes one particle per thread up to two blocks per
   multiprocessor and four past that: bed sizes on both sides, with the counts
   not a multiple of four;
+- the scans take a second level past 4096 tiles of 2048 cells: a search grid
+  just over it;
 - the contact counts of passes that integrate and passes that do not.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
@@ -75,6 +77,29 @@ def test_wall_work_by_size(n_side):
     fo, po = o.download_wall_history()
     assert np.array_equal(fg, fo)
     assert np.array_equal(pg[fg >= 0], po[fo >= 0])
+
+
+def test_scan_of_many_search_cells():
+    """A DES grid of 205^3 cells (8.9 million with its ghost layers, past 4096
+    tiles of 2048)."""
+    from mfix_dem import params as P
+    d, L = 1e-3, 0.65
+    rng = np.random.default_rng(5)
+    k = np.arange(12)
+    cluster = np.stack(np.meshgrid(k, k, k, indexing="ij"), 0).reshape(3, -1) * 1.02 * d
+    pos = np.concatenate([cluster + c for c in (0.004, 0.31, 0.632)], axis=1) + rng.uniform(-2e-5, 2e-5, (3, 3 * 1728))
+    n = pos.shape[1]
+    arr = state_arrays(pos, rng.uniform(-0.1, 0.1, (3, n)), np.zeros((3, n)), np.full(n, 0.5 * d), np.full(n, 2500.0))
+    case = P.DemCase(d_p0=(d,), ro_s0=(2500.0,), coll_model="LSD", kn=1000.0, kn_w=1000.0, des_en_input=0.9,
+                     des_en_wall_input=[0.9], mew=0.1, mew_w=0.1, domain_hi=(L, L, L), desgridsearch=(205, 205, 205),
+                     neighbor_search_n=4)
+    prm, _ = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
+    g, o = pair_both(prm, arr, P.default_walls((0.0, 0.0, 0.0), (L, L, L)))
+    compare_pairs(g, o)
+    g.step(9)
+    o.step(9)
+    compare_state(g, o, exact=True)
+    compare_pairs(g, o)
 
 
 def test_contact_counts_of_mixed_passes():
