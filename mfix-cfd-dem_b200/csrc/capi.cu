@@ -450,6 +450,7 @@ int demb::alloc_handle(dem_handle* h, int nc, int nfc, long long pairs) {
   handle_arrays(h, n, (size_t)nc, (size_t)nfc, A);
   if (!ok) return DEM_ERR_CUDA;
   cudaMemset(h->wall_fid, 0xff, sizeof(int) * cmax * n);  // -1 = free slot
+  cudaMemset(h->fcell_key, 0xff, sizeof(int) * n);        // -1 = not binned
   if (cudaMallocHost((void**)&h->herr, sizeof(DevErr)) != cudaSuccess) return DEM_ERR_CUDA;
   memset(h->herr, 0, sizeof(DevErr));
   h->herr->first_rogue = h->n;
@@ -524,12 +525,12 @@ int dem_destroy(dem_handle* h) {
   invalidate_graphs(h);
   void* ptrs[] = {h->pos4[0], h->pos4[1], h->vel4[0], h->vel4[1], h->omg4[0],
                   h->state, h->phase, h->fc, h->tow, h->acc_old, h->rot_acc_old, h->dg_pijk,
-                  h->cell_cnt, h->cell_start, h->cell_fill, h->cell_list, h->row_cnt,
+                  h->cell_cnt, h->cell_fill, h->row_cnt,
                   h->row_end[0], h->row_end[1], h->nbrs[0], h->nbrs[1], h->pft[0], h->pft[1],
-                  h->in_cnt, h->in_start, h->in_fill, h->in_pair, h->pair_owner, h->vertex,
+                  h->in_cnt, h->in_start, h->in_mid, h->in_pair, h->pair_owner, h->vertex,
                   h->norm_face, h->ignore_edge, h->fbin_start, h->fbin, h->wall_fid, h->wall_pft,
                   h->scan_tmp, h->derr, h->red, h->stage, h->wall_live, h->wf, h->pflagb[0], h->pflagb[1], h->in_pos, h->in_flag, h->prec, h->touched, h->wall_hit, h->wall_cand, h->wgap, h->d_obc, h->d_ibc, h->pic_fresh, h->d_seed, h->skin, h->vslot, h->pgap,
-                  h->fcell_key, h->fcell_cnt, h->fcell_start, h->fcell_list, h->spos, h->sposf, h->sinfo, h->nslot, h->long_rows, h->cand_end, h->cand_cnt, h->cand_start, h->cand_fill, h->qof, h->cand_nb, h->cand, h->slipfix, h->d_np,
+                  h->fcell_key, h->fcell_cnt, h->fcell_start, h->fcell_slot, h->spos, h->sposf, h->sinfo, h->nslot, h->long_rows, h->cand_cnt, h->cand_start, h->cand_fill, h->qof, h->cand_nb, h->cand, h->slipfix, h->d_np,
                   h->d_sys, h->sys_of, h->d_due, h->d_first_rogue};
   for (void* p : ptrs) if (p) cudaFree(p);
   for (auto& e : h->prof_pending) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
@@ -693,7 +694,7 @@ int dem_upload_pairs(dem_handle* h, const int32_t* ni, const int32_t* nb, const 
   h->launches++;
   set_hist_flags(h);
   skin_unknown(h);  // no gaps for an uploaded list: no pair is skipped until the next build
-  if (int rc = build_transpose(h, h->rb)) return rc;
+  if (int rc = build_transpose(h, h->rb, false)) return rc;
   h->have_pairs = true;
   return check_cuda(h, cudaStreamSynchronize(h->stream), "upload pairs");
 }

@@ -248,23 +248,20 @@ struct dem_handle {
   // DES grid
   int* dg_pijk = nullptr;     // 1-based cell, 0 = none
   int* cell_cnt = nullptr;    // ncell2
-  int* cell_start = nullptr;  // ncell2+1
   int* cell_fill = nullptr;   // ncell2
-  int* cell_list = nullptr;   // n
-  int* fcell_key = nullptr;   // n: search-grid cell of each particle (0-based)
-  int* fcell_cnt = nullptr;   // nfcell+1
+  int* fcell_key = nullptr;   // n: search-grid cell of each particle (0-based; -1: not binned)
+  int* fcell_slot = nullptr;  // n: its place in the cell
+  int* fcell_cnt = nullptr;   // nfcell+1, zero between the passes that count into it
   int* fcell_start = nullptr; // nfcell+1
-  int* fcell_list = nullptr;  // n
   double4* spos = nullptr;    // n: positions in search-cell order (pair build)
   float4* sposf = nullptr;    // n: the same rounded to FP32 (conservative distance pre-check)
   int4* sinfo = nullptr;      // n: (particle, packed DES cell (i,j,k), state, search cell) in that order
   uint32_t* nslot = nullptr;  // n * NSLOT: rows kept by the count pass of the pair build, by particle
   int* long_rows = nullptr;   // n + 1: sorted-copy places of the rows longer than NSLOT, count at [n]
-  // candidate list (single-system handles): cand_end[i] ends particle i's
-  // candidates in cand_nb (particle indices); cand_cnt / cand_start /
-  // cand_fill are build scratch, qof[i] the particle's place in the sorted
+  // candidate list (single-system handles): particle i's candidates are entries
+  // [cand_start[i], cand_start[i + 1]) of cand_nb (particle indices); cand_cnt
+  // and cand_fill are build scratch, qof[i] the particle's place in the sorted
   // copy (-1 when not in it)
-  int* cand_end = nullptr;
   int* cand_cnt = nullptr;
   int* cand_start = nullptr;
   int* cand_fill = nullptr;
@@ -307,12 +304,13 @@ struct dem_handle {
   // lie side by side); pft[pcur] is current, the other takes the carry-over
   // of a rebuild
   double* pft[2] = {nullptr, nullptr};
-  int* in_cnt = nullptr;      // n
+  int* in_cnt = nullptr;      // n, zero between the builds that count into it
   int* in_start = nullptr;    // n+1
-  int* in_fill = nullptr;     // n: fill counts while the transpose is made, then the first slot of each
-                              // incoming list whose owner has a higher index (the list's end when none)
+  int* in_mid = nullptr;      // n: the first slot of each incoming list whose owner has a higher index (the
+                              // list's end when none)
   int2* in_pair = nullptr;    // cap
-  int* in_pos = nullptr;      // cap: slot of each pair in its neighbour's incoming list (inverse of in_pair)
+  int* in_pos = nullptr;      // cap: slot of each pair in its neighbour's incoming list (inverse of in_pair; during
+                              // a build its place in the list as found)
   uint8_t* in_flag = nullptr; // cap: PF_CONTACT of the pair at each incoming slot
   int* pair_owner = nullptr;  // cap
   // cap: PF_* bits of each pair, one array per history buffer: pflagb[pcur]
@@ -426,10 +424,11 @@ int run_cfnewvalues(dem_handle* h);
 int run_bin_facets(dem_handle* h, const double* vertex_fortran, const double* norm_fortran, int nf);
 int run_split_force_error(dem_handle* h, double* rel_err);
 void launch_pairs_split(dem_handle* h);         // force_split.cu
-void launch_gather_split(dem_handle* h, int mode, bool joined);
+void launch_gather_split(dem_handle* h, int mode);
 int ensure_pair_capacity(dem_handle* h, long long need);
-int build_transpose(dem_handle* h, int nb);    // neighbor.cu
+int build_transpose(dem_handle* h, int nb, bool counted);    // neighbor.cu
 void launch_neigh_count(dem_handle* h, const int* skip = nullptr);        // neighbor.cu: count pass of the pair build
+void reset_neigh_count(dem_handle* h);         // neighbor.cu: what it counts into, to zero
 void set_hist_flags(dem_handle* h);            // neighbor.cu: PF_HIST from the current history
 // neighbor.cu: the history of pairs [first, first + count) between its planes
 // and PFT_NEIGHBOR's (3,P) order on the host
@@ -474,13 +473,11 @@ void handle_arrays(dem_handle* h, size_t n, size_t nc, size_t nfc, F&& A) {
   A((void**)&h->rot_acc_old, sizeof(double) * 3 * n);
   A((void**)&h->dg_pijk, sizeof(int) * n);
   A((void**)&h->cell_cnt, sizeof(int) * (nc + 1));
-  A((void**)&h->cell_start, sizeof(int) * (nc + 1));
   A((void**)&h->cell_fill, sizeof(int) * (nc + 1));
-  A((void**)&h->cell_list, sizeof(int) * n);
   A((void**)&h->fcell_key, sizeof(int) * n);
   A((void**)&h->fcell_cnt, sizeof(int) * (nfc + 1));
   A((void**)&h->fcell_start, sizeof(int) * (nfc + 1));
-  A((void**)&h->fcell_list, sizeof(int) * n);
+  A((void**)&h->fcell_slot, sizeof(int) * n);
   A((void**)&h->spos, sizeof(double4) * n);
   A((void**)&h->sposf, sizeof(float4) * n);
   A((void**)&h->sinfo, sizeof(int4) * n);
@@ -489,7 +486,7 @@ void handle_arrays(dem_handle* h, size_t n, size_t nc, size_t nfc, F&& A) {
   A((void**)&h->row_cnt, sizeof(int) * n);
   A((void**)&h->in_cnt, sizeof(int) * n);
   A((void**)&h->in_start, sizeof(int) * (n + 1));
-  A((void**)&h->in_fill, sizeof(int) * n);
+  A((void**)&h->in_mid, sizeof(int) * n);
   A((void**)&h->fbin_start, sizeof(int) * (nc + 1));
   A((void**)&h->wall_fid, sizeof(int) * cmax * n);
   A((void**)&h->wall_pft, sizeof(double) * 3 * cmax * n);
@@ -505,7 +502,6 @@ void handle_arrays(dem_handle* h, size_t n, size_t nc, size_t nfc, F&& A) {
   A((void**)&h->d_np, sizeof(int));
   A((void**)&h->slipfix, sizeof(SlipFix));
   if (!h->batch()) {
-    A((void**)&h->cand_end, sizeof(int) * n);
     A((void**)&h->cand_cnt, sizeof(int) * n);
     A((void**)&h->cand_start, sizeof(int) * (n + 1));
     A((void**)&h->cand_fill, sizeof(int) * n);

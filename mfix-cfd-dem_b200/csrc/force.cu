@@ -910,7 +910,7 @@ static void launch_gather_t(dem_handle* h) {
   const int T = h->tune.gather_threads, G = (h->nl() + T - 1) / T;
   const int c = h->cur;
   launch_pdl(h, k_gather<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
-             h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start, h->in_fill, h->in_pair,
+             h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start, h->in_mid, h->in_pair,
              h->pflag(), h->in_flag, h->touched, h->wall_hit, h->recs(), h->fc, h->tow, h->acc_old, h->rot_acc_old,
              h->vslot_note(), gather_cells<MODE, B>(h), step_end(h));
 }
@@ -955,7 +955,7 @@ void launch_pairs_only(dem_handle* h) {
 }
 
 void launch_gather_only(dem_handle* h) {
-  if (h->dp.prec == DEM_PREC_SPLIT) launch_gather_split(h, 0, false);
+  if (h->dp.prec == DEM_PREC_SPLIT) launch_gather_split(h, 0);
   else if (h->batch()) launch_gather_fp64<true>(h, 0);
   else launch_gather_fp64<false>(h, 0);
 }
@@ -997,7 +997,7 @@ static void launch_force_kernels(dem_handle* h, int mode, bool split) {
     h->joined = true;
   }
   ProfScope ps(h, DEM_PROF_GATHER);
-  if (split) launch_gather_split(h, mode, side);
+  if (split) launch_gather_split(h, mode);
   else if (h->batch()) launch_gather_fp64<true>(h, mode);
   else launch_gather_fp64<false>(h, mode);
 }

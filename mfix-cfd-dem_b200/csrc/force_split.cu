@@ -498,32 +498,21 @@ void launch_pairs_split(dem_handle* h) {
   else hz ? launch_pairs_split_t<DEM_COLL_HERTZ, false>(h) : launch_pairs_split_t<DEM_COLL_LSD, false>(h);
 }
 
-// After wall work on the side stream the gather waits for two kernels, which
-// the programmatic launch does not cover.
 template <int MODE, bool B>
-static void launch_gather_split_t(dem_handle* h, bool joined) {
+static void launch_gather_split_t(dem_handle* h) {
   const int T = h->tune.gather_threads, G = (h->nl() + T - 1) / T;
   const int c = h->cur;
-  auto args = [&](auto&& go) {
-    go(h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c], h->vel4[1 - c], h->omg4[1 - c],
-       h->state, h->wf, h->wall_hit, h->touched, h->row_end[h->rb], h->in_start, h->pflag(), h->in_flag,
-       rec_own_of(h), rec_in_of(h), h->fc, h->tow, h->acc_old, h->rot_acc_old, h->vslot_note(),
-       gather_cells<MODE, B>(h), step_end(h));
-  };
-  if (!joined) {
-    args([&](auto&&... a) { launch_pdl(h, k_gather_split<MODE, B>, G, T, a...); });
-    return;
-  }
-  args([&](auto&&... a) { k_gather_split<MODE, B><<<G, T, 0, h->stream>>>(a...); });
-  DEM_LAUNCH(h);
-  h->joined = false;
+  launch_pdl(h, k_gather_split<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
+             h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->wall_hit, h->touched, h->row_end[h->rb], h->in_start,
+             h->pflag(), h->in_flag, rec_own_of(h), rec_in_of(h), h->fc, h->tow, h->acc_old, h->rot_acc_old,
+             h->vslot_note(), gather_cells<MODE, B>(h), step_end(h));
 }
 
-void launch_gather_split(dem_handle* h, int mode, bool joined) {
+void launch_gather_split(dem_handle* h, int mode) {
   const bool bt = h->batch();
-  if (mode == 0) bt ? launch_gather_split_t<0, true>(h, joined) : launch_gather_split_t<0, false>(h, joined);
-  else if (mode == 1) bt ? launch_gather_split_t<1, true>(h, joined) : launch_gather_split_t<1, false>(h, joined);
-  else bt ? launch_gather_split_t<2, true>(h, joined) : launch_gather_split_t<2, false>(h, joined);
+  if (mode == 0) bt ? launch_gather_split_t<0, true>(h) : launch_gather_split_t<0, false>(h);
+  else if (mode == 1) bt ? launch_gather_split_t<1, true>(h) : launch_gather_split_t<1, false>(h);
+  else bt ? launch_gather_split_t<2, true>(h) : launch_gather_split_t<2, false>(h);
 }
 
 }  // namespace demb

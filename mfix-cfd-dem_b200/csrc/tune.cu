@@ -94,7 +94,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   const int nthreads[3] = {32, 64, 128};
   for (int T : nthreads) {
     h->tune.neigh_threads = T;
-    const float ms = time_launches(h, reps, [&] { launch_neigh_count(h); });
+    const float ms = time_launches(h, reps, [&] { reset_neigh_count(h); launch_neigh_count(h); });
     if (ms < best_n) { best_n = ms; best.neigh_threads = T; }
   }
   h->tune = best;
