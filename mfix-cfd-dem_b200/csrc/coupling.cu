@@ -623,6 +623,30 @@ static GasDev gas_view(dem_handle* h) {
   return G;
 }
 
+// VOL_SURR (make_arrays_des.f:78-105), the volume of the fluid cells around
+// each node, and DES_VOL_NODE (cfassign.f:104-228), a quarter (2D) or an
+// eighth (3D) of each of them, both summed in the reference's order; zero
+// past the nodes.
+__global__ void k_grid_volumes(GasDev G, double* __restrict__ vol_surr, double* __restrict__ vol_node) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= G.ncell) return;
+  const int i = c % G.gi2 + 1, j = (c / G.gi2) % G.gj2 + 1, k = c / (G.gi2 * G.gj2) + 1;
+  double vs = 0.0, vn = 0.0;
+  if (i <= G.imax + 1 && j <= G.jmax + 1 && (G.no_k || k <= G.kmax + 1)) {
+    auto fv = [&](int ii, int jj, int kk) { return gfluid(G, ii, jj, kk) ? G.vol : 0.0; };
+    for (int kk = k; kk <= (G.no_k ? k : k + 1); ++kk)
+      for (int jj = j; jj <= j + 1; ++jj)
+        for (int ii = i; ii <= i + 1; ++ii)
+          if (gfluid(G, ii, jj, kk)) vs = vs + G.vol;
+    const double av = G.no_k ? 0.25 : 0.125;
+    vn = av * (fv(i, j, k) + fv(i + 1, j, k) + fv(i, j + 1, k) + fv(i + 1, j + 1, k));
+    if (!G.no_k)
+      vn = vn + av * (fv(i, j, k + 1) + fv(i + 1, j + 1, k + 1) + fv(i, j + 1, k + 1) + fv(i + 1, j, k + 1));
+  }
+  vol_surr[c] = vs;
+  vol_node[c] = vn;
+}
+
 // PARTICLES_IN_CELL; `located`: the integration has done the cell search.
 static int run_pic(dem_handle* h, bool located = false) {
   Gas* s = h->gas;
@@ -775,15 +799,26 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
     return set_err(h, DEM_ERR_ARG, "unknown drag_model");
   if (g->drag_model == DEM_DRAG_SINGLE_SPHERE && !(g->usr_d_p0 > 0.0))
     return set_err(h, DEM_ERR_ARG, "usr_d_p0 must be positive for the single-sphere drag");
-  free_gas(h);
-  Gas* s = new Gas();
-  h->gas = s;
+  const int gi2 = g->imax + 2, gj2 = g->jmax + 2, gk2 = h->dp.no_k ? 1 : g->kmax + 2;
+  // a coupled driver sets the fields of every fluid step: the arrays stay
+  // while their sizes do
+  // (a fluid step of ten DEM steps with 60,000 spheres: 4.8 ms with 20
+  // allocations and the grid volumes summed on the host, 0.97 ms so)
+  Gas* s = h->gas;
+  if (s && !(s->gi2 == gi2 && s->gj2 == gj2 && s->gk2 == gk2 && s->g.kmax == g->kmax && s->M == h->dp.nph &&
+             (s->p_force != nullptr) == (p_force != nullptr))) {
+    free_gas(h);
+    s = nullptr;
+  }
+  const bool fresh = !s;
+  if (fresh) h->gas = s = new Gas();
   s->g = *g;
-  s->gi2 = g->imax + 2; s->gj2 = g->jmax + 2; s->gk2 = h->dp.no_k ? 1 : g->kmax + 2;
-  s->ncell = s->gi2 * s->gj2 * s->gk2;
+  s->gi2 = gi2; s->gj2 = gj2; s->gk2 = gk2;
+  s->ncell = gi2 * gj2 * gk2;
   s->M = h->dp.nph;
   s->pi = 4.0 * std::atan(1.0);
   s->vol = g->dx * g->dy * (h->dp.no_k ? (h->prm.domain_hi[2] - h->prm.domain_lo[2]) : g->dz);
+  s->have_mean = false;
   const size_t nc = s->ncell;
   // face positions, accumulated as the fluid grid set-up does
   auto faces = [](double lo, double d, int n) {
@@ -795,62 +830,33 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
   std::vector<double> fx = faces(h->prm.domain_lo[0], g->dx, g->imax);
   std::vector<double> fy = faces(h->prm.domain_lo[1], g->dy, g->jmax);
   std::vector<double> fz = faces(h->prm.domain_lo[2], g->dz, h->dp.no_k ? 0 : g->kmax);
-  // VOL_SURR (make_arrays_des.f:78-105)
-  auto fluid = [&](int i, int j, int k) {
-    return i >= 2 && i <= g->imax + 1 && j >= 2 && j <= g->jmax + 1 &&
-           (h->dp.no_k ? k == 1 : (k >= 2 && k <= g->kmax + 1));
-  };
-  auto cidx = [&](int i, int j, int k) { return (i - 1) + (j - 1) * s->gi2 + (k - 1) * s->gi2 * s->gj2; };
-  std::vector<double> vs(nc, 0.0);
-  const int nk1 = h->dp.no_k ? 1 : g->kmax + 1;
-  for (int k = 1; k <= nk1; ++k)
-    for (int j = 1; j <= g->jmax + 1; ++j)
-      for (int i = 1; i <= g->imax + 1; ++i) {
-        double v = 0.0;
-        for (int kk = k; kk <= (h->dp.no_k ? k : k + 1); ++kk)
-          for (int jj = j; jj <= j + 1; ++jj)
-            for (int ii = i; ii <= i + 1; ++ii)
-              if (fluid(ii, jj, kk)) v = v + s->vol;
-        vs[cidx(i, j, k)] = v;
-      }
-  // DES_VOL_NODE (cfassign.f:104-228): a quarter (2D) or an eighth (3D) of
-  // each fluid cell sharing the node, summed in the reference's order
-  std::vector<double> vn(nc, 0.0);
-  const double avn = h->dp.no_k ? 0.25 : 0.125;
-  auto fv = [&](int i, int j, int k) { return fluid(i, j, k) ? s->vol : 0.0; };
-  for (int k = 1; k <= nk1; ++k)
-    for (int j = 1; j <= g->jmax + 1; ++j)
-      for (int i = 1; i <= g->imax + 1; ++i) {
-        double v = avn * (fv(i, j, k) + fv(i + 1, j, k) + fv(i, j + 1, k) + fv(i + 1, j + 1, k));
-        if (!h->dp.no_k)
-          v = v + avn * (fv(i, j, k + 1) + fv(i + 1, j + 1, k + 1) + fv(i, j + 1, k + 1) + fv(i + 1, j, k + 1));
-        vn[cidx(i, j, k)] = v;
-      }
-  bool ok = true;
-  auto A = [&](void** p, size_t b) { if (ok && cudaMalloc(p, b ? b : 8) != cudaSuccess) ok = false; };
-  A((void**)&s->xe, sizeof(double) * fx.size());
-  A((void**)&s->yn, sizeof(double) * fy.size());
-  A((void**)&s->zt, sizeof(double) * fz.size());
-  A((void**)&s->ep_g, sizeof(double) * nc);
-  A((void**)&s->u_g, sizeof(double) * nc);
-  A((void**)&s->v_g, sizeof(double) * nc);
-  A((void**)&s->w_g, sizeof(double) * nc);
-  if (p_force) A((void**)&s->p_force, sizeof(double) * 3 * nc);
-  A((void**)&s->vol_surr, sizeof(double) * nc);
-  A((void**)&s->rop_s, sizeof(double) * nc * s->M);
-  A((void**)&s->dens_node, sizeof(double) * nc * s->M);
-  A((void**)&s->vol_node, sizeof(double) * nc);
-  A((void**)&s->drag_am, sizeof(double) * nc);
-  A((void**)&s->drag_bm, sizeof(double) * 3 * nc);
-  A((void**)&s->f_gds, sizeof(double) * nc);
-  A((void**)&s->pijk, sizeof(int4) * (size_t)h->n);
-  A((void**)&s->f_gp, sizeof(double) * (size_t)h->n);
-  A((void**)&s->pic_cnt, sizeof(int) * (nc + 1));
-  A((void**)&s->pic_start, sizeof(int) * (nc + 1));
-  A((void**)&s->pic_tmp, sizeof(int) * (size_t)h->n);
-  A((void**)&s->pic_list, sizeof(int) * (size_t)h->n);
-  A((void**)&s->pic_dat, sizeof(double4) * (size_t)h->n);
-  if (!ok) { free_gas(h); return set_err(h, DEM_ERR_CUDA, "cudaMalloc gas fields"); }
+  if (fresh) {
+    bool ok = true;
+    auto A = [&](void** p, size_t b) { if (ok && cudaMalloc(p, b ? b : 8) != cudaSuccess) ok = false; };
+    A((void**)&s->xe, sizeof(double) * fx.size());
+    A((void**)&s->yn, sizeof(double) * fy.size());
+    A((void**)&s->zt, sizeof(double) * fz.size());
+    A((void**)&s->ep_g, sizeof(double) * nc);
+    A((void**)&s->u_g, sizeof(double) * nc);
+    A((void**)&s->v_g, sizeof(double) * nc);
+    A((void**)&s->w_g, sizeof(double) * nc);
+    if (p_force) A((void**)&s->p_force, sizeof(double) * 3 * nc);
+    A((void**)&s->vol_surr, sizeof(double) * nc);
+    A((void**)&s->rop_s, sizeof(double) * nc * s->M);
+    A((void**)&s->dens_node, sizeof(double) * nc * s->M);
+    A((void**)&s->vol_node, sizeof(double) * nc);
+    A((void**)&s->drag_am, sizeof(double) * nc);
+    A((void**)&s->drag_bm, sizeof(double) * 3 * nc);
+    A((void**)&s->f_gds, sizeof(double) * nc);
+    A((void**)&s->pijk, sizeof(int4) * (size_t)h->n);
+    A((void**)&s->f_gp, sizeof(double) * (size_t)h->n);
+    A((void**)&s->pic_cnt, sizeof(int) * (nc + 1));
+    A((void**)&s->pic_start, sizeof(int) * (nc + 1));
+    A((void**)&s->pic_tmp, sizeof(int) * (size_t)h->n);
+    A((void**)&s->pic_list, sizeof(int) * (size_t)h->n);
+    A((void**)&s->pic_dat, sizeof(double4) * (size_t)h->n);
+    if (!ok) { free_gas(h); return set_err(h, DEM_ERR_CUDA, "cudaMalloc gas fields"); }
+  }
   cudaMemcpyAsync(s->xe, fx.data(), sizeof(double) * fx.size(), cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(s->yn, fy.data(), sizeof(double) * fy.size(), cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(s->zt, fz.data(), sizeof(double) * fz.size(), cudaMemcpyHostToDevice, h->stream);
@@ -859,8 +865,8 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
   cudaMemcpyAsync(s->v_g, v_g, sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(s->w_g, w_g, sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream);
   if (p_force) cudaMemcpyAsync(s->p_force, p_force, sizeof(double) * 3 * nc, cudaMemcpyHostToDevice, h->stream);
-  cudaMemcpyAsync(s->vol_surr, vs.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream);
-  cudaMemcpyAsync(s->vol_node, vn.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream);
+  k_grid_volumes<<<(unsigned)((nc + 255) / 256), 256, 0, h->stream>>>(gas_view(h), s->vol_surr, s->vol_node);
+  DEM_LAUNCH(h);
   cudaMemsetAsync(s->pic_cnt, 0, sizeof(int) * (nc + 1), h->stream);
   cudaMemsetAsync(s->dens_node, 0, sizeof(double) * nc * s->M, h->stream);
   cudaMemsetAsync(s->drag_am, 0, sizeof(double) * nc, h->stream);

@@ -8,19 +8,26 @@ the oracle.
   not a multiple of four;
 - the scans take a second level past 4096 tiles of 2048 cells: a search grid
   just over it;
-- the contact counts of passes that integrate and passes that do not.
+- the contact counts of passes that integrate and passes that do not;
+- gas fields set again, on the same grid (the arrays are kept) and on another.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
-velocities 1e-3 of the largest).
+velocities 1e-3 of the largest); coupled states to 1e-10 relative, since the
+drag calls pow.
 """
 import numpy as np
 import pytest
 
-from cases import settling_case, state_arrays
+from cases import coupled_case, make_coupled, settling_case, state_arrays
 from gpu_util import compare_pairs, compare_state, pair_both, rel_err
 
 pytestmark = pytest.mark.gpu
+
+
+def _gpu(p, n):
+    from mfix_dem import GpuSystem
+    return GpuSystem(p, n)
 
 
 def _chain(m, precision, nsn=10):
@@ -129,3 +136,24 @@ def test_contact_counts_of_mixed_passes():
         s.step(13, nn_first=6)
     same()
     compare_state(g, o, exact=True)
+
+
+@pytest.mark.parametrize("interp", ["GARG_2012", "NONE"])
+def test_gas_fields_set_again(interp):
+    from mfix_dem import configs
+    from oracle_ffi import OracleSystem
+    ct = coupled_case(interp=interp)
+    g, o = make_coupled(_gpu, ct), make_coupled(OracleSystem, ct)
+    grid, f = ct[5], ct[6]
+    coarse = configs.coupled(n=1500, cells=(4, 12, 4), dx=2e-3, interp=interp)[5:7]
+    for again in ((grid, f), (grid, {k: v * (1.0 if k == "ep_g" else 0.7) for k, v in f.items()}), coarse, (grid, f)):
+        for s in (g, o):
+            s.step_coupled(7)
+            s.set_gas_fields(again[0], again[1]["ep_g"], again[1]["u_g"], again[1]["v_g"], again[1]["w_g"])
+            s.step_coupled(6)
+        compare_state(g, o)
+        for a, b in zip(g.get_mean_fields(), o.get_mean_fields()):
+            assert rel_err(a, b) <= 1e-10
+        call = "drag_gs_gas1" if interp == "NONE" else "drag_gs_gas0"
+        for a, b in zip(getattr(g, call)(), getattr(o, call)()):
+            assert rel_err(a, b) <= 1e-10
