@@ -67,7 +67,7 @@ struct CandState {
 
 // Contacts of a split-precision pair pass whose onset-of-slip test lies
 // near its threshold (force_split.cu): 2 * pair index + 1 when the pair
-// had a history.  The count starts at zero and k_slip_fix, which follows
+// had a history.  The count starts at zero and the split gather, which follows
 // every pass, clears it; past SLIP_FIX_CAP a contact keeps its FP32
 // decision.
 constexpr int SLIP_FIX_CAP = 4096;

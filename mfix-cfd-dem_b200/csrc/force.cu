@@ -949,7 +949,11 @@ static void launch_gather_fp64(dem_handle* h, int mode) {
 
 // The two timed parts of the force step for the autotuner.
 void launch_pairs_only(dem_handle* h) {
-  if (h->dp.prec == DEM_PREC_SPLIT) launch_pairs_split(h);
+  if (h->dp.prec == DEM_PREC_SPLIT) {
+    // no gather in between that would clear the slip list
+    cudaMemsetAsync(&h->slipfix->count, 0, sizeof(unsigned), h->stream);
+    launch_pairs_split(h);
+  }
   else if (h->batch()) launch_pairs_fp64<true>(h, false);
   else launch_pairs_fp64<false>(h, false);
 }

@@ -339,13 +339,18 @@ k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long lon
   }
 }
 
+constexpr int FIX_T = 32, FIX_BLOCKS = 64;
+
 // The contacts k_pairs_split left near the onset of slip, evaluated again
 // with the onset decided in FP64 (slip_fp64): history, flag and both
 // records rewritten.  Their history is still the one the pair kernel read.
-// One block; it clears the count for the next pair pass when done.
+// A few contacts each, all blocks' chains of loads and FP64 arithmetic side by
+// side: one block of 128 threads took 6-12 us behind every pair pass, and a
+// step of the bed of 1,000,000 spheres 278 us, 264 us so.  The gather clears
+// the count for the next pass.
 template <int COLL, bool B>
-__global__ void __launch_bounds__(128)
-k_slip_fix(DevParams p0, BatchView bv, SlipFix* __restrict__ fix, const int* __restrict__ owner,
+__global__ void __launch_bounds__(FIX_T)
+k_slip_fix(DevParams p0, BatchView bv, const SlipFix* __restrict__ fix, const int* __restrict__ owner,
            const int* __restrict__ nbrs, const int* __restrict__ in_pos, const double4* __restrict__ pos4,
            const double4* __restrict__ vel4, const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
            double* __restrict__ pft, long long cap, uint8_t* __restrict__ pflag, Rec32* __restrict__ rec_own,
@@ -353,7 +358,7 @@ k_slip_fix(DevParams p0, BatchView bv, SlipFix* __restrict__ fix, const int* __r
   const int z = pdl_wait();
   pdl_next();
   const unsigned n = min(fix[z].count, (unsigned)SLIP_FIX_CAP);
-  for (unsigned t = threadIdx.x; t < n; t += blockDim.x) {
+  for (unsigned t = blockIdx.x * FIX_T + threadIdx.x; t < n; t += FIX_BLOCKS * FIX_T) {
     const long long code = fix->pair[t];
     const long long cc = code >> 1;
     const int ll = owner[cc], i = nbrs[cc];
@@ -373,8 +378,6 @@ k_slip_fix(DevParams p0, BatchView bv, SlipFix* __restrict__ fix, const int* __r
     put_records(o, cc, in_pos, rec_own, rec_in);
     pflag[cc] = PF_CONTACT | ((ot[0] != 0.0 || ot[1] != 0.0 || ot[2] != 0.0) ? PF_HIST : 0);
   }
-  __syncthreads();  // every thread has read the count
-  if (threadIdx.x == 0) fix->count = 0;
 }
 
 // Compensated sums of a particle's records.
@@ -485,11 +488,12 @@ k_gather_split(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, co
                const int* __restrict__ in_start, const uint8_t* __restrict__ pflag, const uint8_t* __restrict__ in_flag,
                const Rec32* __restrict__ rec_own, const Rec32* __restrict__ rec_in, double* __restrict__ fc,
                double* __restrict__ tow, double* __restrict__ acc_old, double* __restrict__ rot_acc_old,
-               unsigned* __restrict__ vslot, CellOut cells, StepEnd end) {
+               unsigned* __restrict__ vslot, CellOut cells, StepEnd end, SlipFix* __restrict__ fix) {
   __shared__ SplitShared s_sh[SPLIT_T / 32];
   const int z = pdl_wait();
   pdl_next();
   if (MODE != 0) end_step(end);
+  if (blockIdx.x == 0 && threadIdx.x == 0) fix->count = 0;
   const int at = blockIdx.x * blockDim.x + threadIdx.x + z;
   const bool mine = at < p0.n;
   const int me = mine ? at : p0.n - 1;  // the lanes past the end help with the warp's records only
@@ -563,7 +567,7 @@ static void launch_pairs_split_t(dem_handle* h) {
              h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c], h->omg4[c], h->state,
              h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin, h->vslot_pending(),
              rec_own_of(h), rec_in_of(h), h->slipfix, &h->derr->count[c], h->derr);
-  launch_pdl(h, k_slip_fix<COLL, B>, 1, 128, h->dp, h->bview(), h->slipfix, h->pair_owner, h->nbrs[h->rb], h->in_pos,
+  launch_pdl(h, k_slip_fix<COLL, B>, FIX_BLOCKS, FIX_T, h->dp, h->bview(), h->slipfix, h->pair_owner, h->nbrs[h->rb], h->in_pos,
              h->pos4[c], h->vel4[c], h->omg4[c], h->phase, h->pft[h->pcur], h->pair_cap, h->pflag(), rec_own_of(h),
              rec_in_of(h));
 }
@@ -581,7 +585,7 @@ static void launch_gather_split_t(dem_handle* h) {
   launch_pdl(h, k_gather_split<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
              h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->wall_hit, h->touched, h->row_end[h->rb], h->in_start,
              h->pflag(), h->in_flag, rec_own_of(h), rec_in_of(h), h->fc, h->tow, h->acc_old, h->rot_acc_old,
-             h->vslot_note(), gather_cells<MODE, B>(h), step_end(h));
+             h->vslot_note(), gather_cells<MODE, B>(h), step_end(h), h->slipfix);
 }
 
 void launch_gather_split(dem_handle* h, int mode) {
