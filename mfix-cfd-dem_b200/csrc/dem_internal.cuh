@@ -285,6 +285,29 @@ struct dem_handle {
     int gather_threads = 256;               // gather kernel: threads per block
     int neigh_threads = 128;                // pair-build scan: threads per block
   } tune;
+  bool tuned = false;         // the shapes were measured or set; otherwise pair_shape chooses
+  // Launch shape of the FP64 pair kernel, which keeps `resident` threads on a
+  // multiprocessor.  With eight windows of pairs or more for each resident
+  // warp: blocks of two warps, as many as fit the device once, since a second
+  // wave of these persistent blocks only waits for the first and small blocks
+  // end more evenly (the bed of 1,000,000 spheres, 34,000 windows: 354 us per
+  // step against 365 with 1184 blocks of eight warps).  With fewer: blocks of
+  // eight warps, whose neighbouring windows share an L1 (coupled bed of 500,000,
+  // five windows a warp: 281 us per step against 288 in blocks of two; gas of
+  // 200,003, less than one: 60 us against 66).  The split kernel, with twice
+  // the warps, gains nothing from small blocks (a batch of columns loses 1 %).
+  // The loops over the list take any grid.
+  struct Shape {
+    int threads, blocks;
+  };
+  Shape pair_shape(int resident) const {
+    if (!tuned && n_pairs / 128 >= 8ll * n_sm * resident / 32) return {64, n_sm * (resident / 64)};
+    return {tune.pair_threads, n_sm * tune.pair_bpsm};
+  }
+  // Threads of a block of the gathers: a block leaves when its slowest warp
+  // does, so small ones refill sooner (1 % of a step of a bed of 150,001 and of
+  // one of 1,000,000 against blocks of 256).
+  int gather_block() const { return tuned ? tune.gather_threads : 128; }
   bool capturing = false;     // inside a CUDA graph capture: no host syncs
   cudaStream_t own_stream = nullptr;
   // the wall kernels of a force pass run on side_stream beside the pair

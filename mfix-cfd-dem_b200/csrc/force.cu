@@ -892,10 +892,11 @@ static void launch_walls_t(dem_handle* h) {
 template <int COLL, bool B>
 static void launch_pairs_t(dem_handle* h, bool walls) {
   const int c = h->cur;
-  const int T = h->tune.pair_threads;
+  const dem_handle::Shape sh = h->pair_shape(512);  // 128 registers
+  const int T = sh.threads;
   const WallArgs wa = wall_args(h, T);
   auto go = [&](auto kernel) {
-    launch_pdl(h, kernel, (unsigned)(h->n_sm * h->tune.pair_bpsm + (walls ? wa.blocks : 0)), T, h->dp, h->bview(), wa,
+    launch_pdl(h, kernel, (unsigned)(sh.blocks + (walls ? wa.blocks : 0)), T, h->dp, h->bview(), wa,
                h->d_np, h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c], h->omg4[c],
                h->state, h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin,
                h->vslot_pending(), h->recs(), &h->derr->count[c], h->derr);
@@ -907,7 +908,7 @@ static void launch_pairs_t(dem_handle* h, bool walls) {
 
 template <int MODE, bool B>
 static void launch_gather_t(dem_handle* h) {
-  const int T = h->tune.gather_threads, G = (h->nl() + T - 1) / T;
+  const int T = h->gather_block(), G = (h->nl() + T - 1) / T;
   const int c = h->cur;
   launch_pdl(h, k_gather<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
              h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start, h->in_mid, h->in_pair,

@@ -59,6 +59,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   if (reps < 1) return set_err(h, DEM_ERR_ARG, "reps must be positive");
   if (!h->have_state || !h->have_pairs) return set_err(h, DEM_ERR_STATE, "state or pair list missing");
   invalidate_graphs(h);
+  h->tuned = true;
   const size_t P = (size_t)host_pairs(h);
   char* snap = (char*)stage_buffer(h, sizeof(double) * 3 * P + 2 * P + 64);
   if (!snap) return set_err(h, DEM_ERR_CUDA, "cudaMalloc stage");
@@ -129,6 +130,7 @@ int dem_set_tuning(dem_handle* h, const dem_tuning* in) {
   h->tune.pair_bpsm = in->pair_blocks_per_sm;
   h->tune.gather_threads = in->gather_threads;
   h->tune.neigh_threads = in->neigh_threads;
+  h->tuned = true;
   invalidate_graphs(h);
   return 0;
 }

@@ -9,7 +9,9 @@ the oracle.
 - the scans take a second level past 4096 tiles of 2048 cells: a search grid
   just over it;
 - the contact counts of passes that integrate and passes that do not;
-- gas fields set again, on the same grid (the arrays are kept) and on another.
+- gas fields set again, on the same grid (the arrays are kept) and on another;
+- the FP64 pair kernel in small blocks, for lists that keep every resident warp
+  busy for eight windows, against the larger ones.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -19,7 +21,7 @@ drag calls pow.
 import numpy as np
 import pytest
 
-from cases import coupled_case, make_coupled, settling_case, state_arrays
+from cases import coupled_case, make_coupled, make_system, settling_case, state_arrays
 from gpu_util import compare_pairs, compare_state, pair_both, rel_err
 
 pytestmark = pytest.mark.gpu
@@ -30,7 +32,7 @@ def _gpu(p, n):
     return GpuSystem(p, n)
 
 
-def _chain(m, precision, nsn=10):
+def _chain(m, precision, nsn=10, rho=2500.0, kn=1000.0, intg="EULER"):
     """m + 1 spheres of 1 mm in a row along x, 0.98 d apart: m pairs, each in
     contact at the start, with small seeded velocities across the row."""
     from mfix_dem import params as P
@@ -40,9 +42,9 @@ def _chain(m, precision, nsn=10):
     pos[0] = (np.arange(n) + 2.0) * 0.98 * d
     pos[1] = pos[2] = 4.0 * d
     vel = rng.uniform(-0.02, 0.02, (3, n))
-    arr = state_arrays(pos, vel, np.zeros((3, n)), np.full(n, 0.5 * d), np.full(n, 2500.0))
+    arr = state_arrays(pos, vel, np.zeros((3, n)), np.full(n, 0.5 * d), np.full(n, rho))
     hi = ((n + 4.0) * d, 8.0 * d, 8.0 * d)
-    case = P.DemCase(d_p0=(d,), ro_s0=(2500.0,), coll_model="LSD", kn=1000.0, kn_w=1000.0, des_en_input=0.9,
+    case = P.DemCase(d_p0=(d,), ro_s0=(rho,), coll_model="LSD", kn=kn, kn_w=kn, des_en_input=0.9, intg_method=intg,
                      des_en_wall_input=[0.9], mew=0.2, mew_w=0.2, mew_r=0.01, mew_rw=0.01, domain_hi=hi,
                      neighbor_search_n=nsn, force_precision=precision)
     prm, _ = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
@@ -157,3 +159,18 @@ def test_gas_fields_set_again(interp):
         call = "drag_gs_gas1" if interp == "NONE" else "drag_gs_gas0"
         for a, b in zip(getattr(g, call)(), getattr(o, call)()):
             assert rel_err(a, b) <= 1e-10
+
+
+def test_dense_list_in_small_blocks():
+    """847,872 touching spheres: past eight windows of 128 pairs for each of
+    the 16 warps that a multiprocessor (of 148) keeps."""
+    n_side = (96, 92, 96)
+    case, prm, arr, walls = settling_case(n_side=n_side, box=tuple(1.0e-3 * (k + 2) for k in n_side), spacing=0.98,
+                                          jitter=0.01, vmax=0.1, nsn=5, seed=7)
+    a, b = make_system(_gpu, prm, arr, walls), make_system(_gpu, prm, arr, walls)
+    b.set_tuning({"pair_threads": 256, "pair_blocks_per_sm": 8, "gather_threads": 256, "neigh_threads": 128})
+    for s in (a, b):
+        s.step(7)
+    assert a.pair_count() >= 8 * 128 * 16 * 148
+    compare_state(a, b, exact=True)
+    assert a.stats()["n_contacts"] == b.stats()["n_contacts"] > a.pair_count() // 2
