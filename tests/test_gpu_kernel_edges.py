@@ -11,7 +11,8 @@ the oracle.
 - the contact counts of passes that integrate and passes that do not;
 - gas fields set again, on the same grid (the arrays are kept) and on another;
 - the FP64 pair kernel in small blocks, for lists that keep every resident warp
-  busy for eight windows, against the larger ones.
+  busy for eight windows, against the larger ones;
+- contact lists of more than 32 entries, and warps with more than 128.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -174,3 +175,43 @@ def test_dense_list_in_small_blocks():
     assert a.pair_count() >= 8 * 128 * 16 * 148
     compare_state(a, b, exact=True)
     assert a.stats()["n_contacts"] == b.stats()["n_contacts"] > a.pair_count() // 2
+
+
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+@pytest.mark.parametrize("big", [0, -1])
+def test_long_contact_lists(big, prec):
+    """A sphere of 10 mm with 80 of 1 mm touching it (numbered first: a row of
+    80 pairs; last: 80 incoming ones) beside a block of 8^3 with up to six
+    contacts each."""
+    from mfix_dem import abi
+    from mfix_dem import params as P
+    R, r = 5e-3, 0.5e-3
+    k = np.arange(80) + 0.5
+    up, turn = 1.0 - 2.0 * k / 80, np.pi * (1.0 + 5.0 ** 0.5) * k
+    ring = np.sqrt(1.0 - up * up)
+    shell = 8e-3 + 0.999 * (R + r) * np.stack([ring * np.cos(turn), up, ring * np.sin(turn)])
+    a = np.arange(8) * 0.98 * 2.0 * r
+    block = np.stack(np.meshgrid(a, a, a, indexing="ij")).reshape(3, -1) + np.array([[20e-3], [4e-3], [4e-3]])
+    small = np.concatenate([shell, block], axis=1)
+    rng = np.random.default_rng(41)
+    pos = np.concatenate([np.full((3, 1), 8e-3), small], axis=1)
+    rad = np.concatenate([[R], np.full(small.shape[1], r)])
+    if big == -1:
+        pos, rad = np.roll(pos, -1, axis=1), np.roll(rad, -1)
+    n = rad.size
+    arr = state_arrays(pos, rng.uniform(-0.02, 0.02, (3, n)), np.zeros((3, n)), rad, np.full(n, 2500.0))
+    hi = (32e-3, 16e-3, 16e-3)
+    case = P.DemCase(d_p0=(2.0 * r,), ro_s0=(2500.0,), coll_model="LSD", kn=1000.0, kn_w=1000.0, des_en_input=0.9,
+                     des_en_wall_input=[0.9], mew=0.2, mew_w=0.2, mew_r=0.01, mew_rw=0.01, domain_hi=hi,
+                     neighbor_search_n=10, force_precision=abi.DEM_PREC_SPLIT if prec == "split" else abi.DEM_PREC_FP64)
+    prm, _ = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
+    g, o = pair_both(prm, arr, P.default_walls((0.0, 0.0, 0.0), hi))
+    for steps in (1, 2, 20):
+        g.step(steps)
+        o.step(steps)
+        if prec == "fp64":
+            compare_state(g, o, exact=True)
+            compare_pairs(g, o)
+    sg, so = g.download_state(), o.download_state()
+    assert rel_err(sg["pos"], so["pos"]) <= 1e-6
+    assert rel_err(sg["vel"], so["vel"]) <= 1e-3
