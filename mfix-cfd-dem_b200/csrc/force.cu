@@ -55,13 +55,26 @@ __device__ __forceinline__ void contact_force(const DevParams& p, const PState& 
   const double rl = L.r, ri = I.r;
   const double r_lm = rl + ri;
   const double dmag = sqrt(d2);
-  double nrm[3] = {dist[0] / dmag, dist[1] / dmag, dist[2] / dmag};
+  // the normal and the two lever arms, all divided by dmag (half a quotient is
+  // the quotient by twice the divisor)
+  const double num_dcl = dmag * dmag + rl * rl - ri * ri, num_dcl2 = rl * rl - ri * ri;
+  const double y_dmag = 1.0 / dmag;
+  double nrm[3], dcl, half;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) nrm[c] = quotient(dist[c], dmag, y_dmag);
+  dcl = 0.5 * quotient(num_dcl, dmag, y_dmag);
+  half = 0.5 * quotient(num_dcl2, dmag, y_dmag);
+  if (!div_range(dmag, fabs(dcl) + fabs(half))) {  // |nrm| is at most one
+#pragma unroll
+    for (int c = 0; c < 3; ++c) nrm[c] = dist[c] / dmag;
+    dcl = num_dcl / (2.0 * dmag);
+    half = num_dcl2 / (2.0 * dmag);
+  }
   const double overlap_n = r_lm - dmag;
   // CFRELVEL
   double vrel[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) vrel[c] = L.v[c] - I.v[c];
-  const double dcl = (dmag * dmag + rl * rl - ri * ri) / (2.0 * dmag);
   const double dci = dmag - dcl;
   double osum[3];
 #pragma unroll
@@ -105,8 +118,7 @@ __device__ __forceinline__ void contact_force(const DevParams& p, const PState& 
     const double fnmd = p.mew * sqrt(dot3(fn, fn));
     if (ftmd > fnmd) {
       double tg[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) tg[c] = ot[c] / mag;
+      div3(ot, mag, tg);
 #pragma unroll
       for (int c = 0; c < 3; ++c) ft[c] = -fnmd * tg[c];
 #pragma unroll
@@ -116,7 +128,7 @@ __device__ __forceinline__ void contact_force(const DevParams& p, const PState& 
     ft[0] = ft[1] = ft[2] = 0.0;
   }
   pout[0] = ot[0]; pout[1] = ot[1]; pout[2] = ot[2];
-  o.dcl2 = dmag / 2.0 + (rl * rl - ri * ri) / (2.0 * dmag);
+  o.dcl2 = dmag / 2.0 + half;
   o.dci2 = dmag - o.dcl2;
   cross3(nrm, ft, o.tf);
 #pragma unroll
@@ -305,7 +317,7 @@ __device__ int wall_contacts(const DevParams& p, const WallCtx& w, int me, const
       const int ph = phase[me];
       const double distmod = sqrt(distsq);
       double nrm[3] = {dist[0], dist[1], dist[2]};
-      if (distsq > 0) { const double sq = sqrt(distsq); for (int c = 0; c < 3; ++c) nrm[c] = dist[c] / sq; }
+      if (distsq > 0) div3(dist, distmod, nrm);
       const double overlap_n = r - distmod;
       double wxn[3]; cross3(sw, nrm, wxn);
       double vrel[3];
@@ -341,8 +353,7 @@ __device__ int wall_contacts(const DevParams& p, const WallCtx& w, int me, const
         const double fnmd = p.mew_w * sqrt(dot3(fn, fn));
         if (ftmd > fnmd) {
           double tg[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) tg[c] = ot[c] / mag;
+          div3(ot, mag, tg);
 #pragma unroll
           for (int c = 0; c < 3; ++c) ft[c] = -fnmd * tg[c];
 #pragma unroll
@@ -360,7 +371,10 @@ __device__ int wall_contacts(const DevParams& p, const WallCtx& w, int me, const
         if (om > 0.0) {
           terms = 2;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) rl[c] = -(p.mew_rw * (2.0 * r) * kn_w * overlap_n * sw[c] / om);
+          for (int c = 0; c < 3; ++c) rl[c] = p.mew_rw * (2.0 * r) * kn_w * overlap_n * sw[c];
+          div3(rl, om, rl);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) rl[c] = -rl[c];
         }
       }
     }
@@ -715,23 +729,28 @@ k_pairs(DevParams p0, BatchView bv, WallArgs wa, const int* __restrict__ d_np, l
 }
 
 // Rolling-friction torque of one particle in a pair (calc_force_dem.f:491-506):
-// -MEW_R*(2*R)*KN_DES*OVERLAP_N*OMEGA/|OMEGA|, evaluated left to right.
-__device__ __forceinline__ void add_rolling(const DevParams& p, double r, const double w[3], double om,
+// -MEW_R*(2*R)*KN_DES*OVERLAP_N*OMEGA/|OMEGA|, evaluated left to right; om is
+// |OMEGA| and its reciprocal, the same for all of the particle's contacts.
+__device__ __forceinline__ void add_rolling(const DevParams& p, double r, const double w[3], double2 om,
                                             const PairRec& q, double t[3]) {
+  const double a = p.mew_r * (2.0 * r) * q.kn * q.ov;
+  const double aw[3] = {a * w[0], a * w[1], a * w[2]};
+  double d[3];
+  div3(aw, om.x, om.y, d);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) t[c] = t[c] + -(p.mew_r * (2.0 * r) * q.kn * q.ov * w[c] / om);
+  for (int c = 0; c < 3; ++c) t[c] = t[c] + -d[c];
 }
 
 // One pair's terms on one of its particles: the owner adds +FC and DCL2*TF,
 // the neighbour -FC and DCI2*TF (calc_force_dem.f:466-506).
 template <bool NBR>
 __device__ __forceinline__ void add_pair_terms(const DevParams& p, const PairRec& o, bool roll, double r,
-                                               const double w[3], double om, double f[3], double t[3]) {
+                                               const double w[3], double2 om, double f[3], double t[3]) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) f[c] = NBR ? f[c] - o.fc[c] : f[c] + o.fc[c];
 #pragma unroll
   for (int c = 0; c < 3; ++c) t[c] = t[c] + (NBR ? o.dci2 : o.dcl2) * o.tf[c];
-  if (roll && om > 0.0) add_rolling(p, r, w, om, o, t);
+  if (roll && om.x > 0.0) add_rolling(p, r, w, om, o, t);
 }
 
 __device__ __forceinline__ PairRec load_record(const RecStore& rec, int cc, bool roll) {
@@ -753,7 +772,7 @@ __device__ __forceinline__ PairRec load_record(const RecStore& rec, int cc, bool
 template <bool NBR>
 __device__ __forceinline__ void add_range(const DevParams& p, int q, int e, const uint8_t* __restrict__ flags,
                                           const int2* __restrict__ in_pair, const RecStore& rec, bool roll, double r,
-                                          const double w[3], double om, double f[3], double t[3]) {
+                                          const double w[3], double2 om, double f[3], double t[3]) {
   for (int base = q; base < e; base += 32) {
     unsigned mask = contact_mask(flags, base, min(32, e - base));
     if (!mask) continue;
@@ -817,8 +836,8 @@ k_gather(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, const do
   if (st != DEM_STATE_NONEXISTENT && ph) {
     const bool roll = p.mew_r > 0.0;
     const double r = pos_c[me].w;
-    double om = 0.0;
-    if (roll) om = sqrt(dot3(w, w));
+    double2 om = make_double2(0.0, 0.0);
+    if (roll) { om.x = sqrt(dot3(w, w)); om.y = 1.0 / om.x; }
     const int is = in_start[me], ie = in_start[me + 1], mid = in_mid[me];
     add_range<true>(p, is, mid, in_flag, in_pair, rec, roll, r, w, om, f, t);
     add_range<false>(p, me ? row_end[me - 1] : 0, row_end[me], pflag, nullptr, rec, roll, r, w, om, f, t);

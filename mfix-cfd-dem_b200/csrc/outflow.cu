@@ -104,7 +104,7 @@ __global__ void k_integrate_outflow(DevParams p, const dem_outflow_bc* __restric
   }
   pos4[me] = make_double4(xn[0], xn[1], xn[2], X.w);
   vel4[me] = make_double4(ve[0], ve[1], ve[2], V.w);
-  note_displacement(vslot, fmax(speed(v), speed(ve)) * dt);
+  note_displacement(vslot, max_speed(v, ve) * dt);
 }
 
 // MASS_OUTFLOW_DEM (mass_outflow_dem.f:13-188) per particle, the boundaries

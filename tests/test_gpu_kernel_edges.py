@@ -12,7 +12,8 @@ the oracle.
 - gas fields set again, on the same grid (the arrays are kept) and on another;
 - the FP64 pair kernel in small blocks, for lists that keep every resident warp
   busy for eight windows, against the larger ones;
-- contact lists of more than 32 entries, and warps with more than 128.
+- contact lists of more than 32 entries, and warps with more than 128;
+- masses past the range in which quotients share a reciprocal.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -215,3 +216,19 @@ def test_long_contact_lists(big, prec):
     sg, so = g.download_state(), o.download_state()
     assert rel_err(sg["pos"], so["pos"]) <= 1e-6
     assert rel_err(sg["vel"], so["vel"]) <= 1e-3
+
+
+@pytest.mark.parametrize("intg", ["EULER", "ADAMS_BASHFORTH"])
+@pytest.mark.parametrize("scale", [1.0, 1e128])
+def test_quotients_of_large_masses(scale, intg):
+    """Density and stiffness times 1e128 (masses past 2^400): the same motion,
+    with the accelerations divided plainly."""
+    from mfix_dem import abi
+    g, o = pair_both(*_chain(70, abi.DEM_PREC_FP64, rho=2500.0 * scale, kn=1000.0 * scale, intg=intg))
+    for steps in (1, 2, 30):
+        g.step(steps)
+        o.step(steps)
+        assert o.stats()["n_contacts"] > 0 or steps == 30
+        compare_state(g, o, exact=True)
+        compare_pairs(g, o)
+    assert np.isfinite(g.download_state()["vel"]).all()
