@@ -602,34 +602,49 @@ __device__ __forceinline__ unsigned contact_mask(const uint8_t* __restrict__ fla
 
 // The pairs of a warp's window [c0, c0 + WIN_PAIRS) that a pair kernel has to
 // look at, as a queue in shared memory: pair offset in the window, PF_HIST
-// and PF_CONTACT of the last pass above it.  A pair whose gap at the build
-// exceeds `reach` (twice the displacement bound since, rounded up) with a
+// and PF_CONTACT of the last pass above it, and the two particles.  A pair
+// whose gap at the build exceeds `reach` (twice the displacement bound since, rounded up) with a
 // zero history is apart without a look at its particles: its flags are
 // cleared and it is left out.  A lane screens four consecutive pairs from one
 // load of flags and one of gaps; the queue then gives every lane a pair, so
 // the contact arithmetic and its gathers run on full warps (about 0.4 of a
-// dense bed's pairs are in contact).  Returns the queue's length, the same
-// in every lane.
+// dense bed's pairs are in contact).  The particles of all 128 pairs are loaded
+// with the flags, in whole lines: looked up for the queued pairs alone they
+// were one more round of loads in the chain (bed of 1,000,000 spheres 334 us
+// per step, 321 us so; split 249 and 244 us; a batch of 16 columns 111 and 108
+// us).  Returns the queue's length, the same in every lane.
+// Also tried: the queue carried over from window to window, so that only full
+// warps take from it (1 % faster in FP64, 5 % slower in split), and a block's
+// windows side by side over several turns (4 to 10 % slower): what counts is
+// that all blocks work at one place of the list, whose particles the L2 holds.
 constexpr int WIN_PAIRS = 128;
 constexpr int WQ_CONTACT = 1 << 7, WQ_HIST = 1 << 8;
+struct WinQueue {
+  int2 who[WIN_PAIRS];
+  uint16_t e[WIN_PAIRS];
+};
 __device__ __forceinline__ int screen_window(long long c0w, long long np, uint8_t* __restrict__ pflag,
                                              uint8_t* __restrict__ in_flag, const int* __restrict__ in_pos,
-                                             const float* __restrict__ pgap, float reach, uint16_t* queue) {
+                                             const float* __restrict__ pgap, const int* __restrict__ owner,
+                                             const int* __restrict__ nbrs, float reach, WinQueue* queue) {
   static_assert(PF_CONTACT << 7 == WQ_CONTACT && PF_HIST << 7 == WQ_HIST, "flags move up by seven bits");
   const int lane = threadIdx.x & 31;
   const long long c0 = c0w + 4 * lane;
   uint32_t fw = 0;  // the four flags, one per byte
   float g[4] = {0.f, 0.f, 0.f, 0.f};
-  int live = 4;
+  int live = 4, ow[4] = {0, 0, 0, 0}, nb[4] = {0, 0, 0, 0};
   if (c0 + 3 < np) {
     fw = *reinterpret_cast<const uint32_t*>(pflag + c0);
     const float4 gq = *reinterpret_cast<const float4*>(pgap + c0);
     g[0] = gq.x; g[1] = gq.y; g[2] = gq.z; g[3] = gq.w;
+    const int4 oq = *reinterpret_cast<const int4*>(owner + c0), nq = *reinterpret_cast<const int4*>(nbrs + c0);
+    ow[0] = oq.x; ow[1] = oq.y; ow[2] = oq.z; ow[3] = oq.w;
+    nb[0] = nq.x; nb[1] = nq.y; nb[2] = nq.z; nb[3] = nq.w;
   } else {
     live = c0 < np ? (int)(np - c0) : 0;
 #pragma unroll
     for (int j = 0; j < 3; ++j)
-      if (j < live) { fw |= (uint32_t)pflag[c0 + j] << (8 * j); g[j] = pgap[c0 + j]; }
+      if (j < live) { fw |= (uint32_t)pflag[c0 + j] << (8 * j); g[j] = pgap[c0 + j]; ow[j] = owner[c0 + j]; nb[j] = nbrs[c0 + j]; }
   }
   unsigned need = 0;
 #pragma unroll
@@ -653,8 +668,10 @@ __device__ __forceinline__ int screen_window(long long c0w, long long np, uint8_
   int at = incl - mine;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    if ((need >> j) & 1u)
-      queue[at++] = (uint16_t)((4 * lane + j) | (((fw >> (8 * j)) & (PF_CONTACT | PF_HIST)) << 7));
+    if ((need >> j) & 1u) {
+      queue->who[at] = make_int2(ow[j], nb[j]);
+      queue->e[at++] = (uint16_t)((4 * lane + j) | (((fw >> (8 * j)) & (PF_CONTACT | PF_HIST)) << 7));
+    }
   __syncwarp();
   return __shfl_sync(0xffffffffu, incl, 31);
 }

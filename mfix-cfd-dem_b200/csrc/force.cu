@@ -632,7 +632,7 @@ k_pairs(DevParams p0, BatchView bv, WallArgs wa, const int* __restrict__ d_np, l
         uint8_t* __restrict__ in_flag, uint8_t* __restrict__ touched, const float* __restrict__ pgap,
         const double* __restrict__ skin, const unsigned* __restrict__ pending, RecStore rec,
         ContactCount* __restrict__ count, DevErr* __restrict__ err) {
-  __shared__ uint16_t s_queue[256 / 32][WIN_PAIRS];
+  __shared__ WinQueue s_queue[256 / 32];
   const int z = pdl_wait();
   pdl_next();
   const double bound = displacement_bound(skin + z, pending + z);
@@ -651,16 +651,17 @@ k_pairs(DevParams p0, BatchView bv, WallArgs wa, const int* __restrict__ d_np, l
   const float reach = __double2float_ru(2.0 * bound);
   unsigned long long ncont = 0;
   unsigned eflags = 0;
-  uint16_t* queue = s_queue[threadIdx.x >> 5];
+  WinQueue* queue = &s_queue[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)WIN_PAIRS * ((blocks * (int)blockDim.x) >> 5);
   for (long long w0 = (long long)WIN_PAIRS * ((block * (int)blockDim.x + (int)threadIdx.x) >> 5) + z; w0 < np; w0 += stride) {
-    const int nq = screen_window(w0, np, pflag, in_flag, in_pos, pgap, reach, queue);
+    const int nq = screen_window(w0, np, pflag, in_flag, in_pos, pgap, owner, nbrs, reach, queue);
     for (int k = lane; k < nq; k += 32) {
-      const int e = queue[k];
+      const int e = queue->e[k];
       const long long cc = w0 + (e & (WIN_PAIRS - 1));
       const uint8_t f0 = (uint8_t)(e >> 7);
-      const int ll = owner[cc], i = nbrs[cc];
+      const int2 who = queue->who[k];
+      const int ll = who.x, i = who.y;
       uint8_t f = f0 & PF_HIST;  // NONEXISTENT partner or zero distance: history kept
       // the states and the positions in one round of loads (any slot's
       // position can be read; it is used only for existing particles)
