@@ -664,9 +664,16 @@ k_pairs(DevParams p0, BatchView bv, WallArgs wa, const int* __restrict__ d_np, l
       const int ll = who.x, i = who.y;
       uint8_t f = f0 & PF_HIST;  // NONEXISTENT partner or zero distance: history kept
       // the states and the positions in one round of loads (any slot's
-      // position can be read; it is used only for existing particles)
+      // position can be read; it is used only for existing particles), with
+      // the history and, for a contact of the last pass, which is nearly always
+      // one of this, the motion (1 % of a step of the beds)
       const double4 a = ld32(pos4 + ll), b = ld32(pos4 + i);
       const int8_t sl = state[ll], si = state[i];
+      double pin[3] = {0.0, 0.0, 0.0};
+      if (f0 & PF_HIST) { pin[0] = pft[cc]; pin[1] = pft[cap + cc]; pin[2] = pft[2 * cap + cc]; }
+      const bool was = f0 & PF_CONTACT;
+      double4 va, vb, wa, wb;
+      if (was) { va = ld32(vel4 + ll); vb = ld32(vel4 + i); wa = ld32(omg4 + ll); wb = ld32(omg4 + i); }
       if (si != DEM_STATE_NONEXISTENT && sl != DEM_STATE_NONEXISTENT) {
         const DevParams& p = sysp<B>(p0, bv, ll);
         PState L, I;
@@ -689,9 +696,7 @@ k_pairs(DevParams p0, BatchView bv, WallArgs wa, const int* __restrict__ d_np, l
           eflags |= EF_ZERO_DIST;
           err->zero_a = ll; err->zero_b = i;
         } else {
-          const double4 va = ld32(vel4 + ll), vb = ld32(vel4 + i), wa = ld32(omg4 + ll), wb = ld32(omg4 + i);
-          double pin[3] = {0.0, 0.0, 0.0};
-          if (f0 & PF_HIST) { pin[0] = pft[cc]; pin[1] = pft[cap + cc]; pin[2] = pft[2 * cap + cc]; }
+          if (!was) { va = ld32(vel4 + ll); vb = ld32(vel4 + i); wa = ld32(omg4 + ll); wb = ld32(omg4 + i); }
           L.v[0] = va.x; L.v[1] = va.y; L.v[2] = va.z; L.m = va.w;
           I.v[0] = vb.x; I.v[1] = vb.y; I.v[2] = vb.z; I.m = vb.w;
           L.w[0] = wa.x; L.w[1] = wa.y; L.w[2] = wa.z;

@@ -279,10 +279,13 @@ k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long lon
       const int ll = who.x, i = who.y;
       uint8_t f = f0 & PF_HIST;  // NONEXISTENT partner or zero distance: history kept
       {
-        // the states and the positions in one round of loads (any slot's
-        // position can be read; it is used only for existing particles)
+        // the states, the positions and the history in one round of loads (any
+        // slot's position can be read; it is used only for existing particles);
+        // the motion too would spill registers here
         const double4 a = ld32(pos4 + ll), b = ld32(pos4 + i);
         const int8_t sl = state[ll], si = state[i];
+        double pin[3] = {0.0, 0.0, 0.0};
+        if (f0 & PF_HIST) { pin[0] = pft[cc]; pin[1] = pft[cap + cc]; pin[2] = pft[2 * cap + cc]; }
         if (si != DEM_STATE_NONEXISTENT && sl != DEM_STATE_NONEXISTENT) {
           const DevParams& p = sysp<B>(p0, bv, ll);
           double dist[3];
@@ -296,8 +299,6 @@ k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long lon
             err->zero_a = ll; err->zero_b = i;
           } else {
             const double4 va = ld32(vel4 + ll), vb = ld32(vel4 + i), wa = ld32(omg4 + ll), wb = ld32(omg4 + i);
-            double pin[3] = {0.0, 0.0, 0.0};
-            if (f0 & PF_HIST) { pin[0] = pft[cc]; pin[1] = pft[cap + cc]; pin[2] = pft[2 * cap + cc]; }
             double ot[3];
             PairTerms o;
             // one solids phase: no phase to look up
