@@ -10,7 +10,8 @@
 //   state[i]   int8 PARTICLE_STATE, phase[i] uint8 (0-based)
 //   fc, tow    (n,3) column blocks, as FC/TOW of discretelement_mod.f:630
 //   pairs      CSR half list: row_end[i] = pairs in rows 0..i,
-//              nbrs[P] 0-based, pft[b][3P] (3,P) like PFT_NEIGHBOR,
+//              nbrs[P] 0-based, pft[b] = PFT_NEIGHBOR as three planes of
+//              pair_cap (one per component),
 //              and the transpose in_start[n+1] / in_pair[] = (owner, cc)
 //              sorted by owner so each particle can gather the forces of
 //              the pairs it does not own in the serial reference's order.

@@ -8,8 +8,8 @@
 // CFUPDATEOLD + CFNEWVALUES (cfupdateold.f:33-41, cfnewvalues.f:669-812).
 //
 // The reference loops over owners LL and scatters each pair's force into
-// FC(LL) and FC(I).  Here each pair is evaluated once (k_pairs, a thread per
-// pair), which updates its tangential history in place and writes the
+// FC(LL) and FC(I).  Here each pair is evaluated once (k_pairs, a lane per
+// pair that may be in contact), which updates its tangential history in place and writes the
 // terms of both particles into a contact record; then one thread per
 // particle gathers (k_gather): walls first, then the records of the pairs
 // it appears in as neighbour I owned by lower-index particles (ascending
@@ -20,7 +20,8 @@
 //
 // This file is compiled with -fmad=false: every FP64 expression rounds as
 // the Fortran does (gfortran emits no FMA without -march).  sqrt and '/' are
-// IEEE round-to-nearest in CUDA, as they are on the host.
+// IEEE round-to-nearest in CUDA, as they are on the host; quotients by one
+// divisor share its reciprocal and round the same (quotient()).
 #include "dem_internal.cuh"
 
 #include <algorithm>
@@ -618,7 +619,9 @@ k_walls(DevParams p0, BatchView bv, WallArgs wa, const double* __restrict__ skin
 // Bound by latency and by the accesses the L1 takes in, not by DRAM (a fifth of
 // its throughput).  The 1,000,000-sphere bed with 1.67 M of its 4.4 M pairs in contact:
 // 248 us with four pairs per thread (12 of 32 lanes in contact at a time) and
-// records written 8 bytes at a time, 156 us so.
+// records written 8 bytes at a time, 156 us with full warps and 32-byte
+// accesses, 141 us with the loads in three dependent rounds instead of five
+// and the quotients side by side.
 // With JW > 0 the first wa.blocks blocks do the wall work instead (JW
 // particles per thread): it reads the same state and writes disjoint arrays,
 // and in one launch the two run side by side with no second stream to fork
@@ -806,7 +809,10 @@ __device__ __forceinline__ void add_range(const DevParams& p, int q, int e, cons
 // (MODE 0) or integrates them in place of CFNEWVALUES (MODE 1 = Euler, MODE
 // 2 = Adams-Bashforth).
 // Same bed: 179 us with records read 8 bytes at a time and each incoming
-// pair's flag looked up at random, 125 us so.
+// pair's flag looked up at random, 134 us now.  Bound by latency at the
+// 24 warps its 80 registers allow (12 % of a step slower at 16 warps and no
+// spills, 18 % at 32 and 90 bytes spilled; staged through shared memory 15 to 20
+// %, the L1 it takes being worth more).
 template <int MODE, bool B>
 __global__ void __launch_bounds__(256, 3)
 k_gather(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, const double4* __restrict__ vel_c,

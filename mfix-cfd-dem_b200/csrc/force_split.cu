@@ -14,8 +14,8 @@
 //         rolling friction; per-particle sums use compensated (Neumaier)
 //         FP32 accumulation.
 //
-// Structure: the pair kernel evaluates every contact once (a thread per
-// pair, consecutive pairs of the half list) and writes each particle's terms
+// Structure: the pair kernel evaluates every contact once (a lane per pair
+// that may be in contact, queued from windows of the half list) and writes each particle's terms
 // as a 32-byte FP32 record: the owner's at the pair index (rec_own, in row
 // order) and the neighbour's at the pair's slot of the neighbour's incoming
 // list (rec_in[in_pos[cc]], the transpose order).  The neighbour-side writes
@@ -246,7 +246,7 @@ __device__ __forceinline__ void put_records(const PairTerms& o, long long cc, co
 // A warp takes a window of WIN_PAIRS pairs, queues those that may be in
 // contact (screen_window) and gives each lane one of the queue.
 // The bed of 1,000,000 spheres (1.67 M contacts of 4.4 M pairs): 160 us with
-// four pairs per thread, 125 us so.
+// four pairs per thread, 107 us so.
 template <int COLL, bool B>
 __global__ void __launch_bounds__(256, 4)
 k_pairs_split(DevParams p0, BatchView bv, const int* __restrict__ d_np, long long cap, const int* __restrict__ owner,
@@ -480,9 +480,10 @@ __device__ __forceinline__ void add_terms(SplitShared& sh, unsigned in, unsigned
 // pair kernel marked as in some contact --, compensated FP32 sums, the
 // rolling-friction torque -MEW_R*(2R)*sum(KN*OVERLAP_N)*OMEGA/|OMEGA|, and
 // the integration (MODE 1 Euler, 2 Adams-Bashforth) or FC/TOW (MODE 0).
-// Same bed: 113 us with two 16-byte loads per record, 80 us with one of 32;
-// staged in shared memory a step is 1 % faster there, and 4 % in a batch of 16
-// columns of 600,000 spheres, whose contacts are spread less evenly.
+// Same bed: 113 us with two 16-byte loads per record lane by lane, 85 us
+// staged in shared memory with the quotients side by side; the staging alone is
+// 1 % of a step there, and 4 % in a batch of 16 columns of 600,000 spheres,
+// whose contacts are spread less evenly.
 template <int MODE, bool B>
 __global__ void __launch_bounds__(SPLIT_T)
 k_gather_split(DevParams p0, BatchView bv, const double4* __restrict__ pos_c, const double4* __restrict__ vel_c,

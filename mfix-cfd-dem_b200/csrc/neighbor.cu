@@ -502,7 +502,7 @@ __device__ __forceinline__ void place_keys(const uint32_t* __restrict__ slot, in
 // the pair is in the list.  The filter gives each entry the exact test of
 // the scan (neigh_exact, in the owner's frame: stencil, periodic image, FP64
 // distance, stencil rank), so the rows are the scan's.  The choice is made
-// on the device at the start of each build (k_cand_decide), so a captured
+// on the device at the start of each build (cand_decide), so a captured
 // period holds both paths: the count pass and the list build return at once
 // when the list is filtered, the filter when it is not.
 
@@ -583,9 +583,8 @@ k_cand_filter(DevParams p, const int* __restrict__ n_exist, const double4* __res
   }
 }
 
-// Count (FILL = false) and fill pass of a list build (when k_cand_decide
-// asks for one): the half scan of
-// k_neigh_count over a reach widened by the skin, each pair within the
+// Count (FILL = false) and fill pass of a list build (when cand_decide asks
+// for one): the half scan of k_neigh_count over a reach widened by the skin, each pair within the
 // search radius plus the skin of its nearest image entered in its owner's
 // row (any NORMAL owner: the rogue limit of a build is applied when the
 // list is filtered).  The fill places entries at cand_start[owner] + an
