@@ -394,8 +394,11 @@ constexpr int NSURV = 24;  // pre-checked candidates buffered per thread
 // thread's column of s_surv and get the exact test in a second loop, so the
 // long exact path runs with every lane holding work instead of one lane at
 // a time inside the candidate scan.
+// A single system's pass keeps 64 registers (more were slower); a batch's,
+// whose parameters come through the system table, spilled 800 bytes so and takes
+// 128 (five hoppers: 55.1 us per step, 54.4 so; 16 columns: 109.4 and 108.4).
 template <bool B>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, B ? 4 : 8)
 k_neigh_count(DevParams p0, BatchView bv, const int* __restrict__ n_exist, const double4* __restrict__ spos,
               const float4* __restrict__ sposf, const int4* __restrict__ sinfo, const int* __restrict__ fstart,
               const DevErr* __restrict__ err, int* __restrict__ row_cnt, uint32_t* __restrict__ nslot,
