@@ -13,7 +13,8 @@ the oracle.
 - the FP64 pair kernel in small blocks, for lists that keep every resident warp
   busy for eight windows, against the larger ones;
 - contact lists of more than 32 entries, and warps with more than 128;
-- masses past the range in which quotients share a reciprocal.
+- masses past the range in which quotients share a reciprocal;
+- the deposition of more than one solids phase.
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -232,3 +233,30 @@ def test_quotients_of_large_masses(scale, intg):
         compare_state(g, o, exact=True)
         compare_pairs(g, o)
     assert np.isfinite(g.download_state()["vel"]).all()
+
+
+@pytest.mark.parametrize("interp", ["GARG_2012", "NONE"])
+def test_deposition_of_two_phases(interp):
+    """The coupled case with every third sphere of a lighter second phase: a
+    node (or cell) sums its phases apart, four entries at a time, counts with
+    every remainder."""
+    import dataclasses
+    from mfix_dem import params as P
+    from oracle_ffi import OracleSystem
+    case, prm, arr, walls, info, grid, f = coupled_case(interp=interp)
+    d, rho = case.d_p0[0], case.ro_s0[0]
+    case = dataclasses.replace(case, n_phases=2, d_p0=(d, d), ro_s0=(rho, 0.5 * rho), des_en_input=0.9,
+                               des_en_wall_input=[0.9, 0.9])
+    ph = 1 + (np.arange(arr["radius"].size) % 3 == 0)
+    arr = state_arrays(arr["pos"], arr["vel"], arr["omega"], arr["radius"], np.where(ph == 1, rho, 0.5 * rho), phase=ph)
+    prm, info = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
+    grid.ro_s[1] = 0.5 * rho
+    ct = (case, prm, arr, walls, info, grid, f)
+    g, o = make_coupled(_gpu, ct), make_coupled(OracleSystem, ct)
+    for s in (g, o):
+        s.step_coupled(8)
+    compare_state(g, o)
+    for a, b in zip(g.get_mean_fields(), o.get_mean_fields()):
+        assert rel_err(a, b) <= 1e-10
+    assert prm.n_phases == 2
+    assert rel_err(g.calc_des_bedheight(), o.calc_des_bedheight()) <= 1e-10
