@@ -237,7 +237,7 @@ int dem_batch_create(const dem_params* q, const dem_batch_limits* lim, dem_handl
   int rc = alloc_handle(h, lim->max_cells, lim->max_search_cells, batch_pair_reserve(lim));
   auto A = [&](void** p, size_t bytes) {
     if (rc) return;
-    if (cudaMalloc(p, bytes > 0 ? bytes : 8) != cudaSuccess) rc = DEM_ERR_CUDA;
+    if (dev_alloc(h, p, bytes > 0 ? bytes : 8) != cudaSuccess) rc = DEM_ERR_CUDA;
     else cudaMemset(*p, 0, bytes > 0 ? bytes : 8);
     h->arr_bytes += (long long)(bytes > 0 ? bytes : 8);
   };

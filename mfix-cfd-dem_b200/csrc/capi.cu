@@ -27,6 +27,18 @@ int check_cuda(dem_handle* h, cudaError_t e, const char* what) {
   return set_err(h, DEM_ERR_CUDA, b);
 }
 
+// CUDA keeps the error of a failed call until somebody asks for it, and the
+// checks behind the launches would take an allocation's for theirs.
+cudaError_t alloc_bytes(dem_handle* h, void** p, size_t bytes) {
+  if (h->fail_alloc > 0 && --h->fail_alloc == 0) bytes = (size_t)1 << 60;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+  }
+  return e;
+}
+
 // Packs Fortran (n,3) columns + scalars into double4 arrays.
 __global__ void k_pack(int n, const double* __restrict__ v3, const double* __restrict__ s, double4* __restrict__ out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -144,7 +156,7 @@ void* stage_buffer(dem_handle* h, size_t bytes) {
     if (h->stage) cudaFree(h->stage);
     h->stage = nullptr;
     h->stage_bytes = 0;
-    if (cudaMalloc(&h->stage, bytes) != cudaSuccess) return nullptr;
+    if (dev_alloc(h, &h->stage, bytes) != cudaSuccess) return nullptr;
     h->stage_bytes = bytes;
   }
   return h->stage;
@@ -259,7 +271,7 @@ int stats_range(dem_handle* h, int off, int cnt, dem_stats* s) {
     if (h->red) cudaFree(h->red);
     h->red = nullptr;
     h->red_elems = 0;
-    if (int rc = check_cuda(h, cudaMalloc(&h->red, sizeof(double) * 8 * B), "cudaMalloc")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &h->red, sizeof(double) * 8 * B), "cudaMalloc")) return rc;
     h->red_elems = 8 * B;
   }
   std::vector<double> part((size_t)8 * B);
@@ -443,7 +455,7 @@ int demb::alloc_handle(dem_handle* h, int nc, int nfc, long long pairs) {
   bool ok = true;
   auto A = [&](void** p, size_t bytes) {
     if (!ok) return;
-    if (cudaMalloc(p, bytes > 0 ? bytes : 8) != cudaSuccess) ok = false;
+    if (dev_alloc(h, p, bytes > 0 ? bytes : 8) != cudaSuccess) ok = false;
     else cudaMemset(*p, 0, bytes > 0 ? bytes : 8);
     h->arr_bytes += (long long)(bytes > 0 ? bytes : 8);
   };
@@ -480,6 +492,14 @@ int demb::alloc_handle(dem_handle* h, int nc, int nfc, long long pairs) {
 extern "C" {
 
 int dem_abi_version(void) { return DEM_ABI_VERSION; }
+
+// For the tests (not in the header): the handle's n-th allocation from now
+// fails as on a full device.
+int dem_test_fail_alloc(dem_handle* h, int32_t n) {
+  if (!h) return DEM_ERR_ARG;
+  h->fail_alloc = n;
+  return 0;
+}
 
 int dem_memory_info(dem_handle* h, dem_memory* out) {
   API_GUARD(h);

@@ -871,7 +871,7 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
   std::vector<double> fz = faces(h->prm.domain_lo[2], g->dz, h->dp.no_k ? 0 : g->kmax);
   if (fresh) {
     bool ok = true;
-    auto A = [&](void** p, size_t b) { if (ok && cudaMalloc(p, b ? b : 8) != cudaSuccess) ok = false; };
+    auto A = [&](void** p, size_t b) { if (ok && dev_alloc(h, p, b ? b : 8) != cudaSuccess) ok = false; };
     A((void**)&s->xe, sizeof(double) * fx.size());
     A((void**)&s->yn, sizeof(double) * fy.size());
     A((void**)&s->zt, sizeof(double) * fz.size());

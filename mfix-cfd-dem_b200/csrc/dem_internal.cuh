@@ -413,6 +413,8 @@ struct dem_handle {
   // coupling (see coupling.cu)
   struct Gas* gas = nullptr;
 
+  int fail_alloc = 0;  // > 0: the allocation that fails (dem_test_fail_alloc)
+
   // host<->device staging (kept between calls)
   void* stage = nullptr;
   size_t stage_bytes = 0;
@@ -431,6 +433,12 @@ namespace demb {
 // set by every API entry point on failure
 int set_err(dem_handle* h, int code, const std::string& msg);
 int check_cuda(dem_handle* h, cudaError_t e, const char* what);
+// capi.cu: cudaMalloc; a failure leaves a null pointer and no pending error
+cudaError_t alloc_bytes(dem_handle* h, void** p, size_t bytes);
+template <class T>
+cudaError_t dev_alloc(dem_handle* h, T** p, size_t bytes) {
+  return alloc_bytes(h, reinterpret_cast<void**>(p), bytes);
+}
 
 // scan.cu: exclusive scan of n ints into out (out may alias in); total
 // written to *d_total (device pointer) when non-null; `clear` zeroes the

@@ -210,7 +210,7 @@ int run_mass_inflow(dem_handle* h) {
     if (h->d_seed) cudaFree(h->d_seed);
     h->d_seed = nullptr;
     h->seed_cap = 0;
-    if (int rc = check_cuda(h, cudaMalloc(&h->d_seed, sizeof(SeedRec) * (size_t)k), "cudaMalloc seeds")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &h->d_seed, sizeof(SeedRec) * (size_t)k), "cudaMalloc seeds")) return rc;
     h->seed_cap = k;
   }
   // pageable source: the copy has read it when the call returns
@@ -272,10 +272,10 @@ int dem_set_inflow_bcs(dem_handle* h, const dem_inflow_bc* bcs, int32_t n, uint6
     h->ibc.push_back(std::move(I));
   }
   if (!h->pic_fresh) {
-    if (int rc = check_cuda(h, cudaMalloc(&h->pic_fresh, (size_t)h->n), "cudaMalloc pic_fresh")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &h->pic_fresh, (size_t)h->n), "cudaMalloc pic_fresh")) return rc;
   }
   cudaMemsetAsync(h->pic_fresh, 0, (size_t)h->n, h->stream);
-  if (int rc = check_cuda(h, cudaMalloc(&h->d_ibc, sizeof(dem_inflow_bc) * n), "cudaMalloc inflow")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &h->d_ibc, sizeof(dem_inflow_bc) * n), "cudaMalloc inflow")) return rc;
   std::vector<dem_inflow_bc> dev(n);
   for (int32_t i = 0; i < n; ++i) dev[i] = h->ibc[i].bc;
   cudaMemcpyAsync(h->d_ibc, dev.data(), sizeof(dem_inflow_bc) * n, cudaMemcpyHostToDevice, h->stream);

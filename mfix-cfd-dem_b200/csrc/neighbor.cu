@@ -1036,7 +1036,7 @@ static int ensure_cand_capacity(dem_handle* h, long long need) {
   if (need <= h->cand_cap) return 0;
   const long long cap = need + need / 4 + 1024;
   int* cnb = nullptr;
-  if (int rc = check_cuda(h, cudaMalloc(&cnb, sizeof(int) * cap), "cudaMalloc candidates")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &cnb, sizeof(int) * cap), "cudaMalloc candidates")) return rc;
   cudaStreamSynchronize(h->stream);
   cudaFree(h->cand_nb);
   h->cand_nb = cnb;
@@ -1055,17 +1055,17 @@ int ensure_pair_capacity(dem_handle* h, long long need) {
   int* nb[2]; double* pf[2]; int2* inp; int* own; uint8_t* pfl[2]; void* prc; float* gap;
   int* ipos; uint8_t* ifl;
   for (int b = 0; b < 2; ++b) {
-    if (int rc = check_cuda(h, cudaMalloc(&nb[b], sizeof(int) * cap), "cudaMalloc nbrs")) return rc;
-    if (int rc = check_cuda(h, cudaMalloc(&pf[b], sizeof(double) * 3 * cap), "cudaMalloc pft")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &nb[b], sizeof(int) * cap), "cudaMalloc nbrs")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &pf[b], sizeof(double) * 3 * cap), "cudaMalloc pft")) return rc;
     // flag arrays carry 16 bytes of padding: the gather reads them as aligned words
-    if (int rc = check_cuda(h, cudaMalloc(&pfl[b], cap + 16), "cudaMalloc pflag")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &pfl[b], cap + 16), "cudaMalloc pflag")) return rc;
   }
-  if (int rc = check_cuda(h, cudaMalloc(&inp, sizeof(int2) * cap), "cudaMalloc in_pair")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&own, sizeof(int) * cap), "cudaMalloc owner")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&prc, sizeof(PairRec) * cap), "cudaMalloc prec")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&gap, sizeof(float) * cap), "cudaMalloc pgap")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&ipos, sizeof(int) * cap), "cudaMalloc in_pos")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&ifl, cap + 16), "cudaMalloc in_flag")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &inp, sizeof(int2) * cap), "cudaMalloc in_pair")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &own, sizeof(int) * cap), "cudaMalloc owner")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &prc, sizeof(PairRec) * cap), "cudaMalloc prec")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &gap, sizeof(float) * cap), "cudaMalloc pgap")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &ipos, sizeof(int) * cap), "cudaMalloc in_pos")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &ifl, cap + 16), "cudaMalloc in_flag")) return rc;
   if (old > 0) {
     // keep the current list and history (the rebuild reads them)
     cudaMemcpyAsync(nb[h->rb], h->nbrs[h->rb], sizeof(int) * old, cudaMemcpyDeviceToDevice, h->stream);

@@ -220,7 +220,7 @@ int dem_set_outflow_bcs(dem_handle* h, const dem_outflow_bc* bcs, int32_t n) {
   h->exit_first_pass = true;
   invalidate_graphs(h);
   if (n > 0) {
-    if (int rc = check_cuda(h, cudaMalloc(&h->d_obc, sizeof(dem_outflow_bc) * n), "cudaMalloc outflow")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &h->d_obc, sizeof(dem_outflow_bc) * n), "cudaMalloc outflow")) return rc;
     cudaMemcpyAsync(h->d_obc, bcs, sizeof(dem_outflow_bc) * n, cudaMemcpyHostToDevice, h->stream);
   }
   return check_cuda(h, cudaStreamSynchronize(h->stream), "outflow boundaries");

@@ -129,7 +129,7 @@ int exclusive_scan(dem_handle* h, int* in, int* out, int n, int* d_total, bool c
     if (h->scan_tmp) cudaFree(h->scan_tmp);
     h->scan_tmp = nullptr;
     h->scan_tmp_elems = 0;
-    if (int rc = check_cuda(h, cudaMalloc(&h->scan_tmp, need * sizeof(int)), "cudaMalloc scan")) return rc;
+    if (int rc = check_cuda(h, dev_alloc(h, &h->scan_tmp, need * sizeof(int)), "cudaMalloc scan")) return rc;
     h->scan_tmp_elems = need;
   }
   scan_rec(h, in, out, n, h->scan_tmp, d_total, clear, go);

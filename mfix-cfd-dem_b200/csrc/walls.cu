@@ -177,9 +177,9 @@ int run_bin_facets(dem_handle* h, const double* vf, const double* nfort, int nf)
     for (int v = 0; v < 3; ++v)
       for (int c = 0; c < 3; ++c) vx[(size_t)9 * f + 3 * v + c] = vf[v + 3 * c + 9 * (size_t)f];
   for (size_t q = 0; q < nx.size(); ++q) nx[q] = nfort[q];
-  if (int rc = check_cuda(h, cudaMalloc(&h->vertex, sizeof(double) * vx.size()), "cudaMalloc")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&h->norm_face, sizeof(double) * nx.size()), "cudaMalloc")) return rc;
-  if (int rc = check_cuda(h, cudaMalloc(&h->ignore_edge, (size_t)4 * nf), "cudaMalloc")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &h->vertex, sizeof(double) * vx.size()), "cudaMalloc")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &h->norm_face, sizeof(double) * nx.size()), "cudaMalloc")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &h->ignore_edge, (size_t)4 * nf), "cudaMalloc")) return rc;
   cudaMemcpyAsync(h->vertex, vx.data(), sizeof(double) * vx.size(), cudaMemcpyHostToDevice, h->stream);
   cudaMemcpyAsync(h->norm_face, nx.data(), sizeof(double) * nx.size(), cudaMemcpyHostToDevice, h->stream);
   cudaMemsetAsync(h->ignore_edge, 0, (size_t)4 * nf, h->stream);
@@ -193,7 +193,7 @@ int run_bin_facets(dem_handle* h, const double* vf, const double* nfort, int nf)
   cudaMemcpyAsync(&nb, total, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
   if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "sync")) return rc;
   cudaMemcpyAsync(h->fbin_start + p.ncell2, &nb, sizeof(int), cudaMemcpyHostToDevice, h->stream);
-  if (int rc = check_cuda(h, cudaMalloc(&h->fbin, sizeof(FacetBinEntry) * (size_t)(nb > 0 ? nb : 1)), "cudaMalloc")) return rc;
+  if (int rc = check_cuda(h, dev_alloc(h, &h->fbin, sizeof(FacetBinEntry) * (size_t)(nb > 0 ? nb : 1)), "cudaMalloc")) return rc;
   h->n_fbin = nb;
   k_bin_facets<true><<<B, T, 0, h->stream>>>(p, nf, h->vertex, buffer, 0, nullptr, h->fbin_start, h->fbin);
   DEM_LAUNCH(h);
