@@ -692,6 +692,7 @@ static int run_pic(dem_handle* h, bool located = false) {
   const GasDev G = gas_view(h);
   const int T = 256, B = (h->n + T - 1) / T;
   const int c = h->cur;
+  if (int rc = reserve_scan(h, s->ncell)) return rc;
   if (!located)
     launch_pdl(h, k_pic_locate, B, T, h->dp, G, h->pos4[c], h->vel4[c], h->omg4[c], h->state, s->pijk, s->pic_cnt,
                h->fc, h->tow, h->wall_fid, h->derr);
@@ -760,6 +761,8 @@ static int run_coupled_step(dem_handle* h, bool locate) {
   const int T = 256, B = (h->n + T - 1) / T;
   const int c = h->cur;
   const bool garg = s->g.interp_scheme != DEM_INTERP_NONE, ab2 = h->dp.intg == DEM_INTG_AB2;
+  if (locate)
+    if (int rc = reserve_scan(h, s->ncell)) return rc;
   launch_pdl(h, garg ? (ab2 ? k_coupled_step<2, true> : k_coupled_step<1, true>)
                      : (ab2 ? k_coupled_step<2, false> : k_coupled_step<1, false>),
              B, T, h->dp, G, h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c], h->vel4[1 - c], h->omg4[1 - c],
@@ -767,7 +770,9 @@ static int run_coupled_step(dem_handle* h, bool locate) {
              h->rot_acc_old, h->vslot_note(), step_end(h), locate ? 1 : 0, s->pic_cnt, h->wall_fid, h->derr);
   h->cur = 1 - c;
   h->first_pass = false;
-  return check_cuda(h, cudaGetLastError(), "coupled step");
+  // with `locate` run_mean_fields follows, whose scan the counts need and which
+  // checks the launches
+  return locate ? 0 : check_cuda(h, cudaGetLastError(), "coupled step");
 }
 
 // DRAG_GS_GAS1: F_GP per particle, then the per-cell gather.

@@ -278,7 +278,8 @@ struct dem_handle {
   long long arr_bytes = 0;    // device bytes of the arrays sized by the counts (handle_arrays and the batch tables)
   long long n_pairs = 0;      // host copy of the pair count (valid when !np_stale)
   bool np_stale = false;      // the last build ran without reading the count back
-  int* d_np = nullptr;        // device pair count (persistent pair kernels read it)
+  int* d_np = nullptr;        // device pair count (persistent pair kernels read it); [1]: the count of the
+                              // list being built, which becomes [0] when its rows are filled
   int n_sm = 148;             // multiprocessors of the device
   // launch shapes of the hot kernels (dem_autotune picks them)
   struct Tune {
@@ -446,6 +447,11 @@ cudaError_t dev_alloc(dem_handle* h, T** p, size_t bytes) {
 // done unless *go is set.
 int exclusive_scan(dem_handle* h, int* in, int* out, int n, int* d_total, bool clear = false,
                    const int* go = nullptr);
+// The scratch of a scan of n ints, so that the scan itself cannot fail for
+// memory.  Counters that a clearing scan leaves at zero (fcell_cnt, in_cnt,
+// pic_cnt) are only counted into behind it: a call that returned between the
+// count and its scan would leave them for the next one to add to.
+int reserve_scan(dem_handle* h, int n);
 
 // desgrid.cu / neighbor.cu / force.cu / walls.cu host drivers
 int run_desgrid_pic(dem_handle* h, bool sort_cells);
@@ -531,7 +537,7 @@ void handle_arrays(dem_handle* h, size_t n, size_t nc, size_t nfc, F&& A) {
   A((void**)&h->skin, sizeof(double));
   A((void**)&h->vslot, sizeof(unsigned) * 64);
   A((void**)&h->derr, sizeof(DevErr));
-  A((void**)&h->d_np, sizeof(int));
+  A((void**)&h->d_np, 2 * sizeof(int));
   A((void**)&h->slipfix, sizeof(SlipFix));
   if (!h->batch()) {
     A((void**)&h->cand_cnt, sizeof(int) * n);

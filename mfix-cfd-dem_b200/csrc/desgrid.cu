@@ -106,6 +106,8 @@ int run_desgrid_pic(dem_handle* h, bool bin_search) {
   // where the pair build reads it
   const int nfc = h->nfl() + 1;
   int* n_binned = h->fcell_start + (bt ? h->nfcell_total : p.nfcell);
+  if (bin_search)
+    if (int rc = reserve_scan(h, nfc)) return rc;
   launch_pdl(h, bt ? (bin_search ? k_cell_keys<true, true> : k_cell_keys<true, false>)
                    : (bin_search ? k_cell_keys<false, true> : k_cell_keys<false, false>),
              B, T, p, bv, h->pos4[h->cur], h->state, h->dg_pijk, h->fbin_start, h->wall_cand, h->wgap, h->fcell_key,

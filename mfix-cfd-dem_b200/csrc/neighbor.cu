@@ -714,7 +714,11 @@ __global__ void k_fill_rows(DevParams p0, int n, int n_old, BatchView bv, const 
   const int z = pdl_wait();
   pdl_next();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + z;
-  if (i == 0 && *d_np > cap) { *d_np = (int)cap; atomicOr(&err->flags, EF_PAIR_CAP); }
+  if (i == 0) {
+    const int np = d_np[1];
+    d_np[0] = (int)min((long long)np, cap);
+    if (np > cap) atomicOr(&err->flags, EF_PAIR_CAP);
+  }
   if (i >= n) return;
   if constexpr (B) {
     if (!bv.due[bv.sys_of[i]]) {
@@ -1013,6 +1017,7 @@ int build_transpose(dem_handle* h, int nb, bool counted) {
   const int n = h->nl();
   const int T = 256, B = (n + T - 1) / T;
   const unsigned BP = pair_grid(h, T);
+  if (int rc = reserve_scan(h, n)) return rc;  // the build's row scan had this size: nothing to do behind its count
   if (!counted) {
     k_in_count<<<BP, T, 0, h->stream>>>(h->d_np, h->nbrs[nb], h->in_cnt, h->in_pos);
     DEM_LAUNCH(h);
@@ -1132,19 +1137,37 @@ int run_neighbour(dem_handle* h, bool carry_history) {
   if (cand)
     launch_pdl(h, k_cand_filter, B, T, p, n_exist, h->spos, h->sinfo, h->qof, e, h->cand_start, h->cand_nb, h->cand,
                h->row_cnt, h->nslot, h->long_rows);
-  if (int rc = exclusive_scan(h, h->row_cnt, h->row_end[nb], n, h->d_np)) return rc;
+  if (int rc = exclusive_scan(h, h->row_cnt, h->row_end[nb], n, h->d_np + 1)) return rc;
+  if (cand) {
+    // the length of a new candidate list, when the build asks for one (each
+    // kernel of it returns at once otherwise)
+    launch_pdl(h, k_cand_build<false>, B, T, p, n_exist, h->spos, h->sposf, h->sinfo, h->fcell_start, h->cand, skin_c,
+               h->cand_cnt, h->cand_fill, h->cand_start, h->cand_nb, h->cand_cap, e);
+    if (int rc = exclusive_scan(h, h->cand_cnt, h->cand_start, n, h->cand_start + n, false, &h->cand->build)) return rc;
+  }
+  // Eager builds read both lengths back and grow the arrays when needed.  All
+  // that may fail for memory lies before the fill: up to here the current list,
+  // its length and the incoming counts are untouched, so a build that fails
+  // can be repeated.  A captured build holds the pairs to the capacity (k_fill_rows)
+  // and leaves a candidate list that does not fit incomplete, unused.
   if (!h->capturing) {
-    // eager steps read the count back and grow the arrays when needed
-    int P = 0;
-    if (int rc = check_cuda(h, cudaMemcpyAsync(&P, h->d_np, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "copy P")) return rc;
+    int P = 0, total = 0;
+    if (int rc = check_cuda(h, cudaMemcpyAsync(&P, h->d_np + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "copy P")) return rc;
+    if (cand)
+      if (int rc = check_cuda(h, cudaMemcpyAsync(&total, h->cand_start + n, sizeof(int), cudaMemcpyDeviceToHost,
+                                                 h->stream), "copy candidates")) return rc;
     if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "sync")) return rc;
     if (int rc = ensure_pair_capacity(h, (long long)P + 1)) return rc;
+    if (int rc = ensure_cand_capacity(h, total)) return rc;
     h->joined = true;
     h->n_pairs = P;
     h->np_stale = false;
   } else {
     h->np_stale = true;
   }
+  if (cand)
+    launch_pdl(h, k_cand_build<true>, B, T, p, n_exist, h->spos, h->sposf, h->sinfo, h->fcell_start, h->cand, skin_c,
+               h->cand_cnt, h->cand_fill, h->cand_start, h->cand_nb, h->cand_cap, e);
   // rows kept whole by the count pass, then the long rows (a fixed grid
   // striding over the list, whose length is on the device)
   launch_pdl(h, bt ? k_fill_rows<true> : k_fill_rows<false>, B, T, p, n, h->n_built, bv, h->row_cnt, h->row_end[nb],
@@ -1154,26 +1177,6 @@ int run_neighbour(dem_handle* h, bool carry_history) {
   launch_pdl(h, bt ? k_fill_long<true> : k_fill_long<false>, 4 * 148, 128, p, bv, h->spos, h->sposf, h->sinfo,
              h->fcell_start, h->row_cnt, h->row_end[nb], h->nbrs[nb], h->pflagb[1 - h->pcur], h->pair_owner,
              h->in_cnt, h->in_pos, h->long_rows, h->pair_cap);
-  if (cand) {
-    // a new candidate list when the build asks for one (each kernel returns at
-    // once otherwise)
-    launch_pdl(h, k_cand_build<false>, B, T, p, n_exist, h->spos, h->sposf, h->sinfo, h->fcell_start, h->cand, skin_c,
-               h->cand_cnt, h->cand_fill, h->cand_start, h->cand_nb, h->cand_cap, e);
-    if (int rc = exclusive_scan(h, h->cand_cnt, h->cand_start, n, h->cand_start + n, false, &h->cand->build)) return rc;
-    if (!h->capturing) {
-      // eager builds read the list's length back and grow its array when
-      // needed; a captured build that overflows leaves the list incomplete,
-      // unused
-      int total = 0;
-      if (int rc = check_cuda(h, cudaMemcpyAsync(&total, h->cand_start + n, sizeof(int), cudaMemcpyDeviceToHost,
-                                                 h->stream), "copy candidates")) return rc;
-      if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "sync")) return rc;
-      if (int rc = ensure_cand_capacity(h, total)) return rc;
-      h->joined = true;
-    }
-    launch_pdl(h, k_cand_build<true>, B, T, p, n_exist, h->spos, h->sposf, h->sinfo, h->fcell_start, h->cand, skin_c,
-               h->cand_cnt, h->cand_fill, h->cand_start, h->cand_nb, h->cand_cap, e);
-  }
   // The transpose of the new list and the history carry-over with the gaps
   // read the list and write disjoint arrays: the transpose runs on the side
   // stream beside them and is joined before the build returns (in sequence

@@ -118,20 +118,24 @@ static void scan_rec(dem_handle* h, int* in, int* out, int n, int* tmp, int* tot
              go);
 }
 
+int reserve_scan(dem_handle* h, int n) {
+  const size_t need = n > 0 ? scratch_need(n) : 0;
+  if (need <= h->scan_tmp_elems) return 0;
+  if (h->scan_tmp) cudaFree(h->scan_tmp);
+  h->scan_tmp = nullptr;
+  h->scan_tmp_elems = 0;
+  if (int rc = check_cuda(h, dev_alloc(h, &h->scan_tmp, need * sizeof(int)), "cudaMalloc scan")) return rc;
+  h->scan_tmp_elems = need;
+  return 0;
+}
+
 int exclusive_scan(dem_handle* h, int* in, int* out, int n, int* d_total, bool clear, const int* go) {
   if (n <= 0) {
     if (d_total) check_cuda(h, cudaMemsetAsync(d_total, 0, sizeof(int), h->stream), "memset");
     h->joined = true;
     return 0;
   }
-  const size_t need = scratch_need(n);
-  if (need > h->scan_tmp_elems) {
-    if (h->scan_tmp) cudaFree(h->scan_tmp);
-    h->scan_tmp = nullptr;
-    h->scan_tmp_elems = 0;
-    if (int rc = check_cuda(h, dev_alloc(h, &h->scan_tmp, need * sizeof(int)), "cudaMalloc scan")) return rc;
-    h->scan_tmp_elems = need;
-  }
+  if (int rc = reserve_scan(h, n)) return rc;
   scan_rec(h, in, out, n, h->scan_tmp, d_total, clear, go);
   return check_cuda(h, cudaGetLastError(), "scan");
 }

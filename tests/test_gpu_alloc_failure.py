@@ -10,8 +10,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from cases import coupled_case, make_coupled, make_system
-from gpu_util import compare_state, rel_err
+from cases import coupled_case, make_system, settling_case
+from gpu_util import compare_pairs, compare_state, pair_both
 
 pytestmark = pytest.mark.gpu
 
@@ -31,6 +31,20 @@ def _refused(call, *args, **kw):
     with pytest.raises(DemError) as e:
         call(*args, **kw)
     assert e.value.code == abi.DEM_ERR_CUDA
+    return str(e.value)
+
+
+def _refused_at(make, what, call):
+    """A system from make() whose call(system) has failed at the allocation
+    that the message calls `what`."""
+    for nth in range(1, 40):
+        g = make()
+        _fail(g, nth)
+        if what in _refused(call, g):
+            _fail(g, 0)
+            return g
+        g.close()
+    raise AssertionError(what)
 
 
 def test_next_call_is_not_blamed():
@@ -47,3 +61,77 @@ def test_next_call_is_not_blamed():
         s.nn = 1
         s.step(5)
     compare_state(g, o, exact=True)
+
+
+@pytest.mark.parametrize("what", ["scan", "candidates"])
+def test_first_build_repeated(what):
+    """The particles counted into the search cells, and the pairs counted into
+    the incoming lists, are counted once when the build is made again."""
+    case, prm, arr, walls = settling_case(n_side=(14, 14, 14), box=(16e-3, 40e-3, 16e-3), spacing=0.99, nsn=5, seed=12)
+
+    def make():
+        s = _gpu(prm, arr["radius"].size)
+        s.upload_state(arr["pos"], arr["vel"], arr["omega"], arr["radius"], arr["pmass"], arr["omoi"], arr["state"],
+                       arr["phase"])
+        return s
+
+    from oracle_ffi import OracleSystem
+    g = _refused_at(make, what, lambda s: s.init_neighbors())
+    o = make_system(OracleSystem, prm, arr, walls)
+    g.init_neighbors()
+    compare_pairs(g, o)
+    g.set_walls(*walls)
+    for s in (g, o):
+        s.step(23)
+    compare_state(g, o, exact=True)
+    compare_pairs(g, o)
+
+
+def test_later_build_repeated():
+    """A build inside a step that fails leaves the list before it whole, its
+    length included: it can be made again and the run continued."""
+    case, prm, sparse, walls = settling_case(n_side=(12, 12, 12), box=(40e-3, 40e-3, 40e-3), spacing=2.5, nsn=5,
+                                             vmax=0.01, seed=13)
+    dense = settling_case(n_side=(12, 12, 12), box=(40e-3, 40e-3, 40e-3), spacing=0.98, nsn=5, vmax=0.01, seed=13)[2]
+    g, o = pair_both(prm, sparse, walls)
+    n0 = g.pair_count()
+    for s in (g, o):
+        s.upload_state(dense["pos"], dense["vel"], dense["omega"], dense["radius"], dense["pmass"], dense["omoi"],
+                       dense["state"], dense["phase"])
+    _fail(g)
+    assert "candidates" in _refused(g.step, 1)
+    assert g.pair_count() == n0
+    o.step(1)
+    for s in (g, o):
+        s.neighbour()
+    assert g.pair_count() > 4 * n0
+    compare_pairs(g, o)
+    for s in (g, o):
+        s.step(28, nn_first=2)
+    compare_state(g, o, exact=True)
+    compare_pairs(g, o)
+
+
+def _fine_gas(interp="GARG_2012"):
+    """Spheres of 1 mm in fluid cells of 0.25 mm, several for each search cell."""
+    prm, arr, walls = settling_case(n_side=(8, 10, 8), box=(10e-3, 15e-3, 10e-3), spacing=1.02, nsn=5, seed=14)[1:]
+    grid, f = coupled_case(cells=(40, 60, 40), dx=0.25e-3, d=0.25e-3, n=600, interp=interp)[5:]
+    return prm, arr, walls, (grid, f["ep_g"], f["u_g"], f["v_g"], f["w_g"])
+
+
+@pytest.mark.parametrize("interp", ["GARG_2012", "NONE"])
+def test_fluid_cells_counted_again(interp):
+    """The particles of the fluid cells, on a grid of more cells than any scan
+    before needed."""
+    from oracle_ffi import OracleSystem
+    prm, arr, walls, fields = _fine_gas(interp)
+    g = _refused_at(lambda: make_system(_gpu, prm, arr, walls), "scan", lambda s: s.set_gas_fields(*fields))
+    g._ncell = fields[1].shape[0]
+    o = make_system(OracleSystem, prm, arr, walls)
+    o.set_gas_fields(*fields)
+    for steps in (0, 4):
+        for s in (g, o):
+            s.step(steps)
+            s.comp_mean_fields()
+        for a, b in zip(g.get_mean_fields(), o.get_mean_fields()):
+            assert np.array_equal(a, b)
