@@ -121,6 +121,9 @@ static void scan_rec(dem_handle* h, int* in, int* out, int n, int* tmp, int* tot
 int reserve_scan(dem_handle* h, int n) {
   const size_t need = n > 0 ? scratch_need(n) : 0;
   if (need <= h->scan_tmp_elems) return 0;
+  if (h->capturing) return set_err(h, DEM_ERR_STATE, "scan scratch too small inside a captured step");
+  invalidate_graphs(h);  // captured builds scan in the old scratch
+  cudaStreamSynchronize(h->stream);
   if (h->scan_tmp) cudaFree(h->scan_tmp);
   h->scan_tmp = nullptr;
   h->scan_tmp_elems = 0;

@@ -7,7 +7,7 @@ the oracle.
   multiprocessor and four past that: bed sizes on both sides, with the counts
   not a multiple of four;
 - the scans take a second level past 4096 tiles of 2048 cells: a search grid
-  just over it;
+  just over it; their scratch grows between replays of captured steps;
 - the contact counts of passes that integrate and passes that do not;
 - gas fields set again, on the same grid (the arrays are kept) and on another;
 - the FP64 pair kernel in small blocks, for lists that keep every resident warp
@@ -110,6 +110,24 @@ def test_scan_of_many_search_cells():
     compare_pairs(g, o)
     g.step(9)
     o.step(9)
+    compare_state(g, o, exact=True)
+    compare_pairs(g, o)
+
+
+def test_scan_scratch_grown_between_replays():
+    """A fluid grid of more cells than any scan before it, set on a system whose
+    steps have been captured: the next replays scan in the new scratch."""
+    from test_gpu_alloc_failure import _fine_gas
+    prm, arr, walls, fields = _fine_gas()
+    g, o = pair_both(prm, arr, walls)
+    for s in (g, o):
+        s.step(1 + 4 + 4 * 5)   # one replay of each buffer parity that follows
+    before = g.memory_info()["scratch_bytes"]
+    for s in (g, o):
+        s.set_gas_fields(*fields)
+    assert g.memory_info()["scratch_bytes"] > before
+    for s in (g, o):
+        s.step(4 * 5)
     compare_state(g, o, exact=True)
     compare_pairs(g, o)
 
