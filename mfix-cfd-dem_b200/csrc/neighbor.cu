@@ -700,8 +700,9 @@ k_cand_build(DevParams p, const int* __restrict__ n_exist, const double4* __rest
 // now, and the slots between systems' ranges belong to none).  The same pass
 // deletes the rogue particles, and holds the pair count to the capacity when a
 // build needed more (only possible inside a captured step, which cannot grow
-// the arrays; reported as DEM_ERR_PAIR_OVERFLOW), which keeps every
-// pair-indexed kernel inside the allocation.
+// the arrays; reported as DEM_ERR_PAIR_OVERFLOW), and with it the end of every
+// row, empty ones included: the rows are read by their ends, the pairs by
+// their count, and both then stay inside the allocation.
 template <bool B>
 __global__ void k_fill_rows(DevParams p0, int n, int n_old, BatchView bv, const int* __restrict__ row_cnt,
                             int* __restrict__ row_se, int* __restrict__ nbrs, int* __restrict__ owner,
@@ -722,9 +723,12 @@ __global__ void k_fill_rows(DevParams p0, int n, int n_old, BatchView bv, const 
   if (i >= n) return;
   if constexpr (B) {
     if (!bv.due[bv.sys_of[i]]) {
-      if (i >= n_old) return;
-      const int s = i ? old_end[i - 1] : 0, e = old_end[i];
       const long long start = row_se[i];
+      if (i >= n_old) {
+        if (start > cap) row_se[i] = (int)cap;
+        return;
+      }
+      const int s = i ? old_end[i - 1] : 0, e = old_end[i];
       for (int c = s; c < e; ++c) {
         const long long slot = start + (c - s);
         if (slot < cap) put_pair(slot, i, old_nbrs[c], nbrs, owner, in_cnt, in_slot);
@@ -737,7 +741,7 @@ __global__ void k_fill_rows(DevParams p0, int n, int n_old, BatchView bv, const 
   if (state[i] == DEM_STATE_NORMAL && is_rogue(p, dg_pijk[i]))
     delete_rogue(p, i, state, pos4, vel4, omg4, fc, tow, wall_fid, err);
   const int kept = row_cnt[i];
-  if (kept == 0 || kept > NSLOT) return;
+  if (kept > NSLOT) return;  // k_fill_long's
   const long long start = min((long long)row_se[i], cap);
   const uint32_t* slot = nslot + (size_t)i * NSLOT;
   if (kept <= NSLOT / 2) place_keys<NSLOT / 2>(slot, kept, start, cap, i, nbrs, owner, in_cnt, in_slot);

@@ -8,6 +8,8 @@ the oracle.
   not a multiple of four;
 - the scans take a second level past 4096 tiles of 2048 cells: a search grid
   just over it; their scratch grows between replays of captured steps;
+- a pair list that outgrows its arrays inside a captured step, with empty rows
+  behind the last one that fits;
 - the contact counts of passes that integrate and passes that do not;
 - gas fields set again, on the same grid (the arrays are kept) and on another;
 - the FP64 pair kernel in small blocks, for lists that keep every resident warp
@@ -130,6 +132,52 @@ def test_scan_scratch_grown_between_replays():
         s.step(4 * 5)
     compare_state(g, o, exact=True)
     compare_pairs(g, o)
+
+
+def test_rows_of_an_overflowing_list():
+    """1,000 spheres drawn together within one captured period, from no pair to
+    several times the capacity of 16 n + 1024: the error is reported, every row
+    ends inside the list that is left, steps over it run, and the list made
+    again is the oracle's."""
+    from mfix_dem import abi
+    from mfix_dem import params as P
+    from mfix_dem.system import DemError
+    d, nsn, L = 1e-3, 5, 24e-3
+    k = np.arange(10) - 4.5
+    rng = np.random.default_rng(17)
+    off = np.stack(np.meshgrid(k, k, k, indexing="ij")).reshape(3, -1) * 1.5 * d + rng.uniform(-1e-5, 1e-5, (3, 1000))
+    n = off.shape[1]
+    arr = state_arrays(0.5 * L + off, np.zeros((3, n)), np.zeros((3, n)), np.full(n, 0.5 * d), np.full(n, 2500.0))
+    case = P.DemCase(d_p0=(d,), ro_s0=(2500.0,), coll_model="LSD", kn=1000.0, kn_w=1000.0, des_en_input=0.9,
+                     des_en_wall_input=[0.9], mew=0.1, mew_w=0.1, grav=(0.0, 0.0, 0.0), domain_hi=(L, L, L),
+                     neighbor_search_n=nsn)
+    prm, _ = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
+    g, o = pair_both(prm, arr, P.default_walls((0.0, 0.0, 0.0), (L, L, L)))
+    vel = -0.75 * off / (nsn * prm.dtsolid)
+    for s in (g, o):
+        s.step(nsn)
+        s.upload_state(arr["pos"], vel, arr["omega"])
+    assert g.pair_count() == 0
+    cap = g.memory_info()["pair_capacity"]
+    with pytest.raises(DemError) as e:
+        g.step(nsn)
+    assert e.value.code == abi.DEM_ERR_PAIR_OVERFLOW
+    o.step(nsn)
+    assert o.pair_count() > 2 * cap
+    ni, nb, _ = g.download_pairs()
+    assert nb.size == cap and ni[-1] == cap + 1
+    assert (np.diff(ni) >= 0).all() and ni.max() <= cap + 1
+    assert nb.min() >= 1 and nb.max() <= n
+    whole = o.download_state()
+    g.step(2, nn_first=2 * nsn + 1)
+    assert np.isfinite(g.download_state()["vel"]).all()
+    for s in (g, o):
+        s.upload_state(whole["pos"], np.zeros((3, n)), whole["omega"])
+        s.init_neighbors()
+    compare_pairs(g, o)
+    for s in (g, o):
+        s.step(3, nn_first=2 * nsn + 1)
+    compare_state(g, o, exact=True)
 
 
 def test_contact_counts_of_mixed_passes():
