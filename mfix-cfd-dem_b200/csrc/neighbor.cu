@@ -1061,20 +1061,34 @@ int ensure_pair_capacity(dem_handle* h, long long need) {
   long long cap = h->pair_cap > 0 ? h->pair_cap : need;
   while (cap < need) cap *= 2;
   const long long old = h->pair_cap;  // the whole old allocation (the count may be stale)
-  int* nb[2]; double* pf[2]; int2* inp; int* own; uint8_t* pfl[2]; void* prc; float* gap;
-  int* ipos; uint8_t* ifl;
+  int *nb[2], *own, *ipos;
+  double* pf[2];
+  uint8_t *pfl[2], *ifl;
+  int2* inp;
+  void* prc;
+  float* gap;
+  std::vector<void*> made;
+  cudaError_t ce = cudaSuccess;
+  auto A = [&](auto** q, size_t bytes) {
+    if (ce != cudaSuccess) return;
+    ce = dev_alloc(h, q, bytes);
+    if (ce == cudaSuccess) made.push_back(*q);
+  };
   for (int b = 0; b < 2; ++b) {
-    if (int rc = check_cuda(h, dev_alloc(h, &nb[b], sizeof(int) * cap), "cudaMalloc nbrs")) return rc;
-    if (int rc = check_cuda(h, dev_alloc(h, &pf[b], sizeof(double) * 3 * cap), "cudaMalloc pft")) return rc;
-    // flag arrays carry 16 bytes of padding: the gather reads them as aligned words
-    if (int rc = check_cuda(h, dev_alloc(h, &pfl[b], cap + 16), "cudaMalloc pflag")) return rc;
+    A(&nb[b], sizeof(int) * cap);
+    A(&pf[b], sizeof(double) * 3 * cap);
+    A(&pfl[b], cap + 16);  // flag arrays carry 16 bytes of padding: the gather reads them as aligned words
   }
-  if (int rc = check_cuda(h, dev_alloc(h, &inp, sizeof(int2) * cap), "cudaMalloc in_pair")) return rc;
-  if (int rc = check_cuda(h, dev_alloc(h, &own, sizeof(int) * cap), "cudaMalloc owner")) return rc;
-  if (int rc = check_cuda(h, dev_alloc(h, &prc, sizeof(PairRec) * cap), "cudaMalloc prec")) return rc;
-  if (int rc = check_cuda(h, dev_alloc(h, &gap, sizeof(float) * cap), "cudaMalloc pgap")) return rc;
-  if (int rc = check_cuda(h, dev_alloc(h, &ipos, sizeof(int) * cap), "cudaMalloc in_pos")) return rc;
-  if (int rc = check_cuda(h, dev_alloc(h, &ifl, cap + 16), "cudaMalloc in_flag")) return rc;
+  A(&inp, sizeof(int2) * cap);
+  A(&own, sizeof(int) * cap);
+  A(&prc, sizeof(PairRec) * cap);
+  A(&gap, sizeof(float) * cap);
+  A(&ipos, sizeof(int) * cap);
+  A(&ifl, cap + 16);
+  if (ce != cudaSuccess) {  // the handle keeps its old arrays and nothing of the new ones
+    for (void* q : made) cudaFree(q);
+    return check_cuda(h, ce, "cudaMalloc pairs");
+  }
   if (old > 0) {
     // keep the current list and history (the rebuild reads them)
     cudaMemcpyAsync(nb[h->rb], h->nbrs[h->rb], sizeof(int) * old, cudaMemcpyDeviceToDevice, h->stream);

@@ -112,6 +112,26 @@ def test_later_build_repeated():
     compare_pairs(g, o)
 
 
+@pytest.mark.parametrize("nth", [2, 6, 12])
+def test_pair_arrays_given_back(nth):
+    """Pair arrays that do not all fit leave the handle its old ones and the
+    device its memory."""
+    import torch
+    prm, arr, walls = settling_case(n_side=(50, 40, 50), box=(52e-3, 42e-3, 52e-3), spacing=1.0, seed=15)[1:]
+    n = arr["radius"].size
+    g = make_system(_gpu, prm, arr, walls)
+    ni, nb, pf = g.download_pairs()
+    before, cap = torch.cuda.mem_get_info()[0], g.memory_info()["pair_capacity"]
+    each = cap // n + 8
+    many = np.minimum(np.arange(1, n + 1) * each, n * each) + 1
+    _fail(g, nth)
+    assert "pairs" in _refused(g.upload_pairs, many, np.ones(n * each, np.int32), np.zeros((n * each, 3)))
+    assert torch.cuda.mem_get_info()[0] == before
+    assert g.memory_info()["pair_capacity"] == cap
+    for a, b in zip(g.download_pairs(), (ni, nb, pf)):
+        assert np.array_equal(a, b)
+
+
 def _fine_gas(interp="GARG_2012"):
     """Spheres of 1 mm in fluid cells of 0.25 mm, several for each search cell."""
     prm, arr, walls = settling_case(n_side=(8, 10, 8), box=(10e-3, 15e-3, 10e-3), spacing=1.02, nsn=5, seed=14)[1:]
