@@ -639,6 +639,7 @@ typedef struct dem_tuning {
  * the fastest; results do not depend on the shapes.  Needs a state and a
  * pair list (after dem_init_neighbors / dem_sys_start). */
 int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out);
+/* the shapes that the next launches have, chosen or not */
 int dem_get_tuning(dem_handle* h, dem_tuning* out);
 int dem_set_tuning(dem_handle* h, const dem_tuning* in);
 

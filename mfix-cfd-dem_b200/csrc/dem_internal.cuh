@@ -288,8 +288,8 @@ struct dem_handle {
     int neigh_threads = 128;                // pair-build scan: threads per block
   } tune;
   bool tuned = false;         // the shapes were measured or set; otherwise pair_shape chooses
-  // Launch shape of the FP64 pair kernel, which keeps `resident` threads on a
-  // multiprocessor.  With eight windows of pairs or more for each resident
+  // Launch shape of the pair kernel.  The FP64 one keeps 512 threads on a
+  // multiprocessor (128 registers).  With eight windows of pairs or more for each resident
   // warp: blocks of two warps, as many as fit the device once, since a second
   // wave of these persistent blocks only waits for the first and small blocks
   // end more evenly (the bed of 1,000,000 spheres, 34,000 windows: 354 us per
@@ -302,14 +302,20 @@ struct dem_handle {
   struct Shape {
     int threads, blocks;
   };
-  Shape pair_shape(int resident) const {
-    if (!tuned && n_pairs / 128 >= 8ll * n_sm * resident / 32) return {64, n_sm * (resident / 64)};
+  Shape pair_shape(bool split) const {
+    constexpr int resident = 512;
+    if (!split && !tuned && n_pairs / 128 >= 8ll * n_sm * resident / 32) return {64, n_sm * (resident / 64)};
     return {tune.pair_threads, n_sm * tune.pair_bpsm};
   }
   // Threads of a block of the gathers: a block leaves when its slowest warp
   // does, so small ones refill sooner (1 % of a step of a bed of 150,001 and of
-  // one of 1,000,000 against blocks of 256).
-  int gather_block() const { return tuned ? tune.gather_threads : 128; }
+  // one of 1,000,000 against blocks of 256).  The split gather stages its warps'
+  // records in shared memory for 128 threads at most.
+  static constexpr int SPLIT_GATHER_MAX = 128;
+  int gather_block(bool split) const {
+    const int t = tuned ? tune.gather_threads : 128;
+    return split && t > SPLIT_GATHER_MAX ? SPLIT_GATHER_MAX : t;
+  }
   bool capturing = false;     // inside a CUDA graph capture: no host syncs
   cudaStream_t own_stream = nullptr;
   // the wall kernels of a force pass run on side_stream beside the pair

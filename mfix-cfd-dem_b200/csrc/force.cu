@@ -927,7 +927,7 @@ static void launch_walls_t(dem_handle* h) {
 template <int COLL, bool B>
 static void launch_pairs_t(dem_handle* h, bool walls) {
   const int c = h->cur;
-  const dem_handle::Shape sh = h->pair_shape(512);  // 128 registers
+  const dem_handle::Shape sh = h->pair_shape(false);
   const int T = sh.threads;
   const WallArgs wa = wall_args(h, T);
   auto go = [&](auto kernel) {
@@ -943,7 +943,7 @@ static void launch_pairs_t(dem_handle* h, bool walls) {
 
 template <int MODE, bool B>
 static void launch_gather_t(dem_handle* h) {
-  const int T = h->gather_block(), G = (h->nl() + T - 1) / T;
+  const int T = h->gather_block(false), G = (h->nl() + T - 1) / T;
   const int c = h->cur;
   launch_pdl(h, k_gather<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
              h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->row_end[h->rb], h->in_start, h->in_mid, h->in_pair,

@@ -432,7 +432,7 @@ __device__ __forceinline__ void add_range(int a, int e, const uint8_t* __restric
 // apart fewer lanes would meet in a bank, but the L1 gets what shared memory
 // leaves, and the bed of 1,000,000 spheres takes 260 us per step so, 264 us the
 // other way.  Chunks of 96 or 64 entries take second turns (3 to 5 % slower).
-constexpr int SPLIT_T = 128;      // threads per block at most
+constexpr int SPLIT_T = dem_handle::SPLIT_GATHER_MAX;
 constexpr int SPLIT_CHUNK = 128;
 struct SplitShared {
   int entry[SPLIT_CHUNK];
@@ -567,8 +567,8 @@ static_assert(2 * sizeof(Rec32) <= sizeof(PairRec) && sizeof(PairRec) == 80, "sp
 template <int COLL, bool B>
 static void launch_pairs_split_t(dem_handle* h) {
   const int c = h->cur;
-  const int T = h->tune.pair_threads;
-  launch_pdl(h, k_pairs_split<COLL, B>, (unsigned)(h->n_sm * h->tune.pair_bpsm), T, h->dp, h->bview(), h->d_np,
+  const dem_handle::Shape sh = h->pair_shape(true);
+  launch_pdl(h, k_pairs_split<COLL, B>, (unsigned)sh.blocks, sh.threads, h->dp, h->bview(), h->d_np,
              h->pair_cap, h->pair_owner, h->nbrs[h->rb], h->in_pos, h->pos4[c], h->vel4[c], h->omg4[c], h->state,
              h->phase, h->pft[h->pcur], h->pflag(), h->in_flag, h->touched, h->pgap, h->skin, h->vslot_pending(),
              rec_own_of(h), rec_in_of(h), h->slipfix, &h->derr->count[c], h->derr);
@@ -585,7 +585,7 @@ void launch_pairs_split(dem_handle* h) {
 
 template <int MODE, bool B>
 static void launch_gather_split_t(dem_handle* h) {
-  const int T = h->tune.gather_threads < SPLIT_T ? h->tune.gather_threads : SPLIT_T, G = (h->nl() + T - 1) / T;
+  const int T = h->gather_block(true), G = (h->nl() + T - 1) / T;
   const int c = h->cur;
   launch_pdl(h, k_gather_split<MODE, B>, G, T, h->dp, h->bview(), h->pos4[c], h->vel4[c], h->omg4[c], h->pos4[1 - c],
              h->vel4[1 - c], h->omg4[1 - c], h->state, h->wf, h->wall_hit, h->touched, h->row_end[h->rb], h->in_start,

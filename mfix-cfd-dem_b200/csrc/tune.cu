@@ -40,9 +40,11 @@ static float time_launches(dem_handle* h, int reps, F&& launch) {
 
 static void fill_out(const dem_handle* h, dem_tuning* o, double pms, double gms, double nms) {
   memset(o, 0, sizeof *o);
-  o->pair_threads = h->tune.pair_threads;
-  o->pair_blocks_per_sm = h->tune.pair_bpsm;
-  o->gather_threads = h->tune.gather_threads;
+  const bool split = h->dp.prec == DEM_PREC_SPLIT;
+  const dem_handle::Shape sh = h->pair_shape(split);
+  o->pair_threads = sh.threads;
+  o->pair_blocks_per_sm = sh.blocks / h->n_sm;
+  o->gather_threads = h->gather_block(split);
   o->neigh_threads = h->tune.neigh_threads;
   o->pair_ms = pms;
   o->gather_ms = gms;
@@ -88,6 +90,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   h->tune.pair_bpsm = best.pair_bpsm;
   for (int T : threads) {
     h->tune.gather_threads = T;
+    if (h->gather_block(h->dp.prec == DEM_PREC_SPLIT) != T) continue;  // not a shape of this gather
     const float ms = time_launches(h, reps, [&] { launch_pairs_only(h); launch_gather_only(h); });
     if (ms - best_p < best_g) { best_g = ms - best_p; best.gather_threads = T; }
   }

@@ -2,11 +2,12 @@
 
 A handle tuned partway (dem_autotune after 10 steps) must reach the same
 state, bit for bit, as an untuned handle over the same steps; tuning a batch
-likewise.  The chosen shapes are among the candidates."""
+likewise.  The chosen shapes are among the candidates, and those reported are
+the ones that run."""
 import numpy as np
 import pytest
 
-from mfix_dem import GpuSystem
+from mfix_dem import GpuSystem, abi
 from cases import make_system, settling_case
 from test_gpu_batch import _add, _batch, _cases, _compare
 
@@ -54,3 +55,40 @@ def test_autotune_batch_keeps_results():
         _compare(bt, sid, g)
         g.close()
     bt.close()
+
+
+def _box(n_side, precision):
+    _, prm, arr, walls = settling_case(n_side=n_side, box=tuple(1.0e-3 * (k + 2) for k in n_side), spacing=0.98,
+                                       jitter=0.01, nsn=5, seed=7, precision=precision)
+    return make_system(lambda p, n: GpuSystem(p, n), prm, arr, walls)
+
+
+SHAPE = ("pair_threads", "pair_blocks_per_sm", "gather_threads", "neigh_threads")
+
+
+# 1,728 spheres; 847,872, past eight windows of 128 pairs for each of the 16
+# warps of a multiprocessor (of 148)
+@pytest.mark.parametrize("n_side,precision,shape", [
+    ((12, 12, 12), abi.DEM_PREC_FP64, (256, 8, 128, 128)),
+    ((12, 12, 12), abi.DEM_PREC_SPLIT, (256, 8, 128, 128)),
+    ((96, 92, 96), abi.DEM_PREC_FP64, (64, 8, 128, 128)),
+    ((96, 92, 96), abi.DEM_PREC_SPLIT, (256, 8, 128, 128))])
+def test_untuned_shapes(n_side, precision, shape):
+    """An untuned handle reports the shapes its rules choose, and setting them
+    changes none."""
+    g = _box(n_side, precision)
+    t = g.get_tuning()
+    assert tuple(t[k] for k in SHAPE) == shape
+    g.set_tuning(t)
+    assert g.get_tuning() == t
+    g.close()
+
+
+def test_split_gather_shapes():
+    """The split gather has blocks of 128 at most: a larger shape is taken as
+    that, and the autotuner does not time it."""
+    g = _box((12, 12, 12), abi.DEM_PREC_SPLIT)
+    g.set_tuning({"pair_threads": 128, "pair_blocks_per_sm": 4, "gather_threads": 256, "neigh_threads": 64})
+    assert g.get_tuning()["gather_threads"] == 128
+    assert g.autotune(reps=3)["gather_threads"] in (64, 128)
+    g.close()
