@@ -636,7 +636,8 @@ typedef struct dem_tuning {
 
 /* Times the candidate launch shapes of the hot kernels on the handle's
  * current state (reps launches each, CUDA events on its stream) and keeps
- * the fastest; results do not depend on the shapes.  Needs a state and a
+ * the fastest; results do not depend on the shapes.  In FP64 the pair
+ * kernel's time includes the wall work, which its launch does as well.  Needs a state and a
  * pair list (after dem_init_neighbors / dem_sys_start). */
 int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out);
 /* the shapes that the next launches have, chosen or not */

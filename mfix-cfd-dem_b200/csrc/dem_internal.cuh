@@ -485,7 +485,9 @@ void launch_wall_gaps(dem_handle* h);          // force.cu: wall clearances at a
 int run_cfnewvalues_outflow(dem_handle* h, bool* force_nsearch);  // outflow.cu: exit velocities, CFNEWVALUES, MASS_OUTFLOW_DEM
 int run_mass_inflow(dem_handle* h);  // inflow.cu: MASS_INFLOW_DEM (entering test, seeding)
 void launch_wall_cand(dem_handle* h);          // desgrid.cu: facet-cell flag of every particle
-void launch_pairs_only(dem_handle* h);         // force.cu: pair kernel of the handle's precision
+void launch_pairs_only(dem_handle* h, bool walls);  // force.cu: pair kernel of the handle's precision; walls: with
+                                               // the wall work, where they are one launch (walls_with_pairs)
+bool walls_with_pairs(const dem_handle* h, bool split);  // force.cu
 void launch_gather_only(dem_handle* h);        // force.cu: gather kernel, forces into FC/TOW
 // capi.cu: parameter block of a system with handle-wide particle count n
 void fill_devparams(const dem_params& q, int n, DevParams& p);

@@ -983,15 +983,18 @@ static void launch_gather_fp64(dem_handle* h, int mode) {
   else launch_gather_t<2, B>(h);
 }
 
+// The wall work and the pairs are one launch (launch_force_kernels).
+bool walls_with_pairs(const dem_handle* h, bool split) { return h->nf > 0 && !split && !h->prof; }
+
 // The two timed parts of the force step for the autotuner.
-void launch_pairs_only(dem_handle* h) {
+void launch_pairs_only(dem_handle* h, bool walls) {
   if (h->dp.prec == DEM_PREC_SPLIT) {
     // no gather in between that would clear the slip list
     cudaMemsetAsync(&h->slipfix->count, 0, sizeof(unsigned), h->stream);
     launch_pairs_split(h);
   }
-  else if (h->batch()) launch_pairs_fp64<true>(h, false);
-  else launch_pairs_fp64<false>(h, false);
+  else if (h->batch()) launch_pairs_fp64<true>(h, walls);
+  else launch_pairs_fp64<false>(h, walls);
 }
 
 void launch_gather_only(dem_handle* h) {
@@ -1012,7 +1015,7 @@ static void launch_force_kernels(dem_handle* h, int mode, bool split) {
   // the gather waits for both (in a captured step, two branches of the
   // graph).  With the parts of the step timed (profiling), they run one after
   // the other.
-  const bool walls = h->nf > 0, merged = walls && !split && !h->prof;
+  const bool walls = h->nf > 0, merged = walls_with_pairs(h, split);
   const bool side = walls && split && h->side_stream && !h->prof;
   if (side) {
     cudaEventRecord(h->ev_fork, h->stream);

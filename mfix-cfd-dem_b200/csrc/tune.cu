@@ -4,9 +4,11 @@
 // resident blocks per SM of its persistent grid), the gather kernel
 // (threads per block) and the count pass of the pair build (threads per
 // block) are timed with CUDA events on the handle's stream, on the handle's
-// own current state, and the fastest shape of each is kept.  The pair
-// history and its flags, which the pair kernel updates in place, are saved
-// before and restored after the timing; everything else the timed launches
+// own current state, and the fastest shape of each is kept.  Where the step's
+// pair launch does the wall work too, the timed one does, since the shape is
+// that of both.  The pair and wall histories and their flags, which these
+// launches update in place, are saved before and restored after the timing;
+// everything else the timed launches
 // write is scratch that the next step rewrites (contact records, FC/TOW, row
 // counts), so tuning does not change any result.  The launch shape does not
 // change the arithmetic, so results are also the same under every shape.
@@ -51,6 +53,38 @@ static void fill_out(const dem_handle* h, dem_tuning* o, double pms, double gms,
   o->neigh_ms = nms;
 }
 
+// What the wall work of the timed pair launches changes, kept for the length
+// of a tuning.
+class WallHistory {
+  dem_handle* h;
+  char* kept = nullptr;
+  size_t n;
+
+  void copy(bool back) {
+    void* const live[3] = {h->wall_pft, h->wall_fid, h->wall_live};
+    const size_t bytes[3] = {sizeof(double) * 3 * h->dp.cmax * n, sizeof(int) * h->dp.cmax * n, n};
+    char* at = kept;
+    for (int k = 0; k < 3; at += bytes[k++])
+      cudaMemcpyAsync(back ? live[k] : at, back ? at : live[k], bytes[k], cudaMemcpyDeviceToDevice, h->stream);
+  }
+
+ public:
+  explicit WallHistory(dem_handle* hh) : h(hh), n((size_t)hh->nl()) {
+    if (!walls_with_pairs(h, h->dp.prec == DEM_PREC_SPLIT)) return;
+    const size_t each = (3 * sizeof(double) + sizeof(int)) * h->dp.cmax + 1;
+    if (dev_alloc(h, &kept, each * n) == cudaSuccess) copy(false);
+  }
+  ~WallHistory() {
+    if (!kept) return;
+    copy(true);
+    cudaStreamSynchronize(h->stream);
+    cudaFree(kept);
+  }
+  WallHistory(const WallHistory&) = delete;
+  // without room for it the pairs are timed alone
+  bool have() const { return kept != nullptr; }
+};
+
 }  // namespace demb
 
 extern "C" {
@@ -72,6 +106,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
     cudaMemcpyAsync(snap + sizeof(double) * 3 * P, h->pflag(), P, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(snap + sizeof(double) * 3 * P + P, h->in_flag, P, cudaMemcpyDeviceToDevice, h->stream);
   }
+  const WallHistory walls(h);
   const int threads[3] = {64, 128, 256};
   const int bpsm[4] = {2, 4, 8, 16};
   float best_p = FLT_MAX, best_g = FLT_MAX, best_n = FLT_MAX;
@@ -80,7 +115,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
     for (int b : bpsm) {
       h->tune.pair_threads = T;
       h->tune.pair_bpsm = b;
-      const float ms = time_launches(h, reps, [&] { launch_pairs_only(h); });
+      const float ms = time_launches(h, reps, [&] { launch_pairs_only(h, walls.have()); });
       if (ms < best_p) { best_p = ms; best.pair_threads = T; best.pair_bpsm = b; }
     }
   // the gather reads the contact marks the pair kernel sets, so each timed
@@ -91,7 +126,7 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   for (int T : threads) {
     h->tune.gather_threads = T;
     if (h->gather_block(h->dp.prec == DEM_PREC_SPLIT) != T) continue;  // not a shape of this gather
-    const float ms = time_launches(h, reps, [&] { launch_pairs_only(h); launch_gather_only(h); });
+    const float ms = time_launches(h, reps, [&] { launch_pairs_only(h, walls.have()); launch_gather_only(h); });
     if (ms - best_p < best_g) { best_g = ms - best_p; best.gather_threads = T; }
   }
   h->tune = t;

@@ -92,3 +92,40 @@ def test_split_gather_shapes():
     assert g.get_tuning()["gather_threads"] == 128
     assert g.autotune(reps=3)["gather_threads"] in (64, 128)
     g.close()
+
+
+def _on_a_floor():
+    """400 spheres sliding on a floor of 12,800 facets of 0.25 mm, some five
+    hundred in each DES cell; each starts inside a facet."""
+    L, m, k = 20e-3, 80, 20
+    case, prm, arr, _ = settling_case(n_side=(k, 1, k), box=(L, 12e-3, L), spacing=1.0, jitter=0.0, vmax=0.05, mew=0.3)
+    arr["pos"] += np.array([[0.06e-3], [0.0], [0.09e-3]])
+    arr["pos"][1], arr["vel"][1] = 0.499e-3, 0.0
+    x, z = np.meshgrid(np.arange(m) * L / m, np.arange(m) * L / m, indexing="ij")
+    p = np.stack([x, 0 * x, z], -1).reshape(-1, 3)
+    ex, ez = np.array([L / m, 0, 0]), np.array([0, 0, L / m])
+    tri = np.concatenate([np.stack([p, p + ez, p + ex], -1), np.stack([p + ex, p + ez, p + ex + ez], -1)])
+    return prm, arr, (tri, np.tile([0.0, 1.0, 0.0], (tri.shape[0], 1)))
+
+
+def test_autotune_times_the_walls():
+    """The FP64 step does the walls in the pair launch, and so does the timed
+    one: on a floor of many facets it takes several times the pairs alone.
+    The wall histories are as they were."""
+    prm, arr, floor = _on_a_floor()
+    a, b, c = (make_system(lambda p, n: GpuSystem(p, n), prm, arr, w) for w in (floor, floor, (floor[0][:0], floor[1][:0])))
+    for s in (a, b, c):
+        s.step(10)
+    t, bare = b.autotune(reps=20), c.autotune(reps=20)
+    assert t["pair_ms"] > 3.0 * bare["pair_ms"]
+    ha, hb = a.download_wall_history(), b.download_wall_history()
+    assert (ha[0] > 0).sum() >= 400 and np.abs(ha[1]).max() > 0.0
+    for x, y in zip(ha, hb):
+        assert np.array_equal(x, y)
+    for s in (a, b):
+        s.step(40)
+    sa, sb = a.download_state(), b.download_state()
+    for k in ("pos", "vel", "omega", "state"):
+        assert np.array_equal(sa[k], sb[k]), k
+    for s in (a, b, c):
+        s.close()
