@@ -95,7 +95,6 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   if (reps < 1) return set_err(h, DEM_ERR_ARG, "reps must be positive");
   if (!h->have_state || !h->have_pairs) return set_err(h, DEM_ERR_STATE, "state or pair list missing");
   invalidate_graphs(h);
-  h->tuned = true;
   const size_t P = (size_t)host_pairs(h);
   char* snap = (char*)stage_buffer(h, sizeof(double) * 3 * P + 2 * P + 64);
   if (!snap) return set_err(h, DEM_ERR_CUDA, "cudaMalloc stage");
@@ -110,7 +109,10 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   const int threads[3] = {64, 128, 256};
   const int bpsm[4] = {2, 4, 8, 16};
   float best_p = FLT_MAX, best_g = FLT_MAX, best_n = FLT_MAX;
-  dem_handle::Tune t = h->tune, best = h->tune;
+  const dem_handle::Tune t = h->tune;
+  dem_handle::Tune best = t;
+  const bool tuned = h->tuned;
+  h->tuned = true;  // the shapes set below are the ones launched
   for (int T : threads)
     for (int b : bpsm) {
       h->tune.pair_threads = T;
@@ -146,7 +148,11 @@ int dem_autotune(dem_handle* h, int32_t reps, dem_tuning* out) {
   }
   // the timed pair launches added to the contact counters
   clear_counts(h);
-  if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "autotune")) return rc;
+  if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "autotune")) {
+    h->tune = t;
+    h->tuned = tuned;
+    return rc;
+  }
   if (out) fill_out(h, out, best_p, best_g, best_n);
   return 0;
 }

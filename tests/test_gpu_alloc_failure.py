@@ -6,6 +6,7 @@ handle's n-th allocation from then on one that no device can serve, so the
 error paths run without filling the device.
 """
 import ctypes as C
+import gc
 
 import numpy as np
 import pytest
@@ -121,15 +122,30 @@ def test_pair_arrays_given_back(nth):
     n = arr["radius"].size
     g = make_system(_gpu, prm, arr, walls)
     ni, nb, pf = g.download_pairs()
+    gc.collect()
     before, cap = torch.cuda.mem_get_info()[0], g.memory_info()["pair_capacity"]
     each = cap // n + 8
     many = np.minimum(np.arange(1, n + 1) * each, n * each) + 1
     _fail(g, nth)
     assert "pairs" in _refused(g.upload_pairs, many, np.ones(n * each, np.int32), np.zeros((n * each, 3)))
-    assert torch.cuda.mem_get_info()[0] == before
+    # 12.8 MB and more were allocated before the one that failed; small blocks
+    # of other handles may have gone back besides
+    assert torch.cuda.mem_get_info()[0] >= before
     assert g.memory_info()["pair_capacity"] == cap
     for a, b in zip(g.download_pairs(), (ni, nb, pf)):
         assert np.array_equal(a, b)
+
+
+def test_tuning_that_fails_chooses_nothing():
+    """The automatic launch shapes stay when the autotuner has no room for the
+    histories it keeps (more of them than the upload staged)."""
+    prm, arr, walls = settling_case(n_side=(12, 12, 12), spacing=0.75, jitter=0.01, seed=16)[1:]
+    g = make_system(_gpu, prm, arr, walls)
+    assert 26 * g.pair_count() > 100 * arr["radius"].size
+    t = g.get_tuning()
+    _fail(g)
+    _refused(g.autotune)
+    assert g.get_tuning() == t and t["gather_threads"] == 128
 
 
 def _fine_gas(interp="GARG_2012"):
