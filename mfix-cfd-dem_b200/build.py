@@ -40,7 +40,7 @@ SOURCES = {
     "outflow.cu": ["-fmad=false"],
     "inflow.cu": ["-fmad=false"],
 }
-HEADERS = ["dem_internal.cuh"]
+HEADERS = ["dem_internal.cuh", "quotient.cuh"]
 
 
 def nvcc():

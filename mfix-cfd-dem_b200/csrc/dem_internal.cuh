@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/dem_b200.h"
+#include "quotient.cuh"
 
 namespace demb {
 
@@ -709,47 +710,6 @@ __device__ __forceinline__ void cross3(const double x[3], const double y[3], dou
   o[0] = x[1] * y[2] - x[2] * y[1];
   o[1] = x[2] * y[0] - x[0] * y[2];
   o[2] = x[0] * y[1] - x[1] * y[0];
-}
-
-// Several quotients by one divisor, each rounded as the IEEE division rounds
-// it.  A division is a chain of some twenty instructions with a branch that
-// keeps the next one from starting beside it, and the contact arithmetic has up to
-// eight by two divisors.  Here the divisor's reciprocal is divided out once
-// and each quotient takes five multiply-adds that run side by side: a product
-// within two units in the last place, one correction that brings it within
-// one, and a last one whose remainder is exact, so that the sum rounds
-// correctly (P. Markstein, Computation of elementary functions on the IBM RISC
-// System/6000 processor, IBM J. Res. Dev. 34 (1990), theorems on the
-// remainder and on the final rounding).  This holds while neither the
-// remainders underflow nor the products overflow: the callers divide plainly
-// unless div_range() holds (numerators under 2^-960 are rounded within a unit
-// in the last place).  Per step, plain divisions and so: bed of 1,000,000
-// spheres 354 and 342 us, split 260 and 249 us; 150,001 with Adams-Bashforth
-// 72.9 and 68.3 us; gas of 200,003 59.6 and 57.5 us; a batch of 16 columns 117
-// and 111 us.
-__device__ __forceinline__ double quotient(double a, double b, double y) {
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return copysign(q, a);  // of a zero: the divisors here are positive
-}
-// Divisor b and the sum of the quotients' magnitudes: in the range of quotient()?
-__device__ __forceinline__ bool div_range(double b, double sum) {
-  return b > 0x1p-400 && b < 0x1p400 && sum < 0x1p600;
-}
-__device__ __forceinline__ void div3(const double a[3], double b, double y, double q[3]) {
-  double d[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) d[c] = quotient(a[c], b, y);
-  if (!div_range(b, fabs(d[0]) + fabs(d[1]) + fabs(d[2]))) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) d[c] = a[c] / b;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) q[c] = d[c];
-}
-__device__ __forceinline__ void div3(const double a[3], double b, double q[3]) {
-  div3(a, b, 1.0 / b, q);
 }
 
 __device__ __forceinline__ int dg_funijk(const DevParams& p, int i, int j, int k) {

@@ -56,21 +56,8 @@ __device__ __forceinline__ void contact_force(const DevParams& p, const PState& 
   const double rl = L.r, ri = I.r;
   const double r_lm = rl + ri;
   const double dmag = sqrt(d2);
-  // the normal and the two lever arms, all divided by dmag (half a quotient is
-  // the quotient by twice the divisor)
-  const double num_dcl = dmag * dmag + rl * rl - ri * ri, num_dcl2 = rl * rl - ri * ri;
-  const double y_dmag = 1.0 / dmag;
   double nrm[3], dcl, half;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) nrm[c] = quotient(dist[c], dmag, y_dmag);
-  dcl = 0.5 * quotient(num_dcl, dmag, y_dmag);
-  half = 0.5 * quotient(num_dcl2, dmag, y_dmag);
-  if (!div_range(dmag, fabs(dcl) + fabs(half))) {  // |nrm| is at most one
-#pragma unroll
-    for (int c = 0; c < 3; ++c) nrm[c] = dist[c] / dmag;
-    dcl = num_dcl / (2.0 * dmag);
-    half = num_dcl2 / (2.0 * dmag);
-  }
+  contact_quotients(dist, dmag, rl, ri, nrm, dcl, half);
   const double overlap_n = r_lm - dmag;
   // CFRELVEL
   double vrel[3];
