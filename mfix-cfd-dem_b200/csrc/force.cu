@@ -1129,12 +1129,14 @@ int run_split_force_error(dem_handle* h, double* rel_err) {
   };
   std::vector<double> f64(3 * n), f32(3 * n);
   h->dp.first_pass = 0;
-  h->count_dirty = true;  // the counts of the two passes stay
   save();
   launch_force_kernels(h, 0, false);
   cudaMemcpyAsync(f64.data(), h->fc, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream);
   restore();
+  clear_counts(h);
   launch_force_kernels(h, 0, true);
+  h->count_set = h->cur;  // the second pass is the last force evaluation
+  h->count_dirty = true;
   cudaMemcpyAsync(f32.data(), h->fc, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream);
   restore();
   if (int rc = check_cuda(h, cudaStreamSynchronize(h->stream), "force error")) return rc;

@@ -209,6 +209,29 @@ def test_contact_counts_of_mixed_passes():
     compare_state(g, o, exact=True)
 
 
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+def test_contact_counts_of_a_force_error(prec):
+    """Behind dem_force_error, whose second pass is the last force evaluation,
+    whether a step or a pass without integration came before."""
+    from mfix_dem import abi
+    case, prm, arr, walls = settling_case(n_side=(6, 10, 6), spacing=0.98, jitter=0.02, vmax=0.0, nsn=5,
+                                          precision=abi.DEM_PREC_SPLIT if prec == "split" else abi.DEM_PREC_FP64)
+    g, o = pair_both(prm, arr, walls)
+    for again in range(2):
+        for s in (g, o):
+            s.calc_force()
+        g.force_error()
+        a, b = g.stats(), o.stats()
+        assert (a["n_contacts"], a["n_wall_contacts"]) == (b["n_contacts"], b["n_wall_contacts"])
+        assert a["n_contacts"] > 0 and a["n_wall_contacts"] > 0
+        for s in (g, o):
+            s.step(1)
+        g.force_error()
+        for s in (g, o):
+            s.calc_force()
+        assert g.stats()["n_contacts"] == o.stats()["n_contacts"]
+
+
 @pytest.mark.parametrize("interp", ["GARG_2012", "NONE"])
 def test_gas_fields_set_again(interp):
     from mfix_dem import configs
