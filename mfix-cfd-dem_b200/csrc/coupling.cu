@@ -43,7 +43,6 @@ struct Gas {
   // ascending index, pic_dat what the deposition needs of each entry
   int* pic_cnt = nullptr; int* pic_start = nullptr; int* pic_tmp = nullptr; int* pic_list = nullptr;
   double4* pic_dat = nullptr;
-  bool have_mean = false;
 };
 
 namespace demb {
@@ -435,10 +434,6 @@ __global__ void k_fgds(GasDev G, const double* __restrict__ drag_am, double* __r
 
 // ---- DES_INTERP_SCHEME = NONE: the ...1 routines without a filter ------
 
-__device__ __forceinline__ double sphere_vol(const GasDev& G, double r) {
-  return ((4.0 / 3.0) * G.pi) * (r * (r * r));
-}
-
 // DRAG_GS_DES1 without a filter (drag_gs_des1.f:34-160, Model A, not
 // explicitly coupled), per NORMAL particle: cell-centre gas velocity, F_GP
 // by DES_DRAG_GP, FC += F_GP*(u_g - v_p) + P_FORCE*PVOL; F_GP = 0 outside the
@@ -712,14 +707,12 @@ static int run_mean_fields(dem_handle* h, bool located = false) {
   if (s->g.interp_scheme == DEM_INTERP_NONE) {   // COMP_MEAN_FIELDS1
     launch_pdl(h, G.M == 1 ? k_mean_fields1<true> : k_mean_fields1<false>, (G.ncell + T - 1) / T, T, G, s->pic_dat, h->phase, s->pic_start, s->pic_list,
                s->rop_s, s->ep_g);
-    s->have_mean = true;
     return check_cuda(h, cudaGetLastError(), "mean fields");
   }
   const int nnodes = (G.imax + 1) * (G.jmax + 1) * (G.no_k ? 1 : G.kmax + 1);
   launch_pdl(h, G.M == 1 ? k_node_deposit<true> : k_node_deposit<false>, (nnodes + T - 1) / T, T, G, s->pic_dat, h->phase, s->pic_start, s->pic_list,
              s->vol_surr, s->dens_node);
   launch_pdl(h, k_cell_fields, (G.ncell + T - 1) / T, T, G, s->dens_node, s->rop_s, s->ep_g);
-  s->have_mean = true;
   return check_cuda(h, cudaGetLastError(), "mean fields");
 }
 
@@ -862,7 +855,6 @@ int dem_set_gas_fields(dem_handle* h, const dem_fluid_grid* g, const double* ep_
   s->M = h->dp.nph;
   s->pi = 4.0 * std::atan(1.0);
   s->vol = g->dx * g->dy * (h->dp.no_k ? (h->prm.domain_hi[2] - h->prm.domain_lo[2]) : g->dz);
-  s->have_mean = false;
   const size_t nc = s->ncell;
   // face positions, accumulated as the fluid grid set-up does
   auto faces = [](double lo, double d, int n) {

@@ -508,8 +508,10 @@ void handle_arrays(dem_handle* h, size_t n, size_t nc, size_t nfc, F&& A) {
     A((void**)&h->vel4[b], sizeof(double4) * n);
     A((void**)&h->row_end[b], sizeof(int) * n);
   }
-  // the spin is one array under both buffer names: only the integrating
-  // gather of a particle writes it, after every kernel that reads it
+  // the spin is one array under both buffer names: the kernels that write it
+  // in a step (the integrating gathers, k_coupled_step, k_integrate and its
+  // outflow form, the deletions) each write the thread's own particle, behind
+  // every kernel that reads other particles' spins
   A((void**)&h->omg4[0], sizeof(double4) * n);
   h->omg4[1] = h->omg4[0];
   A((void**)&h->state, n);

@@ -36,16 +36,6 @@ struct PState {  // one particle's gathered state
   int ph;
 };
 
-__device__ __forceinline__ void load_p(const double4* __restrict__ pos4, const double4* __restrict__ vel4,
-                                       const double4* __restrict__ omg4, const uint8_t* __restrict__ phase,
-                                       int i, PState& s) {
-  double4 a = pos4[i], b = vel4[i], c = omg4[i];
-  s.x[0] = a.x; s.x[1] = a.y; s.x[2] = a.z; s.r = a.w;
-  s.v[0] = b.x; s.v[1] = b.y; s.v[2] = b.z; s.m = b.w;
-  s.w[0] = c.x; s.w[1] = c.y; s.w[2] = c.z;
-  s.ph = phase[i];
-}
-
 // Contact part of one CC iteration of CALC_FORCE_DEM (calc_force_dem.f:
 // 273-363) with CFRELVEL (cfrelvel.f:54-77) for owner L and neighbour I in
 // contact; dist = x_I - x_L and d2 = |dist|^2 come from the apart test.
