@@ -5,7 +5,8 @@ the oracle.
   pair counts at and around multiples of both;
 - the wall work takes one particle per thread up to two blocks per
   multiprocessor and four past that: bed sizes on both sides, with the counts
-  not a multiple of four;
+  not a multiple of four, alone and in a batch, in the launch of the pairs and
+  in one of their own (split precision, timed parts);
 - the scans take a second level past 4096 tiles of 2048 cells: a search grid
   just over it; their scratch grows between replays of captured steps;
 - a pair list that outgrows its arrays inside a captured step, with empty rows
@@ -16,7 +17,9 @@ the oracle.
   busy for eight windows, against the larger ones;
 - contact lists of more than 32 entries, and warps with more than 128;
 - masses past the range in which quotients share a reciprocal;
-- the deposition of more than one solids phase.
+- the deposition of more than one solids phase;
+- coupled steps with either integrator, in split precision, and with periodic axes
+  (where the cell search of the next step cannot ride on the integration).
 
 FP64 results are the oracle's bit for bit (as everywhere in the parity tests);
 the split path is held to the tolerances of its own tests (positions 1e-6,
@@ -91,6 +94,66 @@ def test_wall_work_by_size(n_side):
     fo, po = o.download_wall_history()
     assert np.array_equal(fg, fo)
     assert np.array_equal(pg[fg >= 0], po[fo >= 0])
+
+
+def _full_box(n_side, seed=61, **kw):
+    """Spheres whose outer layers start at or in the walls, one less than the
+    lattice holds."""
+    box = tuple(0.999e-3 * k for k in n_side)
+    case, prm, arr, walls = settling_case(n_side=n_side, box=box, spacing=0.999, jitter=0.01, vmax=0.2, nsn=5, seed=seed,
+                                          **kw)
+    return case, prm, {k: (v[..., :-1].copy() if v.ndim else v) for k, v in arr.items()}, walls
+
+
+@pytest.mark.parametrize("coll", ["LSD", "HERTZ"])
+@pytest.mark.parametrize("prec,timed", [("fp64", True), ("split", False), ("split", True)])
+def test_walls_in_their_own_launch(coll, prec, timed):
+    """79,334 spheres in split precision, or with the parts of the step timed."""
+    from mfix_dem import abi
+    case, prm, arr, walls = _full_box((45, 41, 43), coll=coll,
+                                      precision=abi.DEM_PREC_SPLIT if prec == "split" else abi.DEM_PREC_FP64)
+    g, o = pair_both(prm, arr, walls)
+    if timed:
+        g.set_profiling(2)
+    g.step(17)
+    o.step(17)
+    assert o.stats()["n_wall_contacts"] > 1000
+    if prec == "fp64":
+        compare_state(g, o, exact=True)
+        assert g.stats()["n_wall_contacts"] == o.stats()["n_wall_contacts"]
+        assert all(np.array_equal(a, b) for a, b in zip(g.download_wall_history(), o.download_wall_history()))
+    else:
+        sg, so = g.download_state(), o.download_state()
+        assert rel_err(sg["pos"], so["pos"]) <= 1e-6
+        assert rel_err(sg["vel"], so["vel"]) <= 1e-3
+
+
+@pytest.mark.parametrize("coll", ["LSD", "HERTZ"])
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+def test_wall_work_of_a_batch(coll, prec):
+    """Boxes of 41,327 and 39,311 spheres, together past 75,776, each against
+    the oracle; the second box has other walls and another period."""
+    from mfix_dem import abi
+    from oracle_ffi import OracleSystem
+    from test_gpu_batch import _add, _batch
+    precision = abi.DEM_PREC_SPLIT if prec == "split" else abi.DEM_PREC_FP64
+    cases = [_full_box((36, 28, 41), seed=62, coll=coll, precision=precision),
+             _full_box((27, 52, 28), seed=63, coll=coll, mew=0.3, precision=precision)]
+    bt = _batch(cases)
+    ids = [_add(bt, c) for c in cases]
+    bt.start(ids)
+    bt.step(17)
+    for sid, (case, prm, arr, walls) in zip(ids, cases):
+        o = make_system(OracleSystem, prm, arr, walls)
+        o.step(17)
+        assert o.stats()["n_wall_contacts"] > 500
+        sb, so = bt.download_state(sid), o.download_state()
+        for k in ("pos", "vel", "omega"):
+            if prec == "fp64":
+                assert np.array_equal(sb[k], so[k]), k
+            elif k != "omega":
+                assert rel_err(sb[k], so[k]) <= (1e-6 if k == "pos" else 1e-3), k
+    bt.close()
 
 
 def test_scan_of_many_search_cells():
@@ -349,3 +412,43 @@ def test_deposition_of_two_phases(interp):
         assert rel_err(a, b) <= 1e-10
     assert prm.n_phases == 2
     assert rel_err(g.calc_des_bedheight(), o.calc_des_bedheight()) <= 1e-10
+
+
+@pytest.mark.parametrize("periodic", [(False, False, False), (True, False, True)])
+@pytest.mark.parametrize("interp", ["GARG_2012", "NONE"])
+@pytest.mark.parametrize("intg,prec", [("EULER", "fp64"), ("ADAMS_BASHFORTH", "fp64"), ("EULER", "split"),
+                                       ("ADAMS_BASHFORTH", "split")])
+def test_coupled_step_forms(intg, prec, interp, periodic):
+    """The coupled case with its spheres in contact, 23 steps with three pair
+    builds; with periodic x and z some cross a face."""
+    import dataclasses
+    from mfix_dem import abi
+    from mfix_dem import params as P
+    from oracle_ffi import OracleSystem
+    case, prm, arr, walls, info, grid, f = coupled_case(spacing=0.99, nsn=10, interp=interp)
+    case = dataclasses.replace(case, intg_method=intg, periodic=periodic,
+                               force_precision=abi.DEM_PREC_SPLIT if prec == "split" else abi.DEM_PREC_FP64)
+    prm, info = P.build_params(case, arr["radius"], arr["pmass"], arr["phase"], arr["state"])
+    rng = np.random.default_rng(77)
+    arr = dict(arr, vel=rng.uniform(-2.0, 2.0, arr["vel"].shape))
+    if periodic[0]:   # the first layers about the faces
+        arr["pos"] = arr["pos"] - np.array([[0.24e-3], [0.0], [0.24e-3]])
+    walls = P.default_walls(case.domain_lo, case.domain_hi, periodic=periodic)
+    ct = (case, prm, arr, walls, info, grid, f)
+    g, o = make_coupled(_gpu, ct), make_coupled(OracleSystem, ct)
+    x0 = o.download_state()["pos"][0]
+    for steps in (1, 3, 19):
+        for s in (g, o):
+            s.step_coupled(steps)
+        sg, so = g.download_state(), o.download_state()
+        assert np.array_equal(sg["state"], so["state"])
+        if prec == "fp64":
+            compare_state(g, o)
+            assert g.stats()["n_contacts"] == o.stats()["n_contacts"] > 100
+        else:
+            assert rel_err(sg["pos"], so["pos"]) <= 1e-6
+            assert rel_err(sg["vel"], so["vel"]) <= 1e-3
+        for a, b in zip(g.get_mean_fields(), o.get_mean_fields()):
+            assert rel_err(a, b) <= (1e-10 if prec == "fp64" else 1e-4)
+    if periodic[0]:
+        assert (np.abs(so["pos"][0] - x0) > 4e-3).sum() > 3
