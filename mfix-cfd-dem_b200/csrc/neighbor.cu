@@ -75,9 +75,10 @@ __device__ __forceinline__ void delete_rogue(const DevParams& p, int i, int8_t* 
 // starts the row counts of the build: zero, or for a batch system that does
 // not rebuild now the length of the particle's current row (rows of the
 // current list end at n_old, see k_fill_rows).
-// A build is some twenty launches, most of them short: with the passes over
-// the particles joined (40 launches before) a build of 200,000 spheres of a
-// gas, 31 us less.
+// A build of one system is 20 launches, 21 with walls (15 and 16 in a batch,
+// which has no candidate list), most of them short: with the passes over the
+// particles joined (40 launches before) a build of 200,000 spheres of a gas,
+// 31 us less.
 template <bool B>
 __global__ void k_sorted_copy(DevParams p0, BatchView bv, int n, int n_old, const int* __restrict__ fkey,
                               const int* __restrict__ fslot, const int* __restrict__ fstart,
