@@ -157,7 +157,7 @@ int dem_abi_version(void);
  * BIN_FACETS_TO_DG (model/des/stl_preproc_des_mod.f:135-203, TRI_BOX_OVERLAP
  * in stl_functions_des_mod.f:280-536) and flags edges shared by near-coplanar
  * facets as FLAG_FACETS_WHERE_EDGE_COLLISION_IS_IGNORED (stl_preproc_des_mod.f:
- * 361-490) does.  n_facets may be 0. */
+ * 361-490) does.  n_facets may be 0.  A call that fails leaves no walls. */
 /* DTSOLID of the following steps.  A coupled driver shortens the last DEM
  * step of each fluid step so the solids time lands on the fluid time
  * (DTSOLID = TIME + DT - S_TIME, des_time_march.f:308-314) and puts the
@@ -715,7 +715,8 @@ int dem_batch_create(const dem_params* common, const dem_batch_limits* lim, dem_
 int dem_sys_add(dem_handle* h, const dem_params* p, int32_t max_pip, int32_t* sys);
 /* Removes a system; its ranges become free for later systems. */
 int dem_sys_remove(dem_handle* h, int32_t sys);
-/* dem_set_walls / dem_upload_state / dem_download_state of one system
+/* dem_set_walls (here too a call that fails, DEM_ERR_CAPACITY past the limits,
+ * leaves the system no walls) / dem_upload_state / dem_download_state of one system
  * (arrays with max_pip rows, max_pip <= its capacity). */
 int dem_sys_set_walls(dem_handle* h, int32_t sys, const double* vertex, const double* norm_face, int32_t nf);
 int dem_sys_upload_state(dem_handle* h, int32_t sys, const double* pos, const double* vel,

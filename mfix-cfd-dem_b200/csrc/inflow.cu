@@ -249,8 +249,17 @@ int dem_set_inflow_bcs(dem_handle* h, const dem_inflow_bc* bcs, int32_t n, uint6
       if (b.dg_lo[a] > b.dg_hi[a]) return set_err(h, DEM_ERR_ARG, "empty DES-cell box");
     if (!(b.pi_factor > 0.0) && b.pi_count > 0) return set_err(h, DEM_ERR_ARG, "PI_FACTOR must be positive");
   }
+  // what can fail comes first: the handle then keeps the boundaries it had
+  dem_inflow_bc* d_ibc = nullptr;
+  if (n > 0) {
+    if (!h->pic_fresh) {
+      if (int rc = check_cuda(h, dev_alloc(h, &h->pic_fresh, (size_t)h->n), "cudaMalloc pic_fresh")) return rc;
+    }
+    if (int rc = check_cuda(h, dev_alloc(h, &d_ibc, sizeof(dem_inflow_bc) * n), "cudaMalloc inflow")) return rc;
+  }
   cudaStreamSynchronize(h->stream);
-  if (h->d_ibc) { cudaFree(h->d_ibc); h->d_ibc = nullptr; }
+  if (h->d_ibc) cudaFree(h->d_ibc);
+  h->d_ibc = d_ibc;
   h->ibc.clear();
   h->irand.clear();
   h->irng = seed;
@@ -271,11 +280,7 @@ int dem_set_inflow_bcs(dem_handle* h, const dem_inflow_bc* bcs, int32_t n, uint6
     I.bc.p = nullptr; I.bc.q = nullptr; I.bc.poly_layout = nullptr; I.bc.w_cell = nullptr; I.bc.h_cell = nullptr;
     h->ibc.push_back(std::move(I));
   }
-  if (!h->pic_fresh) {
-    if (int rc = check_cuda(h, dev_alloc(h, &h->pic_fresh, (size_t)h->n), "cudaMalloc pic_fresh")) return rc;
-  }
   cudaMemsetAsync(h->pic_fresh, 0, (size_t)h->n, h->stream);
-  if (int rc = check_cuda(h, dev_alloc(h, &h->d_ibc, sizeof(dem_inflow_bc) * n), "cudaMalloc inflow")) return rc;
   std::vector<dem_inflow_bc> dev(n);
   for (int32_t i = 0; i < n; ++i) dev[i] = h->ibc[i].bc;
   cudaMemcpyAsync(h->d_ibc, dev.data(), sizeof(dem_inflow_bc) * n, cudaMemcpyHostToDevice, h->stream);

@@ -214,13 +214,17 @@ int dem_set_outflow_bcs(dem_handle* h, const dem_outflow_bc* bcs, int32_t n) {
       if (overlap) return set_err(h, DEM_ERR_ARG, "outflow boundary boxes overlap");
     }
   }
+  // what can fail comes first: the handle then keeps the boundaries it had
+  dem_outflow_bc* d_obc = nullptr;
+  if (n > 0)
+    if (int rc = check_cuda(h, dev_alloc(h, &d_obc, sizeof(dem_outflow_bc) * n), "cudaMalloc outflow")) return rc;
   cudaStreamSynchronize(h->stream);
-  if (h->d_obc) { cudaFree(h->d_obc); h->d_obc = nullptr; }
+  if (h->d_obc) cudaFree(h->d_obc);
+  h->d_obc = d_obc;
   h->obc.assign(bcs, bcs + n);
   h->exit_first_pass = true;
   invalidate_graphs(h);
   if (n > 0) {
-    if (int rc = check_cuda(h, dev_alloc(h, &h->d_obc, sizeof(dem_outflow_bc) * n), "cudaMalloc outflow")) return rc;
     cudaMemcpyAsync(h->d_obc, bcs, sizeof(dem_outflow_bc) * n, cudaMemcpyHostToDevice, h->stream);
   }
   return check_cuda(h, cudaStreamSynchronize(h->stream), "outflow boundaries");

@@ -159,7 +159,7 @@ __global__ void k_edge_flags(int ncell, const int* __restrict__ start, const Fac
   }
 }
 
-int run_bin_facets(dem_handle* h, const double* vf, const double* nfort, int nf) {
+static int bin_facets(dem_handle* h, const double* vf, const double* nfort, int nf) {
   const DevParams& p = h->dp;
   invalidate_graphs(h);
   cudaFree(h->vertex); cudaFree(h->norm_face); cudaFree(h->ignore_edge); cudaFree(h->fbin);
@@ -207,6 +207,18 @@ int run_bin_facets(dem_handle* h, const double* vf, const double* nfort, int nf)
   return check_cuda(h, cudaStreamSynchronize(h->stream), "bin facets");
 }
 
+// Walls that could not be set leave none: the bins of a call that failed point
+// at arrays that are not there.
+int run_bin_facets(dem_handle* h, const double* vf, const double* nfort, int nf) {
+  const int rc = bin_facets(h, vf, nfort, nf);
+  if (rc) {
+    h->nf = 0;
+    cudaMemsetAsync(h->fbin_start, 0, sizeof(int) * (h->dp.ncell2 + 1), h->stream);
+    launch_wall_cand(h);
+  }
+  return rc;
+}
+
 __global__ void k_add_int(int n, int* __restrict__ a, int v) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] += v;
@@ -217,13 +229,17 @@ __global__ void k_add_int(int n, int* __restrict__ a, int v) {
 // ncell2 + 1 entries of fbin_start from its cell_off (its own end pointer
 // included), so binning one system leaves the others untouched.  Facet ids
 // in the bins and in the wall history are handle-wide.
-int run_bin_facets_sys(dem_handle* h, int sys, const double* vf, const double* nfort, int nf) {
-  SysSlot& S = h->sys[sys];
-  const DevParams& p = S.dp;
-  invalidate_graphs(h);
+static void give_facets(dem_handle* h, SysSlot& S) {
   if (S.nf > 0) h->fac_alloc.give(S.fac_off, S.nf);
   if (S.nbin > 0) h->bin_alloc.give(S.bin_off, S.nbin);
   S.nf = 0; S.nbin = 0; S.fac_off = 0; S.bin_off = 0;
+}
+
+static int bin_facets_sys(dem_handle* h, int sys, const double* vf, const double* nfort, int nf) {
+  SysSlot& S = h->sys[sys];
+  const DevParams& p = S.dp;
+  invalidate_graphs(h);
+  give_facets(h, S);
   int* fs = h->fbin_start + p.cell_off;
   if (int rc = check_cuda(h, cudaMemsetAsync(fs, 0, sizeof(int) * (p.ncell2 + 1), h->stream), "memset")) return rc;
   if (nf == 0) {
@@ -262,6 +278,17 @@ int run_bin_facets_sys(dem_handle* h, int sys, const double* vf, const double* n
   DEM_LAUNCH(h);
   launch_wall_cand(h);
   return check_cuda(h, cudaStreamSynchronize(h->stream), "bin facets");
+}
+
+int run_bin_facets_sys(dem_handle* h, int sys, const double* vf, const double* nfort, int nf) {
+  const int rc = bin_facets_sys(h, sys, vf, nfort, nf);
+  if (rc) {  // none, as for a single system
+    SysSlot& S = h->sys[sys];
+    give_facets(h, S);
+    cudaMemsetAsync(h->fbin_start + S.dp.cell_off, 0, sizeof(int) * (S.dp.ncell2 + 1), h->stream);
+    launch_wall_cand(h);
+  }
+  return rc;
 }
 
 }  // namespace demb

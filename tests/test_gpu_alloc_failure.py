@@ -136,6 +136,81 @@ def test_pair_arrays_given_back(nth):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("nth", [1, 2, 3, 4])
+def test_walls_that_do_not_fit(nth):
+    """Facets, or their bins, without room: no walls, until they are set again."""
+    from oracle_ffi import OracleSystem
+    prm, arr, walls = settling_case(n_side=(8, 6, 8), box=(9e-3, 40e-3, 9e-3), spacing=1.05, nsn=5, vmax=0.3, seed=18)[1:]
+    none = (walls[0][:0], walls[1][:0])
+    g, o = make_system(_gpu, prm, arr, walls), make_system(OracleSystem, prm, arr, none)
+    _fail(g, nth)
+    _refused(g.set_walls, *walls)
+    for s in (g, o):
+        s.step(12)
+    compare_state(g, o, exact=True)
+    for s in (g, o):
+        s.set_walls(*walls)
+        s.step(40)
+    assert o.stats()["n_wall_contacts"] == g.stats()["n_wall_contacts"] > 0
+    compare_state(g, o, exact=True)
+
+
+def test_walls_past_the_limits_of_a_batch():
+    """Facet bins that a batch has no room for: the system has no walls, the
+    other keeps its own, and the room is free for smaller ones."""
+    from mfix_dem import GpuBatch, abi, load_library
+    from mfix_dem import params as P
+    from mfix_dem.system import DemError
+    from test_gpu_batch import _add, _compare, _entry
+    a = settling_case(n_side=(8, 6, 8), box=(9e-3, 40e-3, 9e-3), spacing=1.05, nsn=5, vmax=0.3, seed=19)
+    b = settling_case(n_side=(6, 6, 6), box=(9e-3, 40e-3, 9e-3), spacing=1.05, nsn=5, vmax=0.3, seed=20)
+    lim = P.batch_limits(load_library(), [_entry(a), _entry(b)])
+    many = tuple(np.concatenate([w] * 40) for w in b[3])
+    lim.max_facets = 4000
+    bt = GpuBatch(a[1], lim)
+    ids = [_add(bt, a), _add(bt, (b[0], b[1], b[2], (b[3][0][:0], b[3][1][:0])))]
+    with pytest.raises(DemError) as e:
+        bt.set_walls(ids[1], *many)
+    assert e.value.code == abi.DEM_ERR_CAPACITY and "bin" in str(e.value)
+    bt.start(ids)
+    bt.step(12)
+    alone = [make_system(_gpu, *a[1:]), make_system(_gpu, b[1], b[2], (b[3][0][:0], b[3][1][:0]))]
+    for sid, g in zip(ids, alone):
+        g.step(12)
+        _compare(bt, sid, g)
+    bt.set_walls(ids[1], *b[3])
+    alone[1].set_walls(*b[3])
+    bt.step(40)
+    for sid, g in zip(ids, alone):
+        g.step(40)
+        assert g.stats()["n_wall_contacts"] > 0
+        _compare(bt, sid, g)
+    bt.close()
+
+
+@pytest.mark.parametrize("kind,nth", [("outflow", 1), ("inflow", 1), ("inflow", 2)])
+def test_boundaries_that_do_not_fit(kind, nth):
+    """The boundaries before stay (here none), until they are set again."""
+    from inflow_cases import inflow_case
+    from oracle_ffi import OracleSystem
+    case, prm, arr, walls, bc, obc = inflow_case(outflow=True)
+    g, o = make_system(_gpu, prm, arr, walls), make_system(OracleSystem, prm, arr, walls)
+    _fail(g, nth)
+    if kind == "outflow":
+        _refused(g.set_outflow_bcs, [obc])
+    else:
+        _refused(g.set_inflow_bcs, [bc], seed=9)
+    for s in (g, o):
+        s.step(12)
+    compare_state(g, o, exact=True)
+    for s in (g, o):
+        s.set_outflow_bcs([obc])
+        s.set_inflow_bcs([bc], seed=9)
+        s.step(100)
+    compare_state(g, o, exact=True)
+    assert g.stats()["n_inflow_added"] == o.stats()["n_inflow_added"] > 0
+
+
 def test_tuning_that_fails_chooses_nothing():
     """The automatic launch shapes stay when the autotuner has no room for the
     histories it keeps (more of them than the upload staged)."""
