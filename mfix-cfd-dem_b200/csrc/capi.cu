@@ -834,6 +834,9 @@ static int replay_period(dem_handle* h, int nn0) {
     if (int rc = ensure_pair_capacity(h, 2 * P + 1024)) return rc;
     invalidate_graphs(h);
   }
+  // the scratch of the build's scans, which a capture cannot make (a handle
+  // whose pairs were uploaded may not have built a list yet)
+  if (int rc = reserve_scan(h, std::max(h->nl(), h->nfl() + 1))) return rc;
   if (h->count_dirty) clear_counts(h);  // a captured step relies on the gather before it
   const int key = (h->cur << 2) | (h->pcur << 1) | h->rb;
   if (!h->graphs[key]) {

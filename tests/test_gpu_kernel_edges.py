@@ -197,6 +197,23 @@ def test_scan_scratch_grown_between_replays():
     compare_pairs(g, o)
 
 
+def test_captured_build_is_the_first():
+    """A handle with uploaded pairs whose first build lies in a captured period,
+    with many more search cells than particles."""
+    from oracle_ffi import OracleSystem
+    case, prm, arr, walls = settling_case(n_side=(8, 8, 8), box=(40e-3, 40e-3, 40e-3), spacing=1.0, nsn=5, seed=23)
+    g, o = _gpu(prm, arr["radius"].size), make_system(OracleSystem, prm, arr, walls)
+    g.upload_state(arr["pos"], arr["vel"], arr["omega"], arr["radius"], arr["pmass"], arr["omoi"], arr["state"],
+                   arr["phase"])
+    g.upload_pairs(*o.download_pairs())
+    o.set_walls(walls[0][:0], walls[1][:0])
+    for s in (g, o):
+        s.step(1, nn_first=2)
+        s.step(10, nn_first=6)
+    compare_state(g, o, exact=True)
+    compare_pairs(g, o)
+
+
 def test_rows_of_an_overflowing_list():
     """1,000 spheres drawn together within one captured period, from no pair to
     several times the capacity of 16 n + 1024: the error is reported, every row
